@@ -12,7 +12,7 @@
 // nearest strictly smaller gap on either side (k_radix_tree; the few gaps
 // whose answer lies beyond the tile's window are searched for in the keys by
 // the block at its end).  Node 0
-// keeps the reference's own search over [0, n_brt-1] (brt_node, write_node);
+// keeps the reference's own range [0, n_brt-1] (coop_root_split, write_root);
 // nodes i >= 1 are the true Karras nodes and each names its children once, so
 // the parent writes are deterministic.
 //
@@ -284,15 +284,6 @@ __global__ void __launch_bounds__(kUniqueThreads)
 // stage 4: Karras radix tree node (func_brt.hpp:45-138)
 // ---------------------------------------------------------------------------
 
-__device__ __forceinline__ int log2_ceil_u(uint32_t x) {
-  const uint32_t lower = 31u - uint32_t(__clz(x));
-  return int(lower + ((uint32_t(1) << lower) < x));
-}
-
-struct BrtNode {
-  int d, j, gamma, dnode;
-};
-
 // delta(a, b) > d, for codes whose top bit is clear (the reference asserts it,
 // func_brt.hpp:30-31): clz(a ^ b) - 1 > d  <=>  a ^ b < 2^(W - 2 - d).  `lim`
 // is that bound (0 when d >= W - 1: never true).
@@ -302,99 +293,28 @@ __device__ __forceinline__ K delta_limit(int d) {
   return (d >= 0 && d <= W - 2) ? (K(1) << (W - 2 - d)) : K(0);
 }
 
-// n = n_brt_nodes; keys live in [0, n].  Same searches as func_brt.hpp:45-138
-// (power-of-two divisions written as shifts, delta comparisons as bounds).
-template <typename K, typename KeyAt>
-__device__ __forceinline__ BrtNode brt_node(int i, int n, const KeyAt& key) {
-  const K ci = key(i);
-  int d;
-  if (i == 0) {
-    d = 1;
-  } else {
-    const int diff = delta(ci, key(i + 1)) - delta(ci, key(i - 1));
-    d = (diff > 0) - (diff < 0);
-  }
-  int l = 0;
-  if (i == 0) {
-    l = n - 1;
-  } else {
-    const K lim = delta_limit<K>(delta(ci, key(i - d)));
-    int lmax = 2;
-    while ((long long)i + (long long)lmax * d >= 0 && i + lmax * d <= n &&
-           (ci ^ key(i + lmax * d)) < lim)
-      lmax *= 2;
-    const int lcut = (d == -1) ? i : n - i;
-    for (int t = lmax >> 1; t >= 1; t >>= 1)
-      if (l + t <= lcut && (ci ^ key(i + (l + t) * d)) < lim) l += t;
-  }
-  BrtNode r;
-  r.d = d;
-  r.j = i + l * d;
-  r.dnode = delta(ci, key(r.j));
-  const K lim = delta_limit<K>(r.dnode);
-  int s = 0;
-  const int kmax = log2_ceil_u(uint32_t(l));  // divisor runs 2, 4, .. 2^kmax
-  const int scut = (d == -1) ? i - 1 : n - i - 1;
-  for (int k = 1; k <= kmax; ++k) {
-    const uint32_t t = (uint32_t(l) + (1u << k) - 1u) >> k;
-    if (uint32_t(s) + t <= uint32_t(scut) &&
-        (ci ^ key(int(uint32_t(i) + (uint32_t(s) + t) * uint32_t(d)))) < lim)
-      s += int(t);
-  }
-  r.gamma = i + s * d + min(d, 0);
-  return r;
-}
-
-// Writes prefix_n / leaf flags / left_child of node i and its parent links.
-// Node 0 writes parents[0] = 0 and a zero for each internal child of the
-// true root of [0, n] (the reference's root covers only [0, n-1]; sequential
+// Writes node 0 (the reference's root over [0, n - 1], func_brt.hpp:80-138),
+// which splits at gamma: prefix_n / leaf flags / left_child, parents[0] = 0
+// and a zero for each internal child of the true root of [0, n] (sequential
 // execution on a zeroed buffer leaves exactly those entries 0, and no other
-// node names them).  Every other entry is written once, by its true parent.
-template <typename K, typename KeyAt>
-__device__ __forceinline__ void write_node(int i, int n, const KeyAt& key,
-                                           const BrtNode& r, uint8_t* prefix_n,
-                                           uint8_t* hl, uint8_t* hr, int32_t* lc,
-                                           int32_t* parents) {
-  prefix_n[i] = uint8_t(r.dnode);
-  const int lo = min(i, r.j), hi = max(i, r.j);
-  const bool leaf_l = lo == r.gamma, leaf_r = hi == r.gamma + 1;
-  hl[i] = leaf_l;
-  hr[i] = leaf_r;
-  lc[i] = r.gamma;
-  if (i > 0) {
-    if (!leaf_l) parents[r.gamma] = i;
-    if (!leaf_r) parents[r.gamma + 1] = i;
-  } else {
-    parents[0] = 0;
-    const int gamma_true = delta(key(n - 1), key(n)) < r.dnode ? n - 1 : r.gamma;
-    if (gamma_true > 0) parents[gamma_true] = 0;
-    if (gamma_true + 1 < n) parents[gamma_true + 1] = 0;
-  }
-}
-
-// Edge count of node i >= 1 without reading parent[] (see file comment).
-template <typename K, typename KeyAt>
-__device__ __forceinline__ int fused_edge_count(int i, int n, const KeyAt& key,
-                                                const BrtNode& r, int root_true_delta,
-                                                int root_prefix) {
-  const int lo = min(i, r.j), hi = max(i, r.j);
-  const int dl = lo > 0 ? delta(key(lo - 1), key(lo)) : -1;
-  const int dr = hi < n ? delta(key(hi), key(hi + 1)) : -1;
-  const int pd = max(dl, dr);
-  const int parent_prefix = pd == root_true_delta ? root_prefix : pd;
-  return r.dnode / 3 - parent_prefix / 3;
+// node names them).
+template <typename K>
+__device__ __forceinline__ void write_root(const K* __restrict__ codes, int n, int dnode,
+                                           int gamma, uint8_t* prefix_n, uint8_t* hl,
+                                           uint8_t* hr, int32_t* lc, int32_t* parents) {
+  prefix_n[0] = uint8_t(dnode);
+  hl[0] = gamma == 0;
+  hr[0] = gamma + 1 == n - 1;
+  lc[0] = gamma;
+  parents[0] = 0;
+  const int gamma_true = delta(codes[n - 1], codes[n]) < dnode ? n - 1 : gamma;
+  if (gamma_true > 0) parents[gamma_true] = 0;
+  if (gamma_true + 1 < n) parents[gamma_true + 1] = 0;
 }
 
 __device__ __forceinline__ void seg_error(int32_t* seg_err, uint32_t c, int32_t code) {
   atomicCAS(reinterpret_cast<int*>(seg_err + c), 0, code);
 }
-
-// Key reads of node 0's searches: global memory only.
-template <typename K>
-struct GlobalKeys {
-  const K* __restrict__ codes;
-  __device__ __forceinline__ K operator()(int j) const { return codes[j]; }
-};
 
 // ---- stages 4 (+5) from nearest smaller values ----------------------------
 //
@@ -408,8 +328,7 @@ struct GlobalKeys {
 // Every node's outputs follow without a search: left_child = g, leaf flags
 // g == L+1 and g+1 == R, the internal children's parent links, and the edge
 // count from the parent's prefix max(D[L], D[R]).  The root (L = -1, R = n)
-// is node 0, which keeps the reference's own computation over [0, n-1]
-// (brt_node / write_node above).
+// is node 0, which keeps the reference's own range [0, n-1] (write_root above).
 //
 // L and R per gap: in chunks of 32 gaps (one per lane) a bit-serial warp
 // comparison of E = D + 1 (0 marks the walls at -1 and n) gives every lane
@@ -517,6 +436,34 @@ __device__ void coop_node_keys(const K* __restrict__ codes, int n, int g, int D,
   *last_key = rlo;
 }
 
+// Last b in [0, n - 1) with delta(key 0, key b) > D, for a D with delta(key 0,
+// key n - 1) = D (so key n - 1 does not qualify): where node 0 splits.  One
+// warp, 32 probes a round (doubling distances, then 32-ary refinement).
+template <typename K>
+__device__ int coop_root_split(const K* __restrict__ codes, int n, int D) {
+  const int lane = int(lane_id());
+  const K c0 = codes[0], lim = delta_limit<K>(D);
+  const int pd = lane < 31 ? (1 << lane) : 0x7fffffff;
+  const bool t = pd < n - 1 && (codes[pd] ^ c0) < lim;
+  const int j = __ffs(__ballot_sync(0xffffffffu, !t)) - 1;  // lane 31 never holds
+  int lo = j == 0 ? 0 : 1 << (j - 1);                       // holds
+  int hi = j < 31 ? min(1 << j, n - 1) : n - 1;             // does not
+  while (hi - lo > 1) {
+    const int st = (hi - lo + 31) / 32, q = lo + (lane + 1) * st;
+    const bool in = lane < 31 && q < hi;
+    const uint32_t f = __ballot_sync(0xffffffffu, in && !((codes[q] ^ c0) < lim));
+    const uint32_t mi = __ballot_sync(0xffffffffu, in);
+    if (f) {
+      const int ff = __ffs(f) - 1;
+      hi = lo + (ff + 1) * st;
+      lo += ff * st;
+    } else {
+      lo += (32 - __clz(mi)) * st;  // every probe in range holds
+    }
+  }
+  return lo;
+}
+
 // Writes the node that splits at gap g, given its nearest smaller gaps L, R
 // (see the ANSV comment below); the root (L = -1, R = n) is skipped.
 // dl, dr: D of gaps L and R (-1 for the walls at -1 and n).
@@ -598,11 +545,17 @@ __global__ void __launch_bounds__(kTreeThreads, 8)  // 8 blocks (64 warps) per S
     root_true_delta = delta(codes[0], codes[n]);
     root_prefix = delta(codes[0], codes[n - 1]);
   }
-  if (blockIdx.x == first && threadIdx.x == 0) {  // node 0, the reference's way
-    const GlobalKeys<K> gk{codes};
-    const BrtNode r = brt_node<K>(0, n, gk);
-    write_node<K>(0, n, gk, r, pn, l8, r8, lcs, par);
-    if (EDGES) edge_count[sb] = 0;
+  // node 0, the reference's range [0, n - 1], by the last warp: as one thread's
+  // binary search it was a chain of about 2 log2(n) dependent loads that the
+  // whole first block waited for (16.5 us for the kernel at 3,001 points, two
+  // blocks); 32 probes a round need at most 6
+  if (blockIdx.x == first && threadIdx.x >= kTreeThreads - 32) {
+    const int d0 = delta(codes[0], codes[n - 1]);
+    const int gamma = coop_root_split<K>(codes, n, d0);
+    if (lane_id() == 0) {
+      write_root<K>(codes, n, d0, gamma, pn, l8, r8, lcs, par);
+      if (EDGES) edge_count[sb] = 0;
+    }
   }
 
   __shared__ uint32_t s_far[kTreeFarPerTile];  // the tile's gaps left to phase D
