@@ -1,9 +1,9 @@
 // The boundary MLP of the learned-CDF sort: 16 -> 64 -> 64 -> 1, ReLU,
 // BF16 weights with FP32 master copies, FP32 biases and FP32 accumulation.
 // Training (forward + backward, FP32 activations) and Adam are hand-written
-// for the CUDA cores: a block takes 32 rows and runs the layers as small
-// matrix products in shared memory; weight gradients are reduced per block and
-// added to the global gradient once.  Inference runs on the tensor cores
+// for the CUDA cores: a block takes tiles of 64 rows and runs the layers as
+// small matrix products in shared memory; the gradient stays in registers over
+// a block's tiles and is added to the global one once per block.  Inference runs on the tensor cores
 // (mlp.cuh).  No reference counterpart (the reference has no learned
 // component).
 #include <cuda_bf16.h>
@@ -25,9 +25,64 @@ __device__ __forceinline__ float bf16_round(float x) {
   return __bfloat162float(__float2bfloat16_rn(x));
 }
 
-// Rows per block and threads per block of the training kernel (4 threads per
-// row, 16 hidden units each).
-constexpr int kRows = 32, kMlpThreads = 128;
+// The training kernel: a block of 256 threads takes tiles of 64 rows.  Every
+// product of a layer (forward, weight gradient, input gradient) is 64 x 64
+// outputs, 4 x 4 per thread (thread = column group tx, row group ty), reduced
+// over k with two 16-byte shared loads per 16 multiply-adds; operands that are
+// reduced over both of their axes are kept in both orders.  The output layer
+// needs no shared memory: 16 lanes hold a row's 64 hidden units.  The gradient
+// stays in registers over the block's tiles and is added to the global one
+// once per block.
+//
+// Bound by the FP32 pipe and the shared loads (about 3,600 multiply-adds per
+// thread and tile), behind the latency of loading the parameters.  Before, a
+// block of 128 threads took 32 rows with one dot product per output (eight
+// rows of a warp on one bank) and added 5,313 values to global memory per 32
+// rows: 63.6 us for 8,192 rows.
+constexpr int kRows = 64, kMlpThreads = 256;
+constexpr int kP = 68, kPx = 20;  // row pitches in floats (16-byte multiples)
+
+struct MlpGradSmem {
+  float w1t[kIn][kP];   // [k][u]
+  float w2t[kH][kP];    // [k][u]
+  float w2[kH][kP];     // [u][k]
+  float xt[kIn][kP];    // [k][row]
+  float xr[kRows][kPx]; // [row][k]
+  float h1t[kH][kP];    // [k][row]
+  float h1[kRows][kP];  // [row][k]
+  float d2t[kH][kP];    // [u][row]
+  float d2[kRows][kP];  // [row][u]: dz2, then dz1
+  float red[3][kH];     // db1, db2, dW3 over the block
+};
+
+__device__ __forceinline__ float4 ld4(const float* p) {
+  return *reinterpret_cast<const float4*>(p);
+}
+
+// acc[i][j] += a[k][i] * b[k][j] over k < N; a and b point at the thread's
+// four columns of row 0.
+template <int N>
+__device__ __forceinline__ void outer_sum(float (&acc)[4][4], const float* a, const float* b) {
+#pragma unroll 8
+  for (int k = 0; k < N; ++k) {
+    const float4 x = ld4(a + k * kP), y = ld4(b + k * kP);
+    const float xa[4] = {x.x, x.y, x.z, x.w}, yb[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xa[i], yb[j], acc[i][j]);
+  }
+}
+
+// grad[0..4) += v; one 16-byte reduction when the gradient is aligned for it.
+__device__ __forceinline__ void add4(float* g, const float (&v)[4], bool vec) {
+  if (vec) {
+    atomicAdd(reinterpret_cast<float4*>(g), make_float4(v[0], v[1], v[2], v[3]));
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) atomicAdd(g + j, v[j]);
+  }
+}
 
 // Forward + backward over `rows` examples: grad += d(mean squared error)/d
 // params for the batch, loss_sum += sum of squared errors.  Weights are used
@@ -36,108 +91,167 @@ __global__ void __launch_bounds__(kMlpThreads)
     k_mlp_grad(const float* __restrict__ params, const float* __restrict__ x,
                const float* __restrict__ t, uint32_t rows, float inv_batch,
                float* __restrict__ grad, float* __restrict__ loss_sum) {
-  __shared__ float s_w1[kH * kIn], s_w2[kH * kH], s_w3[kH], s_b1[kH], s_b2[kH];
-  __shared__ float s_x[kRows * kIn];
-  __shared__ float s_z1[kRows * kH], s_z2[kRows * kH];  // pre-activations
-  __shared__ float s_d[kRows * kH];                      // dz2, then dz1
-  __shared__ float s_dy[kRows];
-  __shared__ float s_loss;
-  const int tid = threadIdx.x;
-  for (int i = tid; i < kH * kIn; i += kMlpThreads) s_w1[i] = bf16_round(params[kOffW1 + i]);
-  for (int i = tid; i < kH * kH; i += kMlpThreads) s_w2[i] = bf16_round(params[kOffW2 + i]);
-  for (int i = tid; i < kH; i += kMlpThreads) {
-    s_w3[i] = bf16_round(params[kOffW3 + i]);
-    s_b1[i] = params[kOffB1 + i];
-    s_b2[i] = params[kOffB2 + i];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  MlpGradSmem& sm = *reinterpret_cast<MlpGradSmem*>(smem_raw);
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int c0 = tx * 4, r0 = ty * 4;  // this thread's columns and rows of a product
+  for (int i = tid; i < kH * kIn; i += kMlpThreads)
+    sm.w1t[i % kIn][i / kIn] = bf16_round(params[kOffW1 + i]);
+  for (int i = tid; i < kH * kH; i += kMlpThreads) {
+    const float w = bf16_round(params[kOffW2 + i]);
+    sm.w2[i / kH][i % kH] = w;
+    sm.w2t[i % kH][i / kH] = w;
+  }
+  if (tid < 3 * kH) sm.red[tid / kH][tid % kH] = 0.0f;
+  float w3[4], b1[4], b2[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    w3[j] = bf16_round(params[kOffW3 + c0 + j]);
+    b1[j] = params[kOffB1 + c0 + j];
+    b2[j] = params[kOffB2 + c0 + j];
   }
   const float b3 = params[kOffB3];
-  if (tid == 0) s_loss = 0.0f;
-  const uint32_t r0 = blockIdx.x * kRows;
-  const int nr = int(min(uint32_t(kRows), rows - r0));
-  for (int i = tid; i < kRows * kIn; i += kMlpThreads) {
-    const int r = i / kIn;
-    s_x[i] = r < nr ? x[size_t(r0 + r) * kIn + (i % kIn)] : 0.0f;
-  }
-  __syncthreads();
 
-  // z1 = W1 x + b1 ; z2 = W2 relu(z1) + b2   (thread: row r = tid / 4, 16 units)
-  static_assert(kRows * 4 == kMlpThreads, "four threads per row");
-  const int r = tid >> 2, u0 = (tid & 3) * 16;
-  for (int u = u0; u < u0 + 16; ++u) {
-    float acc = s_b1[u];
-    for (int k = 0; k < kIn; ++k) acc = fmaf(s_w1[u * kIn + k], s_x[r * kIn + k], acc);
-    s_z1[r * kH + u] = acc;
-  }
-  __syncthreads();
-  for (int u = u0; u < u0 + 16; ++u) {
-    float acc = s_b2[u];
-    for (int k = 0; k < kH; ++k) acc = fmaf(s_w2[u * kH + k], fmaxf(s_z1[r * kH + k], 0.0f), acc);
-    s_z2[r * kH + u] = acc;
-  }
-  __syncthreads();
-  // y, dy (one thread per row)
-  if (tid < kRows) {
-    const int rr = tid;
-    float y = b3;
-    for (int k = 0; k < kH; ++k) y = fmaf(s_w3[k], fmaxf(s_z2[rr * kH + k], 0.0f), y);
-    float dy = 0.0f;
-    if (rr < nr) {
-      const float e = y - t[r0 + rr];
-      atomicAdd(&s_loss, e * e);
-      dy = 2.0f * e * inv_batch;
+  float gw2[4][4] = {}, gw1[4] = {}, gw3[4] = {}, gb1[4] = {}, gb2[4] = {};
+  float gb3 = 0.0f, loss = 0.0f;
+  const uint32_t tiles = (rows + kRows - 1) / kRows;
+  for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const uint32_t row0 = tile * kRows;
+    const int nr = int(min(uint32_t(kRows), rows - row0));
+#pragma unroll
+    for (int q = 0; q < kRows * kIn / kMlpThreads; ++q) {
+      const int i = q * kMlpThreads + tid, r = i / kIn, k = i % kIn;
+      const float v = r < nr ? x[size_t(row0 + r) * kIn + k] : 0.0f;
+      sm.xr[r][k] = v;
+      sm.xt[k][r] = v;
     }
-    s_dy[rr] = dy;
-  }
-  __syncthreads();
-  // dz2 = dy * w3 * [z2 > 0]
-  for (int i = tid; i < kRows * kH; i += kMlpThreads) {
-    const int rr = i / kH, k = i % kH;
-    s_d[i] = s_z2[i] > 0.0f ? s_dy[rr] * s_w3[k] : 0.0f;
-  }
-  __syncthreads();
-  // gradients of layer 3 and 2: dW3[k] = sum dy h2 ; db3 ; dW2[u][k] = sum dz2[u] h1[k]
-  for (int k = tid; k < kH; k += kMlpThreads) {
-    float g3 = 0.0f, gb2 = 0.0f;
-    for (int rr = 0; rr < kRows; ++rr) {
-      g3 = fmaf(s_dy[rr], fmaxf(s_z2[rr * kH + k], 0.0f), g3);
-      gb2 += s_d[rr * kH + k];
+    float tgt[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) tgt[i] = r0 + i < nr ? t[row0 + r0 + i] : 0.0f;
+    __syncthreads();
+
+    // h1 = relu(W1 x + b1): rows r0.., units c0..
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = b1[j];
+    outer_sum<kIn>(acc, &sm.xt[0][r0], &sm.w1t[0][c0]);
+    uint32_t on = 0;  // bit 4 i + j: z1 > 0
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        on |= uint32_t(acc[i][j] > 0.0f) << (4 * i + j);
+        acc[i][j] = fmaxf(acc[i][j], 0.0f);
+      }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      *reinterpret_cast<float4*>(&sm.h1[r0 + i][c0]) =
+          make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+      *reinterpret_cast<float4*>(&sm.h1t[c0 + i][r0]) =
+          make_float4(acc[0][i], acc[1][i], acc[2][i], acc[3][i]);
     }
-    atomicAdd(&grad[kOffW3 + k], g3);
-    atomicAdd(&grad[kOffB2 + k], gb2);
+    __syncthreads();
+
+    // z2 = W2 h1 + b2, y = W3 relu(z2) + b3, dz2 = dy w3 [z2 > 0]
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = b2[j];
+    outer_sum<kH>(acc, &sm.h1t[0][r0], &sm.w2t[0][c0]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float y = 0.0f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) y = fmaf(w3[j], fmaxf(acc[i][j], 0.0f), y);
+#pragma unroll
+      for (int d = 1; d < 16; d <<= 1) y += __shfl_xor_sync(0xffffffffu, y, d);
+      const float e = r0 + i < nr ? y + b3 - tgt[i] : 0.0f;
+      const float dy = 2.0f * e * inv_batch;
+      if (tx == 0) {
+        loss = fmaf(e, e, loss);
+        gb3 += dy;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        gw3[j] = fmaf(dy, fmaxf(acc[i][j], 0.0f), gw3[j]);
+        acc[i][j] = acc[i][j] > 0.0f ? dy * w3[j] : 0.0f;
+        gb2[j] += acc[i][j];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      *reinterpret_cast<float4*>(&sm.d2[r0 + i][c0]) =
+          make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+      *reinterpret_cast<float4*>(&sm.d2t[c0 + i][r0]) =
+          make_float4(acc[0][i], acc[1][i], acc[2][i], acc[3][i]);
+    }
+    __syncthreads();
+
+    // dW2[u][k] += sum over rows of dz2[u] h1[k]: units r0.., inputs c0..
+    outer_sum<kRows>(gw2, &sm.d2[0][r0], &sm.h1[0][c0]);
+    // dz1 = (W2^T dz2) [z1 > 0]: rows r0.., units c0..
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+    outer_sum<kH>(acc, &sm.d2t[0][r0], &sm.w2[0][c0]);
+    __syncthreads();  // every read of dz2 is done before dz1 takes its place
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        acc[i][j] = (on >> (4 * i + j)) & 1u ? acc[i][j] : 0.0f;
+        gb1[j] += acc[i][j];
+      }
+      *reinterpret_cast<float4*>(&sm.d2[r0 + i][c0]) =
+          make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    }
+    __syncthreads();
+    // dW1[u][k] += sum over rows of dz1[u] x[k]: unit tid / 4, four inputs
+    {
+      const int u = tid >> 2, k0 = (tid & 3) * 4;
+#pragma unroll 8
+      for (int r = 0; r < kRows; ++r) {
+        const float d = sm.d2[r][u];
+        const float4 v = ld4(&sm.xr[r][k0]);
+        gw1[0] = fmaf(d, v.x, gw1[0]);
+        gw1[1] = fmaf(d, v.y, gw1[1]);
+        gw1[2] = fmaf(d, v.z, gw1[2]);
+        gw1[3] = fmaf(d, v.w, gw1[3]);
+      }
+    }
+    __syncthreads();  // the next tile writes x
   }
-  if (tid == 0) {
-    float gb3 = 0.0f;
-    for (int rr = 0; rr < kRows; ++rr) gb3 += s_dy[rr];
+
+  // the block's sums: the bias and output-layer gradients over its row groups
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    gb1[j] += __shfl_xor_sync(0xffffffffu, gb1[j], 16);
+    gb2[j] += __shfl_xor_sync(0xffffffffu, gb2[j], 16);
+    gw3[j] += __shfl_xor_sync(0xffffffffu, gw3[j], 16);
+    if ((tid & 16) == 0) {
+      atomicAdd(&sm.red[0][c0 + j], gb1[j]);
+      atomicAdd(&sm.red[1][c0 + j], gb2[j]);
+      atomicAdd(&sm.red[2][c0 + j], gw3[j]);
+    }
+  }
+  gb3 += __shfl_xor_sync(0xffffffffu, gb3, 16);
+  loss += __shfl_xor_sync(0xffffffffu, loss, 16);
+  if ((tid & 31) == 0) {
     atomicAdd(&grad[kOffB3], gb3);
+    if (loss_sum) atomicAdd(loss_sum, loss);
   }
-  for (int i = tid; i < kH * kH; i += kMlpThreads) {
-    const int u = i / kH, k = i % kH;
-    float g = 0.0f;
-    for (int rr = 0; rr < kRows; ++rr) g = fmaf(s_d[rr * kH + u], fmaxf(s_z1[rr * kH + k], 0.0f), g);
-    atomicAdd(&grad[kOffW2 + i], g);
-  }
-  __syncthreads();  // every read of z2 is done before it is overwritten
-  // dh1 = W2^T dz2 ; dz1 = dh1 * [z1 > 0]   (written over s_z2, no longer needed)
-  for (int k = u0; k < u0 + 16; ++k) {
-    float acc = 0.0f;
-    for (int u = 0; u < kH; ++u) acc = fmaf(s_w2[u * kH + k], s_d[r * kH + u], acc);
-    s_z2[r * kH + k] = s_z1[r * kH + k] > 0.0f ? acc : 0.0f;
-  }
+  static_assert(kOffW1 % 4 == 0 && kOffW2 % 4 == 0, "four parameters at a time");
+  const bool vec = (reinterpret_cast<uintptr_t>(grad) & 15u) == 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) add4(grad + kOffW2 + (r0 + i) * kH + c0, gw2[i], vec);
+  add4(grad + kOffW1 + tid * 4, gw1, vec);
   __syncthreads();
-  // dW1[u][k] = sum dz1[u] x[k] ; db1[u] = sum dz1[u]
-  for (int i = tid; i < kH * kIn; i += kMlpThreads) {
-    const int u = i / kIn, k = i % kIn;
-    float g = 0.0f;
-    for (int rr = 0; rr < kRows; ++rr) g = fmaf(s_z2[rr * kH + u], s_x[rr * kIn + k], g);
-    atomicAdd(&grad[kOffW1 + i], g);
-  }
-  for (int u = tid; u < kH; u += kMlpThreads) {
-    float g = 0.0f;
-    for (int rr = 0; rr < kRows; ++rr) g += s_z2[rr * kH + u];
-    atomicAdd(&grad[kOffB1 + u], g);
-  }
-  __syncthreads();
-  if (tid == 0 && loss_sum) atomicAdd(loss_sum, s_loss);
+  if (tid < kH) atomicAdd(&grad[kOffB1 + tid], sm.red[0][tid]);
+  else if (tid < 2 * kH) atomicAdd(&grad[kOffB2 + tid - kH], sm.red[1][tid - kH]);
+  else if (tid < 3 * kH) atomicAdd(&grad[kOffW3 + tid - 2 * kH], sm.red[2][tid - 2 * kH]);
 }
 
 // Adam on the FP32 master parameters (Kingma & Ba 2015, bias-corrected).
@@ -193,9 +307,17 @@ int rw_tree_mlp_grad(const float* d_params, const float* d_x, const float* d_t, 
                      uint32_t batch, float* d_grad, float* d_loss_sum, rw_stream_t stream) {
   if (!d_params || !d_x || !d_t || !d_grad || rows < 1 || batch < 1) return RW_ERR_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  const uint32_t blocks = (rows + rwt::kRows - 1) / rwt::kRows;
-  rwt::k_mlp_grad<<<blocks, rwt::kMlpThreads, 0, s>>>(d_params, d_x, d_t, rows,
-                                                     1.0f / float(batch), d_grad, d_loss_sum);
+  const uint32_t tiles = (rows + rwt::kRows - 1) / rwt::kRows;
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(rwt::k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             int(sizeof(rwt::MlpGradSmem)));
+  if (e != cudaSuccess) return RW_ERR_CUDA;
+  const uint32_t blocks = tiles < uint32_t(sms) ? tiles : uint32_t(sms);  // one per SM
+  rwt::k_mlp_grad<<<blocks, rwt::kMlpThreads, sizeof(rwt::MlpGradSmem), s>>>(
+      d_params, d_x, d_t, rows, 1.0f / float(batch), d_grad, d_loss_sum);
   return cudaGetLastError() == cudaSuccess ? RW_OK : RW_ERR_CUDA;
 }
 
