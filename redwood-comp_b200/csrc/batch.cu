@@ -451,7 +451,7 @@ int rw_tree_batch_enqueue(rw_tree_batch* b, const rw_tree_batch_buffers* u, rw_s
     RWB_CUDA(rwt::launch_sort_passes(x, sk, pk, s));
   }
   RWB_CUDA(rwt::launch_unique(x, sc, pl, s));
-  RWB_CUDA(rwt::launch_radix_tree(x, sc, pl, true, s));
+  RWB_CUDA(rwt::launch_radix_tree(x, sc, pl, true, false, s));
   RWB_CUDA(rwt::launch_edge_sums(x, sc, pl, s));
   RWB_CUDA(rwt::launch_octree(x, sc, pl, s, nullptr, true));
   const size_t c = b->n_clouds;

@@ -432,9 +432,7 @@ int rw_tree_run_stage4(rw_tree_app_data* app, rw_tree_im_storage* im,
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (int rc = upload_counts(app, im, s)) return rc;
   RW_CUDA(rwt::launch_radix_tree(bufs_of(*app, im), scratch_of(im), plan_of(*app, im), false,
-                                 s));
-  if (geometric_delta(im))
-    RW_CUDA(rwt::launch_prefix_shift(bufs_of(*app, im), scratch_of(im), plan_of(*app, im), s));
+                                 geometric_delta(im), s));
   return sync_status(im, s);
 }
 
@@ -516,15 +514,7 @@ int enqueue_impl(rw_tree_app_data* app, rw_tree_im_storage* im, cudaStream_t s,
   }
   RW_CUDA(rwt::launch_unique(b, sc, pl, s));
   RW_CUDA(mark());
-  if (geometric_delta(im)) {
-    // the tree with the reference's delta, every prefix lowered by one, then
-    // the edge counts from the lowered prefixes
-    RW_CUDA(rwt::launch_radix_tree(b, sc, pl, false, s));
-    RW_CUDA(rwt::launch_prefix_shift(b, sc, pl, s));
-    RW_CUDA(rwt::launch_edge_count(b, sc, pl, s));
-  } else {
-    RW_CUDA(rwt::launch_radix_tree(b, sc, pl, true, s));
-  }
+  RW_CUDA(rwt::launch_radix_tree(b, sc, pl, true, geometric_delta(im), s));
   RW_CUDA(mark());
   RW_CUDA(rwt::launch_edge_sums(b, sc, pl, s));
   RW_CUDA(mark());

@@ -194,9 +194,11 @@ cudaError_t launch_unique(const Bufs& b, const Scratch& sc, const Plan& pl, cuda
 cudaError_t launch_unique_raw(const void* sorted, void* out, uint32_t n, int key_bits,
                               uint32_t* counts, DevStatus* status, int num_sms,
                               cudaStream_t s);
-// Stage 4 alone (edges = false) or stages 4 and 5 in one pass (edges = true).
+// Stage 4 alone (edges = false) or stages 4 and 5 in one pass (edges = true);
+// geometric: every prefix length lowered by one (RW_TREE_OPT_GEOMETRIC_DELTA,
+// 32-bit keys).
 cudaError_t launch_radix_tree(const Bufs& b, const Scratch& sc, const Plan& pl, bool edges,
-                              cudaStream_t s);
+                              bool geometric, cudaStream_t s);
 cudaError_t launch_edge_count(const Bufs& b, const Scratch& sc, const Plan& pl,
                               cudaStream_t s);
 cudaError_t launch_edge_scan(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_t s);
@@ -207,11 +209,7 @@ cudaError_t launch_edge_sums(const Bufs& b, const Scratch& sc, const Plan& pl, c
 cudaError_t launch_octree(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_t s,
                           cudaEvent_t* marks = nullptr, bool fused_offsets = false);
 
-// Options outside the reference contract (RW_TREE_OPT_*), single cloud only:
-// prefix_n[0, n_brt) -= 1 after stage 4 (the clz - 2 delta of 32-bit keys),
-// and the leaf links after stage 7.
-cudaError_t launch_prefix_shift(const Bufs& b, const Scratch& sc, const Plan& pl,
-                                cudaStream_t s);
+// The leaf links after stage 7 (RW_TREE_OPT_LINK_LEAVES), single cloud only.
 cudaError_t launch_leaf_links(const Bufs& b, const Scratch& sc, const Plan& pl,
                               cudaStream_t s);
 

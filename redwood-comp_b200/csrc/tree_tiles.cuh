@@ -1,0 +1,1043 @@
+// Device code of stages 4 to 7 over one tile of radix-tree gaps or nodes, shared
+// by the kernels that launch a block per tile (k_tree.cu) and the one that
+// keeps a whole small cloud on the chip (k_small.cu).
+#pragma once
+
+#include "internal.hpp"
+#include "morton.cuh"
+
+namespace rwt {
+
+// ---------------------------------------------------------------------------
+// stage 4: radix-tree nodes (func_brt.hpp:45-138)
+// ---------------------------------------------------------------------------
+
+// delta(a, b) > d, for codes whose top bit is clear (the reference asserts it,
+// func_brt.hpp:30-31): clz(a ^ b) - 1 > d  <=>  a ^ b < 2^(W - 2 - d).  `lim`
+// is that bound (0 when d >= W - 1: never true).
+template <typename K>
+__device__ __forceinline__ K delta_limit(int d) {
+  constexpr int W = KeyTraits<K>::kWordBits;
+  return (d >= 0 && d <= W - 2) ? (K(1) << (W - 2 - d)) : K(0);
+}
+
+// Writes node 0 (the reference's root over [0, n - 1], func_brt.hpp:80-138),
+// which splits at gamma: prefix_n / leaf flags / left_child, parents[0] = 0
+// and a zero for each internal child of the true root of [0, n] (sequential
+// execution on a zeroed buffer leaves exactly those entries 0, and no other
+// node names them).
+template <typename K, int LESS>
+__device__ __forceinline__ void write_root(const K* __restrict__ codes, int n, int dnode,
+                                           int gamma, uint8_t* prefix_n, uint8_t* hl,
+                                           uint8_t* hr, int32_t* lc, int32_t* parents) {
+  prefix_n[0] = uint8_t(dnode - LESS);
+  hl[0] = gamma == 0;
+  hr[0] = gamma + 1 == n - 1;
+  lc[0] = gamma;
+  parents[0] = 0;
+  const int gamma_true = delta(codes[n - 1], codes[n]) < dnode ? n - 1 : gamma;
+  if (gamma_true > 0) parents[gamma_true] = 0;
+  if (gamma_true + 1 < n) parents[gamma_true + 1] = 0;
+}
+
+__device__ __forceinline__ void seg_error(int32_t* seg_err, uint32_t c, int32_t code) {
+  atomicCAS(reinterpret_cast<int*>(seg_err + c), 0, code);
+}
+
+// ---- stages 4 (+5) from nearest smaller values ----------------------------
+//
+// With D[k] = delta(key k, key k+1) for the n gaps k in [0, n), the binary
+// radix tree of the keys is the Cartesian tree of D: the node that splits at
+// gap g covers keys [L+1, R], where L < g and R > g are the nearest gaps with
+// D strictly smaller than D[g] (-1 and n when there are none); its prefix
+// length is D[g]; its parent splits at whichever of L, R has the larger D; and
+// its Karras index (the one process_radix_tree_i gives it, func_brt.hpp:45-138)
+// is R when it is its parent's left child and L+1 when it is the right child.
+// Every node's outputs follow without a search: left_child = g, leaf flags
+// g == L+1 and g+1 == R, the internal children's parent links, and the edge
+// count from the parent's prefix max(D[L], D[R]).  The root (L = -1, R = n)
+// is node 0, which keeps the reference's own range [0, n-1] (write_root above).
+//
+// L and R per gap: in chunks of 32 gaps (one per lane) a bit-serial warp
+// comparison of E = D + 1 (0 marks the walls at -1 and n) gives every lane
+// the lanes with a smaller value, hence the nearest smaller in the chunk, and
+// every value v the last / first position in the chunk below v.  Across the
+// tile and a halo of kAnsvHalo chunks on either side, per-value bitmasks of
+// the chunks whose minimum lies below v find the nearest such chunk in one
+// clz / ffs, and its summary gives the answer; a gap whose nearest smaller
+// lies beyond the halo (a node near the top of the tree) goes to a list in
+// shared memory that the block resolves at its end with warp-cooperative
+// searches of the keys.
+constexpr int kAnsvHalo = 8;             // chunks per side
+constexpr int kAnsvNone = -0x7fffffff;     // "no smaller gap found to the left"
+constexpr int kAnsvNoneR = 0x7fffffff;     // "none to the right"
+
+// Last / first position in a chunk of 32 E values (4-byte aligned) whose
+// value is below e; the caller knows there is one.
+__device__ __forceinline__ int chunk_last_below(const uint8_t* ce, int e) {
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(ce);
+  const uint32_t ev = 0x01010101u * uint32_t(e);
+  for (int q = 7; q > 0; --q) {
+    const uint32_t below = __vcmpltu4(w[q], ev);  // 0xff in each byte below e
+    if (below) return 4 * q + (31 - __clz(below)) / 8;
+  }
+  return (31 - __clz(__vcmpltu4(w[0], ev))) / 8;
+}
+
+__device__ __forceinline__ int chunk_first_below(const uint8_t* ce, int e) {
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(ce);
+  const uint32_t ev = 0x01010101u * uint32_t(e);
+  for (int q = 0; q < 7; ++q) {
+    const uint32_t below = __vcmpltu4(w[q], ev);
+    if (below) return 4 * q + (__ffs(below) - 1) / 8;
+  }
+  return 28 + (__ffs(__vcmpltu4(w[7], ev)) - 1) / 8;
+}
+
+// TCH: the most chunks of 32 gaps that a tile has.
+template <typename K, int TCH>
+struct AnsvCfg {
+  static constexpr int NV = sizeof(K) == 4 ? 32 : 64;  // values of E
+  static constexpr int VB = sizeof(K) == 4 ? 5 : 6;    // bits of E
+  static constexpr int kChunks = TCH + 2 * kAnsvHalo;  // chunks per window
+  static constexpr int kWin = kChunks * 32;            // gaps per window
+  static constexpr int kRow = TCH + 1;  // padded: lane v and chunk c in different banks
+  static constexpr size_t kKeyBytes = (size_t(kWin) + 1) * sizeof(K);
+  static constexpr int MW = (kChunks + 31) / 32;  // mask words per value
+  static constexpr size_t kSmem = kKeyBytes + size_t(NV) * MW * 4 + 4 * size_t(TCH) * 32 +
+                                  size_t(kWin) + 2 * size_t(NV) * kRow + size_t(kChunks);
+};
+
+// Warp-cooperative search for the nearest smaller gaps of gap g beyond any
+// window, both sides in lockstep: 32 probes per side and round (doubling
+// distances, then 32-ary refinement), the two sides' loads issued together,
+// so the pair costs about as many dependent loads as the longer side.
+// Left: pred(a) = delta(key a, key g) > D is true from some a_min up to g;
+// *first_key = a_min (the node's first key).  Right: pred(b) = delta(key g+1,
+// key b) > D is true from g+1 up to some b_max <= n; *last_key = b_max.
+template <typename K>
+__device__ void coop_node_keys(const K* __restrict__ codes, int n, int g, int D,
+                               int* first_key, int* last_key) {
+  const uint32_t lane = lane_id();
+  const K cl = codes[g], cr = codes[g + 1], lim = delta_limit<K>(D);
+  const int pl = lane < 31 ? g - (1 << lane) : -1;
+  const long long pr = lane < 31 ? (long long)g + 1 + (1ll << lane) : (long long)n + 1;
+  const bool fl = pl >= 0 && (codes[pl] ^ cl) < lim;
+  const bool fr = pr <= n && (codes[int(pr)] ^ cr) < lim;
+  const int jl = __ffs(__ballot_sync(0xffffffffu, !fl)) - 1;  // a false probe exists
+  const int jr = __ffs(__ballot_sync(0xffffffffu, !fr)) - 1;
+  int llo = max(jl < 31 ? g - (1 << jl) : -1, -1);                // pred(llo) false
+  int lhi = jl == 0 ? g : g - (1 << (jl - 1));                    // pred(lhi) true
+  int rhi = jr < 31 ? int(min((long long)g + 1 + (1ll << jr), (long long)n + 1)) : n + 1;
+  int rlo = jr == 0 ? g + 1 : g + 1 + (1 << (jr - 1));            // pred(rlo) true
+  while (lhi - llo > 1 || rhi - rlo > 1) {
+    const bool la = lhi - llo > 1, ra = rhi - rlo > 1;  // warp-uniform
+    const int ls = la ? (lhi - llo + 31) / 32 : 0, rs = ra ? (rhi - rlo + 31) / 32 : 0;
+    const int lq = llo + (int(lane) + 1) * ls, rq = rlo + (int(lane) + 1) * rs;
+    const bool lin = la && lane < 31 && lq < lhi, rin = ra && lane < 31 && rq < rhi;
+    const bool lt = lin && (codes[lq] ^ cl) < lim;
+    const bool rt = rin && (codes[rq] ^ cr) < lim;
+    const uint32_t mlt = __ballot_sync(0xffffffffu, lt), mli = __ballot_sync(0xffffffffu, lin);
+    const uint32_t mrf = __ballot_sync(0xffffffffu, rin && !rt),
+                   mri = __ballot_sync(0xffffffffu, rin);
+    if (la) {
+      if (mlt) {
+        const int ft = __ffs(mlt) - 1;
+        lhi = llo + (ft + 1) * ls;
+        llo = ft > 0 ? llo + ft * ls : llo;
+      } else {
+        llo = llo + (32 - __clz(mli)) * ls;  // the last probe in range is false
+      }
+    }
+    if (ra) {
+      if (mrf) {
+        const int ff = __ffs(mrf) - 1;
+        rhi = rlo + (ff + 1) * rs;
+        rlo = ff > 0 ? rlo + ff * rs : rlo;
+      } else {
+        rlo = rlo + (32 - __clz(mri)) * rs;  // every probe in range is true
+      }
+    }
+  }
+  *first_key = lhi;
+  *last_key = rlo;
+}
+
+// Last b in [0, n - 1) with delta(key 0, key b) > D, for a D with delta(key 0,
+// key n - 1) = D (so key n - 1 does not qualify): where node 0 splits.  One
+// warp, 32 probes a round (doubling distances, then 32-ary refinement).
+template <typename K>
+__device__ int coop_root_split(const K* __restrict__ codes, int n, int D) {
+  const int lane = int(lane_id());
+  const K c0 = codes[0], lim = delta_limit<K>(D);
+  const int pd = lane < 31 ? (1 << lane) : 0x7fffffff;
+  const bool t = pd < n - 1 && (codes[pd] ^ c0) < lim;
+  const int j = __ffs(__ballot_sync(0xffffffffu, !t)) - 1;  // lane 31 never holds
+  int lo = j == 0 ? 0 : 1 << (j - 1);                       // holds
+  int hi = j < 31 ? min(1 << j, n - 1) : n - 1;             // does not
+  while (hi - lo > 1) {
+    const int st = (hi - lo + 31) / 32, q = lo + (lane + 1) * st;
+    const bool in = lane < 31 && q < hi;
+    const uint32_t f = __ballot_sync(0xffffffffu, in && !((codes[q] ^ c0) < lim));
+    const uint32_t mi = __ballot_sync(0xffffffffu, in);
+    if (f) {
+      const int ff = __ffs(f) - 1;
+      hi = lo + (ff + 1) * st;
+      lo += ff * st;
+    } else {
+      lo += (32 - __clz(mi)) * st;  // every probe in range holds
+    }
+  }
+  return lo;
+}
+
+// Writes the node that splits at gap g, given its nearest smaller gaps L, R
+// (see the ANSV comment below); the root (L = -1, R = n) is skipped.
+// dl, dr: D of gaps L and R (-1 for the walls at -1 and n).  LESS (0 or 1) is
+// taken off every prefix length that is written or counted
+// (RW_TREE_OPT_GEOMETRIC_DELTA: the tree's shape depends only on comparisons
+// between deltas, so the clz - 2 tree is the clz - 1 tree with every prefix,
+// at least 1 for distinct 30-bit keys, lowered by one).
+template <bool EDGES, int LESS>
+__device__ __forceinline__ void write_gap_node_d(int g, int D, int L, int R, int dl, int dr,
+                                                 int root_true_delta, int root_prefix,
+                                                 uint8_t* pn, uint8_t* l8, uint8_t* r8,
+                                                 int32_t* lcs, int32_t* par, int32_t* ec) {
+  const int i = dr > dl ? R : L + 1;  // left child of R's node, else right child of L's
+  const bool leaf_l = g == L + 1, leaf_r = g + 1 == R;
+  pn[i] = uint8_t(D - LESS);
+  l8[i] = leaf_l;
+  r8[i] = leaf_r;
+  lcs[i] = g;
+  if (!leaf_l) par[g] = i;
+  if (!leaf_r) par[g + 1] = i;
+  if (EDGES) {
+    const int pd = max(dl, dr);
+    const int pp = pd == root_true_delta ? root_prefix : pd;
+    ec[i] = (D - LESS) / 3 - (pp - LESS) / 3;
+  }
+}
+
+template <typename K, bool EDGES, int LESS, typename DAt>
+__device__ __forceinline__ void write_gap_node(int g, int n, int D, int L, int R, const DAt& d_at,
+                                               int root_true_delta, int root_prefix,
+                                               uint8_t* pn, uint8_t* l8, uint8_t* r8,
+                                               int32_t* lcs, int32_t* par, int32_t* ec) {
+  if (L < 0 && R >= n) return;
+  write_gap_node_d<EDGES, LESS>(g, D, L, R, L >= 0 ? d_at(L) : -1, R < n ? d_at(R) : -1,
+                          root_true_delta, root_prefix, pn, l8, r8, lcs, par, ec);
+}
+
+// The shared words of a tile besides the arrays in dynamic shared memory.
+struct TreeTileShared {
+  uint32_t far[kTreeFarPerTile];  // the tile's gaps left to phase D
+  uint32_t far_n, pend_n;
+  alignas(8) uint64_t bar;
+};
+
+// Stage 4 (and 5 with EDGES) for the gaps [g0, g0 + 32 tch) of a cloud whose n
+// gaps lie between codes[0 .. n], by a block of NT threads.  DYN: tch is a run
+// time number up to TCH, else it is TCH.  BULK: the keys may come by a bulk
+// copy (not in a kernel that wrote them itself: the copy engine would need a
+// proxy fence).  `err` takes the first error.  The tile that starts at 0 also
+// writes node 0.
+template <typename K, bool EDGES, int LESS, int NT, int TCH, bool DYN, bool BULK>
+__device__ __forceinline__ void tree_tile(unsigned char* smem_raw, TreeTileShared& sh,
+                                          const K* __restrict__ codes, int n, int g0,
+                                          int tch_arg, int32_t* err, uint8_t* __restrict__ pn,
+                                          uint8_t* __restrict__ l8, uint8_t* __restrict__ r8,
+                                          int32_t* __restrict__ lcs, int32_t* __restrict__ par,
+                                          int32_t* __restrict__ ec) {
+  using C = AnsvCfg<K, TCH>;
+  constexpr int NV = C::NV, VB = C::VB, NW = NT / 32, JN = DYN ? 1 : 2;
+  static_assert(kTreeFarPerTile >= 2 * uint32_t(NV), "far gaps of a tile: NV per side");
+  const int tch = DYN ? tch_arg : TCH;
+  const int chunks = tch + 2 * kAnsvHalo, win = chunks * 32;
+  // positions inside a chunk are kept as lane indices (0xff: none)
+  K* s_key = reinterpret_cast<K*>(smem_raw);                                // [win + 1]
+  uint32_t* s_mask = reinterpret_cast<uint32_t*>(smem_raw + C::kKeyBytes);  // [NV][MW]
+  // the tile's gaps left to phase C: tile index | in-chunk left << 16 |
+  // in-chunk right << 24 (lane indices, 0xff: none)
+  uint32_t* s_pend = s_mask + NV * C::MW;                                   // [32 TCH]
+  uint8_t* s_e = reinterpret_cast<uint8_t*>(s_pend + 32 * TCH);             // [win]
+  // summaries of the tile's chunks only (a halo chunk is scanned when asked)
+  uint8_t* s_last = s_e + C::kWin;                                          // [NV][kRow]
+  uint8_t* s_first = s_last + NV * C::kRow;                                 // [NV][kRow]
+  uint8_t* s_cmin = s_first + NV * C::kRow;                                 // [chunks]
+  const int wlo = g0 - kAnsvHalo * 32;  // first gap of the window
+
+  int root_true_delta = 0, root_prefix = 0;
+  if (EDGES) {
+    root_true_delta = delta(codes[0], codes[n]);
+    root_prefix = delta(codes[0], codes[n - 1]);
+  }
+  // node 0, the reference's range [0, n - 1], by the last warp: as one thread's
+  // binary search it was a chain of about 2 log2(n) dependent loads that the
+  // whole first block waited for (16.5 us for the kernel at 3,001 points, two
+  // blocks); 32 probes a round need at most 6
+  auto root_node = [&] {
+    const int d0 = delta(codes[0], codes[n - 1]);
+    const int gamma = coop_root_split<K>(codes, n, d0);
+    if (lane_id() == 0) {
+      write_root<K, LESS>(codes, n, d0, gamma, pn, l8, r8, lcs, par);
+      if (EDGES) ec[0] = 0;
+    }
+  };
+  if (!DYN && g0 == 0 && threadIdx.x >= NT - 32) root_node();
+
+  if (threadIdx.x == 0) {  // read after the barriers below
+    sh.far_n = 0;
+    sh.pend_n = 0;
+  }
+
+  // the window's keys [wlo, wlo + kAnsvWin]: one bulk copy when the window
+  // lies inside the keys and starts on a 16-byte boundary (every interior
+  // tile of a plain run), else key by key with zeros outside [0, n]
+  static_assert((size_t(C::kWin) * sizeof(K)) % 16 == 0, "bulk copies move 16-byte units");
+  const bool bulk = BULK && wlo >= 0 && wlo + win <= n &&
+                    (reinterpret_cast<uintptr_t>(codes + wlo) & 15u) == 0;
+  if (bulk) {
+    if (threadIdx.x == 0) bulk_barrier_init(&sh.bar);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      bulk_load(s_key, codes + wlo, uint32_t(win * sizeof(K)), &sh.bar);
+      s_key[win] = codes[wlo + win];
+    }
+    const bool landed = bulk_wait(&sh.bar, kSpinLimit);
+    if (__syncthreads_or(!landed)) {  // the whole block gives up together
+      // report, and let the copy land before the block's shared memory goes
+      if (threadIdx.x == 0) atomicCAS(reinterpret_cast<int*>(err), 0, RW_ERR_TIMEOUT);
+      bulk_wait(&sh.bar, kSpinLimit);
+      return;
+    }
+  } else {
+    for (int j = threadIdx.x; j <= win; j += NT) {
+      const int k = wlo + j;
+      s_key[j] = (k >= 0 && k <= n) ? codes[k] : K(0);
+    }
+  }
+  __syncthreads();
+
+  // phase A: per chunk, E, the nearest smaller inside the chunk, and the
+  // chunk's summaries (last / first position with E below each value).  A gap
+  // of the tile whose nearest smaller gaps on both sides lie in its own chunk
+  // (about four in five on uniform keys) writes its node here, with the D of
+  // both from its neighbours' lanes; the others go to the list of phase C.
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+  static_assert(C::kKeyBytes % 4 == 0, "the masks follow the keys");
+  // the halo chunks need only E and their minimum: a lookup that ends in one
+  // scans its 32 values (phase C)
+  static_assert(2 * kAnsvHalo % NW == 0 || NW > 2 * kAnsvHalo, "whole rounds of halo chunks");
+  for (int hc = int(warp); hc < 2 * kAnsvHalo; hc += NW) {
+    const int ch = hc < kAnsvHalo ? hc : hc + tch;
+    const int w = ch * 32 + int(lane);
+    const int g = wlo + w;
+    const int e = uint32_t(g) < uint32_t(n) ? KeyTraits<K>::clz(s_key[w] ^ s_key[w + 1]) : 0;
+    s_e[w] = uint8_t(e);
+    const uint32_t cmin = __reduce_min_sync(0xffffffffu, uint32_t(e));
+    if (lane == 0) s_cmin[ch] = uint8_t(cmin);
+  }
+  // the tile's chunks two at a time per warp, so that their ballot chains
+  // interleave (one at a time where a warp has few)
+  static_assert(DYN || TCH % (JN * NW) == 0, "whole groups of chunks per warp");
+  // lane v's threshold bits as masks (all ones where v has the bit), the same
+  // for every chunk: kept in registers, since the kernel is bound by its
+  // integer instructions
+  uint32_t mlane[VB];
+#pragma unroll
+  for (int bt = 0; bt < VB; ++bt) mlane[bt] = 0u - ((lane >> bt) & 1u);
+  for (int ch0 = kAnsvHalo + int(warp); ch0 < kAnsvHalo + tch; ch0 += JN * NW) {
+    int e[JN];
+#pragma unroll
+    for (int j = 0; j < JN; ++j) {
+      const int ch = ch0 + j * NW;
+      const int w = ch * 32 + int(lane);  // window index of this lane's gap
+      const int g = wlo + w;
+      const bool real = uint32_t(g) < uint32_t(n);
+      // distinct keys whose top bit is clear: E = delta + 1 = clz of the xor,
+      // at least 1 for a real gap, so 0 marks walls only
+      e[j] = real ? KeyTraits<K>::clz(s_key[w] ^ s_key[w + 1]) : 0;
+      s_e[w] = uint8_t(e[j]);
+      const uint32_t cmin = __reduce_min_sync(0xffffffffu, uint32_t(e[j]));
+      if (lane == 0) s_cmin[ch] = uint8_t(cmin);
+    }
+    // bit-serial comparison of every lane's E against v = lane (and lane + 32
+    // for 64-bit keys): lane v ends with the lanes whose E is below v; the
+    // lanes below my own value are then lane e's result
+    // (branch-free: with m = all ones where v has the bit, a lane stays equal
+    // while its bit matches, eq &= ~(B ^ m), and falls below where v has the
+    // bit and it has not, lt |= eq & ~B & m)
+    uint32_t lt0[JN], eq0[JN];  // below v = lane
+    uint32_t lt1[JN], eq1[JN];  // below v = lane + 32
+#pragma unroll
+    for (int j = 0; j < JN; ++j) {
+      lt0[j] = lt1[j] = 0;
+      eq0[j] = eq1[j] = 0xffffffffu;
+    }
+#pragma unroll
+    for (int bt = VB - 1; bt >= 0; --bt) {
+      uint32_t B[JN];
+#pragma unroll
+      for (int j = 0; j < JN; ++j) B[j] = __ballot_sync(0xffffffffu, (e[j] >> bt) & 1);
+      // v = lane + 32 has bit 5 set and lane's bits below it
+      const uint32_t m0 = mlane[bt], m1 = bt == 5 ? 0xffffffffu : mlane[bt];
+#pragma unroll
+      for (int j = 0; j < JN; ++j) {
+        lt0[j] |= eq0[j] & ~B[j] & m0;
+        eq0[j] &= ~(B[j] ^ m0);
+        if (NV > 32) {
+          lt1[j] |= eq1[j] & ~B[j] & m1;
+          eq1[j] &= ~(B[j] ^ m1);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < JN; ++j) {
+      const int ch = ch0 + j * NW;
+      const uint32_t from0 = __shfl_sync(0xffffffffu, lt0[j], e[j] & 31);
+      const uint32_t from1 = NV > 32 ? __shfl_sync(0xffffffffu, lt1[j], e[j] & 31) : 0u;
+      const uint32_t lt = (NV > 32 && e[j] >= 32) ? from1 : from0;
+      {
+        const int tg = (ch - kAnsvHalo) * 32 + int(lane);
+        // lt never holds the lane itself; clz(0) = 32 and ffs(0) = 0 give -1
+        const uint32_t lm = lt & lanemask_lt(), rm = lt & ~lm;
+        const int lp = 31 - __clz(lm);
+        const int rp = __ffs(rm) - 1;
+        // E of the two nearest smaller lanes (a wall lane past the last gap
+        // has E = 0, so D = -1 there as for the wall at n)
+        const int el = __shfl_sync(0xffffffffu, e[j], lp & 31);
+        const int er = __shfl_sync(0xffffffffu, e[j], rp & 31);
+        const int g = g0 + tg;
+        const bool real = g < n;
+        const bool here = real && lp >= 0 && rp >= 0;
+        if (here)
+          write_gap_node_d<EDGES, LESS>(g, e[j] - 1, g - int(lane) + lp, g - int(lane) + rp, el - 1,
+                                  er - 1, root_true_delta, root_prefix, pn, l8, r8, lcs, par,
+                                  ec);
+        const uint32_t pm = __ballot_sync(0xffffffffu, real && !here);
+        if (pm) {
+          uint32_t at = 0;
+          if (lane == uint32_t(__ffs(pm) - 1)) at = atomicAdd(&sh.pend_n, uint32_t(__popc(pm)));
+          at = __shfl_sync(0xffffffffu, at, __ffs(pm) - 1) + __popc(pm & lanemask_lt());
+          if (real && !here)
+            s_pend[at] = uint32_t(tg) | uint32_t(lp & 0xff) << 16 | uint32_t(rp & 0xff) << 24;
+        }
+      }
+      // an empty mask gives 0xff (none) by itself: 31 - clz(0) = ffs(0) - 1 = -1
+      const int tc = ch - kAnsvHalo;  // the chunk's column among the tile's
+      s_last[int(lane) * C::kRow + tc] = uint8_t(31 - __clz(lt0[j]));
+      s_first[int(lane) * C::kRow + tc] = uint8_t(__ffs(lt0[j]) - 1);
+      if (NV > 32) {
+        s_last[(int(lane) + 32) * C::kRow + tc] = uint8_t(31 - __clz(lt1[j]));
+        s_first[(int(lane) + 32) * C::kRow + tc] = uint8_t(__ffs(lt1[j]) - 1);
+      }
+    }
+  }
+  __syncthreads();
+
+  // phase B: for every value v, a bitmask of the window's chunks whose
+  // minimum lies below v (bit c of word c / 32)
+  for (int v = int(warp); v < NV; v += NW) {
+#pragma unroll
+    for (int wd = 0; wd < C::MW; ++wd) {
+      const int cidx = wd * 32 + int(lane);
+      const uint32_t bits = __ballot_sync(0xffffffffu, cidx < chunks && int(s_cmin[cidx]) < v);
+      if (lane == 0) s_mask[v * C::MW + wd] = bits;
+    }
+  }
+  __syncthreads();
+
+  // phase C: every gap of the list writes its node; a gap whose nearest
+  // smaller gap lies beyond the window goes to the far-search list
+  const int wend = wlo + win - 1;  // last gap of the window
+  auto d_at = [&](int p) -> int {       // D of gap p in [0, n)
+    return (p >= wlo && p <= wend) ? int(s_e[p - wlo]) - 1 : delta(codes[p], codes[p + 1]);
+  };
+  const int np = int(sh.pend_n);
+  for (int q = int(threadIdx.x); q < np; q += NT) {
+    const uint32_t pw = s_pend[q];
+    const int tg = int(pw & 0xffffu), lp = int((pw >> 16) & 0xffu), rp = int(pw >> 24);
+    const int g = g0 + tg;
+    const int ch = kAnsvHalo + tg / 32;
+    const int e = s_e[g - wlo];
+    // not inside its own chunk: the nearest chunk on that side whose minimum
+    // is below e holds the answer in its summary
+    const int cb = wlo + ch * 32;  // first gap of this chunk
+    int L = lp != 0xff ? cb + lp : kAnsvNone;
+    if (L == kAnsvNone) {
+      for (int wd = (ch - 1) >> 5; wd >= 0; --wd) {
+        uint32_t bits = s_mask[e * C::MW + wd];
+        if (wd == (ch - 1) >> 5) bits &= 0xffffffffu >> (31 - ((ch - 1) & 31));
+        if (bits) {
+          const int c2 = wd * 32 + 31 - __clz(bits);
+          L = wlo + c2 * 32 + (c2 >= kAnsvHalo ? int(s_last[e * C::kRow + c2 - kAnsvHalo])
+                                               : chunk_last_below(s_e + c2 * 32, e));
+          break;
+        }
+      }
+    }
+    int R = rp != 0xff ? cb + rp : kAnsvNoneR;
+    if (R == kAnsvNoneR) {
+      for (int wd = (ch + 1) >> 5; wd < C::MW; ++wd) {
+        uint32_t bits = s_mask[e * C::MW + wd];
+        if (wd == (ch + 1) >> 5) bits &= 0xffffffffu << ((ch + 1) & 31);
+        if (bits) {
+          const int c2 = wd * 32 + __ffs(bits) - 1;
+          R = wlo + c2 * 32 +
+              (c2 < kAnsvHalo + tch ? int(s_first[e * C::kRow + c2 - kAnsvHalo])
+                                                : chunk_first_below(s_e + c2 * 32, e));
+          break;
+        }
+      }
+    }
+    if (L == kAnsvNone || R == kAnsvNoneR) {
+      // resolved by this block below.  The list cannot overflow: two gaps
+      // whose nearest smaller gap on the left lies beyond the window never
+      // share a value (if a < b did, every gap between them would be at least
+      // that value, so the keys a+1 .. b would all have the bit at which keys
+      // a and a+1 first differ set, while gap b needs key b to have it clear),
+      // so the tile holds at most NV such gaps, and NV more on the right
+      const uint32_t local = atomicAdd(&sh.far_n, 1u);
+      if (local < kTreeFarPerTile) sh.far[local] = uint32_t(g);
+      else atomicCAS(reinterpret_cast<int*>(err), 0, RW_ERR_CAPACITY);  // not reachable, see above
+      continue;
+    }
+    write_gap_node<K, EDGES, LESS>(g, n, e - 1, max(L, -1), min(R, n), d_at, root_true_delta,
+                             root_prefix, pn, l8, r8, lcs, par,
+                             ec);
+  }
+  __syncthreads();
+
+  // phase D: the tile's gaps whose nearest smaller gap lies beyond the
+  // window, one warp per gap (the warp-cooperative search of the keys in
+  // global memory); their latency overlaps the other resident blocks' work
+  // (with DYN node 0 too: the other blocks wait for this one at a barrier)
+  if (DYN && g0 == 0 && warp == uint32_t(NW - 1)) root_node();
+  const uint32_t nf = min(sh.far_n, kTreeFarPerTile);
+  auto d_glob = [&](int p) -> int { return delta(codes[p], codes[p + 1]); };
+  for (uint32_t f = warp; f < nf; f += NW) {
+    const int g = int(sh.far[f]);
+    const int D = delta(codes[g], codes[g + 1]);
+    int first_key, last_key;
+    coop_node_keys<K>(codes, n, g, D, &first_key, &last_key);
+    if (lane == 0)
+      write_gap_node<K, EDGES, LESS>(g, n, D, first_key - 1, last_key, d_glob, root_true_delta,
+                               root_prefix, pn, l8, r8, lcs, par,
+                               ec);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// stage 7: octree rows and links (func_octree.hpp:28-112)
+// ---------------------------------------------------------------------------
+
+struct OctOut {
+  int32_t* children;
+  float4* corner;
+  float* cell_size;
+  int32_t* node_mask;
+  int32_t* leaf_mask;
+  const uint32_t* oct_off;  // [segments + 1] row offsets; null with one segment
+  uint32_t capacity;        // rows with one segment
+};
+
+struct OctSeg {
+  uint32_t row0, cap, m;
+  int n;        // radix-tree nodes
+  bool counts;  // the counts are valid (the edge offsets can be made)
+  bool ok;      // ... and the octree fits its rows
+};
+
+// The segment's octree rows and counts; reports a too small octree.
+__device__ __forceinline__ OctSeg oct_segment(const SegTable& seg, const OctOut& o,
+                                              const uint32_t* n_unique,
+                                              const uint32_t* n_octree, int32_t* seg_err,
+                                              uint32_t c, bool report) {
+  OctSeg r{};
+  const uint32_t nu = *reinterpret_cast<const volatile uint32_t*>(n_unique + c);
+  r.ok = nu >= 3 && nu != RW_COUNT_UNSET && nu <= seg_size(seg, c);
+  if (!r.ok) return r;
+  r.n = int(nu - 1);
+  r.m = *reinterpret_cast<const volatile uint32_t*>(n_octree + c);
+  r.row0 = o.oct_off ? o.oct_off[c] : 0u;
+  r.cap = o.oct_off ? o.oct_off[c + 1] - o.oct_off[c] : o.capacity;
+  r.counts = true;
+  if (uint64_t(r.m) + 1 > r.cap) {
+    if (report) seg_error(seg_err, c, RW_ERR_CAPACITY);
+    r.ok = false;
+  }
+  return r;
+}
+
+// Nearest ancestor of node c that owns rows: parents are followed while the
+// count is zero, at most 31 steps as in the reference (func_octree.hpp:80-92).
+// Returns -1 when a parent index is outside [0, n).
+__device__ __forceinline__ int link_parent(const int32_t* __restrict__ parents,
+                                           const int32_t* __restrict__ ec, int c, int n) {
+  int rp = parents[c];
+  if (uint32_t(rp) >= uint32_t(n)) return -1;
+  int counter = 0;
+  while (ec[rp] == 0) {
+    rp = parents[rp];
+    if (uint32_t(rp) >= uint32_t(n)) return -1;
+    if (++counter > 30) break;
+  }
+  return rp;
+}
+
+// The link of node c (count cnt > 0) into the global rows: child slot of the
+// chain's top row (level prefix_n[c] / 3 - cnt + 1) in row offset[rp]
+// (func_octree.hpp:94-102).  The reference overwrites in ascending node
+// order; the value off[c] + cnt - 1 grows with c, so the maximum is the last
+// write.
+template <typename K>
+__device__ __forceinline__ void link_global(const K* __restrict__ codes,
+                                            const uint8_t* __restrict__ prefix_n,
+                                            const int32_t* __restrict__ off, int c, int cnt,
+                                            int rp, const OctSeg& os, const OctOut& o) {
+  constexpr int B = KeyTraits<K>::kCodeBits;
+  const int oct_parent = off[rp];
+  const int top = prefix_n[c] / 3 - cnt + 1;
+  const int slot = int((codes[c] >> (B - 3 * top)) & K(7));
+  if (uint32_t(oct_parent) < os.cap) {
+    const size_t r = size_t(os.row0) + uint32_t(oct_parent);
+    atomicMax(o.children + 8 * r + slot, off[c] + cnt - 1);
+    atomicOr(o.node_mask + r, 1 << slot);
+  }
+}
+
+// A far link (16 bytes): segment, node, kind << 30 | counter << 3 | slot,
+// link value.  kFarFromParent: the walk starts at parents[node] (node = the
+// linking node); kFarFromStep: node is the last ancestor reached inside the
+// tile, count 0, the walk continues at parents[node] with counter + 1;
+// kFarFinal: node is the ancestor whose row takes the link.  kFarLocal is
+// used inside k_octree only.
+constexpr uint32_t kFarFromParent = 0, kFarFromStep = 1, kFarFinal = 2, kFarLocal = 3;
+
+// Stage 7 in one pass over a tile of radix-tree nodes (func_octree.hpp:28-112).
+//
+// Rows [off[i], off[i] + cnt[i]) belong to node i (i >= 1); the offsets are
+// an exclusive scan of non-negative counts, so a tile of nodes owns one
+// contiguous run of rows, and the owner of row p is the last node whose
+// first row is <= p.  Row off+k sits at level L - k (L = prefix_n[i] / 3);
+// for k > 0 its one child is the chain row off+k-1 (func_octree.hpp:56-78).
+// A row with k = 0 gets its children only from links: the chain's top row
+// p = off[c] + cnt[c] - 1 of node c is named in row off[rp] of c's nearest
+// ancestor rp that owns rows (func_octree.hpp:80-111).  When rp lies in the
+// tile and owns rows, that row is a k = 0 row of the tile: the link is
+// merged in shared memory and every row is written once, complete.  Other
+// links go to the far list (node, segment), applied after this kernel with
+// global atomics; a list that overflows makes the far kernel apply every
+// link again (the atomics are idempotent).
+//
+// Threads take the tile's rows in turn (row r by thread r mod threads), so
+// that every lane has a row; the owner comes from a binary search over the
+// tile's first rows.
+//
+// Node 0 owns no row; tile 0 writes the root initialisation when there is
+// no octree row at all (07_octree.cu:188-198) and clears the spare row m
+// that a link may name.
+//
+// With OFFS the offsets are not read but made here (stage 6's write folded
+// into stage 7): tile_prefix holds the exclusive scan of every tile's count
+// sum (k_node_sums, k_tile_scan), the block scans its tile's counts on top
+// of it and writes them to off_all.
+template <typename K>
+struct OctTileShared {
+  // k = 0 row of each node: child slot values relative to the tile's first
+  // row, plus one (0: no child; the nonzero slots are the node mask)
+  uint4 child[kOctTile];  // 8 x u16
+  K code[kOctTile];
+  // first row of each node relative to the tile's first row (a tile's rows
+  // number at most kTile times the largest count, 21 levels; 0xffff past the
+  // tile's nodes); [kOctTile]: end of the tile's rows
+  uint16_t off[kOctTile + 2];
+  // per node: (count class << 12) | tile-relative parent (0xfff: outside);
+  // class 0: count 0, 1: count > 0, 2: count < 0
+  uint16_t node[kOctTile];
+  uint16_t owner[kOctTile];  // of the first rows
+  uint8_t level[kOctTile];   // prefix_n / 3
+  uint32_t wsum[4 * (kOctThreads / 32) + 1];
+};
+
+// The tile of nodes from tile0 on, of a segment os (number c) whose arrays are
+// given, by kOctThreads threads (tid) that sync() synchronises.  first_row():
+// the tile's first row, with OFFS.
+template <typename K, bool OFFS, typename Sync, typename FirstRow>
+__device__ __forceinline__ void octree_tile(
+    OctTileShared<K>& sh, const Sync& sync, int tid, const K* __restrict__ codes,
+    const uint8_t* __restrict__ prefix_n, const int32_t* __restrict__ parents,
+    const int32_t* __restrict__ ec, int32_t* __restrict__ off, const OctSeg& os, uint32_t c,
+    int tile0, const FirstRow& first_row, float min_coord, float range, const OctOut& o,
+    uint32_t* __restrict__ far, uint32_t far_cap, uint32_t* __restrict__ far_n) {
+  constexpr int B = KeyTraits<K>::kCodeBits;
+  constexpr int kTile = int(kOctTile);
+  constexpr int kRowCap = kTile;  // rows whose owner is kept
+  static_assert(kTile < 0xfff && (kTile & (kTile - 1)) == 0, "12-bit parents, 2^k tile");
+  static_assert(kTile == 4 * kOctThreads && 4 * (kOctThreads / 32) == 32,
+                "four groups of 256 nodes, 32 warp sums");
+  const int n = os.n;
+  const uint32_t m = os.m;
+  const int tile_end = min(tile0 + kTile, n);
+
+  // thread tid: nodes tile0 + tid + 256 q, q < 4 (coalesced loads)
+  int ev[4], ov[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int t = tid + q * kOctThreads;
+    const int i = tile0 + t;
+    const bool valid = i < tile_end;
+    ev[q] = valid ? ec[i] : 0;
+    const int pa = valid ? parents[i] : -1;
+    const int pr = pa >= tile0 && pa < tile_end ? pa - tile0 : 0xfff;
+    sh.node[t] = uint16_t((ev[q] == 0 ? 0 : ev[q] > 0 ? 1 : 2) << 12 | pr);
+    ov[q] = (!OFFS && valid) ? off[i] : 0;
+    sh.code[t] = valid ? codes[i] : K(0);
+    sh.level[t] = valid ? uint8_t(prefix_n[i] / 3) : uint8_t(0);
+    sh.child[t] = make_uint4(0, 0, 0, 0);
+  }
+  uint32_t rows_end = 0;
+  int rbase = 0;  // the tile's first row
+  if (OFFS) {
+    // exclusive scan of the counts in node order, as stage 6 computes it: a
+    // warp scan per group of 32 nodes, then one warp scans the 32 group sums
+    const uint32_t lane = lane_id(), warp = uint32_t(tid) >> 5;
+    uint32_t inc[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      inc[q] = warp_inclusive_scan(uint32_t(ev[q]));
+      if (lane == 31) sh.wsum[q * (kOctThreads / 32) + warp] = inc[q];
+    }
+    sync();
+    if (warp == 0) {
+      const uint32_t v = sh.wsum[lane];
+      const uint32_t wi = warp_inclusive_scan(v);
+      sh.wsum[lane] = wi - v;
+      if (lane == 31) sh.wsum[32] = wi;
+    }
+    sync();
+    const uint32_t base = first_row();
+    rbase = int(base);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      ov[q] = int32_t(base + sh.wsum[q * (kOctThreads / 32) + warp] + inc[q] - uint32_t(ev[q]));
+      const int i = tile0 + tid + q * kOctThreads;
+      if (i < tile_end) off[i] = ov[q];
+    }
+    rows_end = base + sh.wsum[32];
+  } else {
+    rbase = off[tile0];
+  }
+  if (!os.ok) return;  // the whole block: no octree row is written
+  // relative rows kept in [0, 0xfffe] (offsets made by stage 6 stay far inside)
+  auto rel16 = [&](int v) -> uint16_t { return uint16_t(min(max(v - rbase, 0), 0xfffe)); };
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int t = tid + q * kOctThreads;
+    sh.off[t] = tile0 + t < tile_end ? rel16(ov[q]) : uint16_t(0xffff);
+  }
+  if (tid == 0) {
+    sh.off[kTile] = rel16(OFFS ? int(rows_end) : (tile_end < n ? off[tile_end] : int(m)));
+    if (tile0 == 0) {
+      const size_t rm = size_t(os.row0) + m;
+      int4* row = reinterpret_cast<int4*>(o.children + 8 * rm);
+      row[0] = make_int4(0, 0, 0, 0);
+      row[1] = make_int4(0, 0, 0, 0);
+      o.node_mask[rm] = 0;
+      o.leaf_mask[rm] = 0;
+      if (m == 0) {
+        const int root_level = prefix_n[0] / 3;
+        const K pre = codes[0] >> (B - 3 * root_level);
+        o.corner[os.row0] = decode<K>(K(pre << (B - 3 * root_level)), min_coord, range);
+        o.cell_size[os.row0] = range;
+      }
+    }
+  }
+  sync();
+  if (tile_end < tile0 + kTile && tid == 0) sh.off[tile_end - tile0] = sh.off[kTile];
+  sync();
+
+  const int rend = min(rbase + int(sh.off[kTile]), int(m));  // rows [rbase, rend)
+  const int root_level = prefix_n[0] / 3;
+  auto owner_of = [&](int r) -> int {  // last node whose first row is <= rbase + r
+    int t = 0;
+#pragma unroll
+    for (int step = kTile / 2; step >= 1; step >>= 1)
+      if (int(sh.off[t + step]) <= r) t += step;
+    return t;
+  };
+
+  // links, from the chain top rows; the walk of link_parent over the tile's
+  // counts and parents.  A walk that leaves the tile, ends on a node without
+  // rows or gives up, and a value that does not fit 16 bits, go to the far
+  // list with the walk's state (FarLink), where k_octree_far_links finishes
+  // the walk in global memory and merges with atomics.  Several links may
+  // name one slot (the reference keeps the last, the largest value): the
+  // 16-bit maximum is taken with compare-and-swap on the slot's word.
+  for (int r = tid; rbase + r < rend; r += kOctThreads) {
+    const int p = rbase + r;
+    const int t = owner_of(r);
+    if (r < kRowCap) sh.owner[r] = uint16_t(t);
+    if (r != int(sh.off[t + 1]) - 1) continue;  // not the top row of its chain
+    const int level = int(sh.level[t]) - (r - int(sh.off[t]));  // the top row's level
+    const int slot = int((sh.code[t] >> (B - 3 * level)) & K(7));
+    int rp = int(sh.node[t] & 0xfffu), counter = 0, x = t;
+    uint32_t kind = kFarFromParent;
+    if (rp != 0xfff) {
+      for (;;) {
+        const uint32_t w = sh.node[rp];
+        if (w >> 12) {
+          kind = (w >> 12) == 1 ? kFarLocal : kFarFinal;
+          break;
+        }
+        const int nx = int(w & 0xfffu);
+        if (nx == 0xfff) {  // the parent lies outside the tile
+          kind = kFarFromStep;
+          x = rp;
+          break;
+        }
+        rp = nx;
+        if (++counter > 30) {
+          kind = kFarFinal;
+          break;
+        }
+      }
+    }
+    if (kind == kFarLocal) {
+      bool done = false;
+      if (r < 0xffff) {
+        uint32_t* wp = reinterpret_cast<uint32_t*>(&sh.child[rp]) + (slot >> 1);
+        const int sh = 16 * (slot & 1);
+        const uint32_t rel = uint32_t(r) + 1u;  // the link value is p itself
+        uint32_t cur = *reinterpret_cast<volatile uint32_t*>(wp);
+        for (int tries = 0; tries < 64 && !done; ++tries) {  // each failure is another's success
+          if (((cur >> sh) & 0xffffu) >= rel) {
+            done = true;
+          } else {
+            const uint32_t nv = (cur & ~(0xffffu << sh)) | (rel << sh);
+            const uint32_t prev = atomicCAS(wp, cur, nv);
+            done = prev == cur;
+            cur = prev;
+          }
+        }
+      }
+      if (done) continue;
+      kind = kFarFinal;
+    }
+    const uint32_t at = atomicAdd(far_n, 1u);
+    if (at < far_cap) {
+      const int node = kind == kFarFinal ? tile0 + rp : tile0 + x;
+      reinterpret_cast<uint4*>(far)[at] =
+          make_uint4(c, uint32_t(node), kind << 30 | uint32_t(counter) << 3 | uint32_t(slot),
+                     uint32_t(p));
+    }
+  }
+  sync();
+
+  // rows
+  for (int r = tid; rbase + r < rend; r += kOctThreads) {
+    const int p = rbase + r;
+    const int t = r < kRowCap ? int(sh.owner[r]) : owner_of(r);
+    const size_t rp = size_t(os.row0) + uint32_t(p);
+    const int k = r - int(sh.off[t]);
+    const int level = int(sh.level[t]) - k;
+    const K code = sh.code[t];
+    const K pre = code >> (B - 3 * level);
+    o.corner[rp] = decode<K>(K(pre << (B - 3 * level)), min_coord, range);
+    // range / 2^s, s = level - root_level in [0, 21]: the product with the
+    // exact reciprocal 2^-s is the same correctly rounded value
+    o.cell_size[rp] =
+        __fmul_rn(range, __uint_as_float(uint32_t(127 - (level - root_level)) << 23));
+    int4* row = reinterpret_cast<int4*>(o.children + 8 * rp);
+    if (k == 0) {
+      const uint4 a = sh.child[t];
+      const uint32_t wv[4] = {a.x, a.y, a.z, a.w};
+      int32_t child[8];
+      uint32_t mask = 0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const uint32_t v = (wv[q >> 1] >> (16 * (q & 1))) & 0xffffu;
+        child[q] = v ? int32_t(v) - 1 + rbase : 0;
+        mask |= uint32_t(v != 0) << q;
+      }
+      row[0] = make_int4(child[0], child[1], child[2], child[3]);
+      row[1] = make_int4(child[4], child[5], child[6], child[7]);
+      o.node_mask[rp] = int32_t(mask);
+    } else {
+      int32_t child[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      const int slot = int((code >> (B - 3 * (level + 1))) & K(7));
+      child[slot] = p - 1;
+      row[0] = make_int4(child[0], child[1], child[2], child[3]);
+      row[1] = make_int4(child[4], child[5], child[6], child[7]);
+      o.node_mask[rp] = 1 << slot;
+    }
+    o.leaf_mask[rp] = 0;
+  }
+}
+
+// Links that k_octree left to the far list, with global atomics; when the
+// list overflowed, every node's link again (blocks stride over all tiles).
+template <typename K>
+__device__ __forceinline__ void octree_far_links(
+    const K* __restrict__ codes_all, const uint8_t* __restrict__ prefix_all,
+    const int32_t* __restrict__ parents_all, const int32_t* __restrict__ ec_all,
+    const int32_t* __restrict__ off_all, const SegTable& seg, const TileMap& map,
+    const uint32_t* __restrict__ n_unique, const uint32_t* __restrict__ n_octree,
+    int32_t* __restrict__ seg_err, const OctOut& o, const uint32_t* __restrict__ far,
+    uint32_t far_cap, const uint32_t* __restrict__ far_n) {
+  const uint32_t count = *far_n;
+  if (count <= far_cap) {
+    for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < count;
+         w += gridDim.x * blockDim.x) {
+      // the walk is a chain of dependent loads: every step loads the count,
+      // the parent and the offset of its node together, and the first step
+      // goes out with the segment's counts (k_octree wrote only nodes of the
+      // segment, in [0, n), into the list)
+      const uint4 f = reinterpret_cast<const uint4*>(far)[w];
+      const uint32_t c = f.x, kind = f.z >> 30, slot = f.z & 7u;
+      const uint32_t sb = seg_begin(seg, c);
+      const int32_t* parents = parents_all + sb;
+      const int32_t* ec = ec_all + sb;
+      const int32_t* off = off_all + sb;
+      int rp = int(f.y);
+      const int first = kind != kFarFinal ? parents[rp] : rp;
+      const OctSeg os = oct_segment(seg, o, n_unique, n_octree, seg_err, c, false);
+      if (!os.ok) continue;
+      const int n = os.n;
+      int oct_parent;
+      if (kind != kFarFinal) {  // the rest of link_parent's walk
+        int counter = int((f.z >> 3) & 31u);
+        rp = first;
+        if (uint32_t(rp) >= uint32_t(n)) continue;
+        bool stop = kind == kFarFromStep && ++counter > 30;
+        int cnt = ec[rp], par = parents[rp];
+        oct_parent = off[rp];
+        while (!stop && cnt == 0) {
+          rp = par;
+          if (uint32_t(rp) >= uint32_t(n)) break;
+          stop = ++counter > 30;
+          cnt = ec[rp];
+          par = parents[rp];
+          oct_parent = off[rp];
+        }
+        if (uint32_t(rp) >= uint32_t(n)) continue;
+      } else {
+        oct_parent = off[rp];
+      }
+      if (uint32_t(oct_parent) < os.cap) {
+        const size_t r = size_t(os.row0) + uint32_t(oct_parent);
+        atomicMax(o.children + 8 * r + slot, int32_t(f.w));
+        atomicOr(o.node_mask + r, 1 << slot);
+      }
+    }
+    return;
+  }
+  for (uint32_t tile = blockIdx.x; tile < map.n_tiles; tile += gridDim.x) {
+    uint32_t first;
+    const uint32_t c = tile_segment(seg, map, tile, &first);
+    const OctSeg os = oct_segment(seg, o, n_unique, n_octree, seg_err, c, false);
+    if (!os.ok) continue;
+    const uint32_t sb = seg_begin(seg, c);
+    const int32_t* ec = ec_all + sb;
+    const int base = int(tile - first) * int(kOctTile);
+    for (int q = int(threadIdx.x); q < int(kOctTile); q += int(blockDim.x)) {
+      const int i = base + q;
+      if (i >= os.n) break;
+      if (i == 0) continue;
+      const int cnt = ec[i];
+      if (cnt <= 0) continue;
+      const int rp = link_parent(parents_all + sb, ec, i, os.n);
+      if (rp < 0) continue;
+      link_global<K>(codes_all + sb, prefix_all + sb, off_all + sb, i, cnt, rp, os, o);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// leaf links (rw_tree_im_storage_set_options)
+// ---------------------------------------------------------------------------
+
+// RW_TREE_OPT_LINK_LEAVES: process_link_leaf (func_octree.hpp:114-163) for
+// every radix-tree node, as if run in ascending order after stage 7.  Leaf
+// `side` of node i goes to slot (leaf code at level prefix_n[i]/3 + 1) & 7 of
+// the bottom octree row of the nearest ancestor-or-self with octree rows.
+// The walk stops after 31 steps (the reference CPU walk has no bound and
+// never ends at a root without rows; its CUDA left-leaf walk stops there),
+// and a negative level shift (32-bit keys, prefix_n = 30) is taken modulo
+// the word width, as an x86 build of the reference does.  Returns false when
+// the node has no such leaf or the row is out of range.
+template <typename K>
+__device__ __forceinline__ bool leaf_target(int i, int side, int n, const K* __restrict__ codes,
+                                            const uint8_t* __restrict__ pn,
+                                            const uint8_t* __restrict__ hl,
+                                            const uint8_t* __restrict__ hr,
+                                            const int32_t* __restrict__ lc,
+                                            const int32_t* __restrict__ par,
+                                            const int32_t* __restrict__ ec,
+                                            const int32_t* __restrict__ off, uint32_t rows,
+                                            uint32_t* slot, int* leaf) {
+  if (!(side ? hr[i] : hl[i])) return false;
+  constexpr int B = KeyTraits<K>::kCodeBits, W = KeyTraits<K>::kWordBits;
+  const int lf = min(max(lc[i] + side, 0), n);  // keys are [0, n]
+  const int level = pn[i] / 3 + 1;
+  const uint32_t which = uint32_t(codes[lf] >> ((B - 3 * level) & (W - 1))) & 7u;
+  int rt = i;
+  for (int step = 0; step < 31 && ec[rt] == 0; ++step) {
+    const int p = par[rt];
+    rt = uint32_t(p) < uint32_t(n) ? p : 0;
+  }
+  const int bottom = off[rt];
+  if (uint32_t(bottom) >= rows) return false;
+  *slot = uint32_t(bottom) * 8u + which;
+  *leaf = lf;
+  return true;
+}
+
+// Pass 1: every writer claims its slot with atomicMin of -(2 i + side) - 2,
+// so the slot ends holding the claim of the last writer in sequential order
+// (claims are negative, the rows' node links are not); set_leaf's clear of
+// the leaf-mask bit commutes and is applied here.
+template <typename K>
+__device__ __forceinline__ void leaf_claim(const K* __restrict__ codes, const uint8_t* __restrict__ pn,
+                 const uint8_t* __restrict__ hl, const uint8_t* __restrict__ hr,
+                 const int32_t* __restrict__ lc, const int32_t* __restrict__ par,
+                 const int32_t* __restrict__ ec, const int32_t* __restrict__ off,
+                 int32_t* __restrict__ children, int32_t* __restrict__ leaf_mask,
+                 const uint32_t* __restrict__ n_unique, uint32_t rows) {
+  const uint32_t nu = *n_unique;
+  if (nu < 3 || nu == RW_COUNT_UNSET) return;
+  const int n = int(nu - 1);
+  for (int i = int(blockIdx.x * blockDim.x + threadIdx.x); i < n; i += int(gridDim.x * blockDim.x))
+    for (int side = 0; side < 2; ++side) {
+      uint32_t slot;
+      int leaf;
+      if (!leaf_target<K>(i, side, n, codes, pn, hl, hr, lc, par, ec, off, rows, &slot, &leaf))
+        continue;
+      atomicMin(children + slot, int(-(int64_t(2 * i + side) + 2)));
+      atomicAnd(leaf_mask + slot / 8u, ~(1 << (slot & 7u)));
+    }
+}
+
+// Pass 2: the writer whose claim survived stores its leaf index.
+template <typename K>
+__device__ __forceinline__ void leaf_write(const K* __restrict__ codes, const uint8_t* __restrict__ pn,
+                 const uint8_t* __restrict__ hl, const uint8_t* __restrict__ hr,
+                 const int32_t* __restrict__ lc, const int32_t* __restrict__ par,
+                 const int32_t* __restrict__ ec, const int32_t* __restrict__ off,
+                 int32_t* __restrict__ children, const uint32_t* __restrict__ n_unique,
+                 uint32_t rows) {
+  const uint32_t nu = *n_unique;
+  if (nu < 3 || nu == RW_COUNT_UNSET) return;
+  const int n = int(nu - 1);
+  for (int i = int(blockIdx.x * blockDim.x + threadIdx.x); i < n; i += int(gridDim.x * blockDim.x))
+    for (int side = 0; side < 2; ++side) {
+      uint32_t slot;
+      int leaf;
+      if (!leaf_target<K>(i, side, n, codes, pn, hl, hr, lc, par, ec, off, rows, &slot, &leaf))
+        continue;
+      // a loser reads the winner's claim or its leaf index, never its own claim
+      if (children[slot] == int(-(int64_t(2 * i + side) + 2))) children[slot] = leaf;
+    }
+}
+
+}  // namespace rwt
