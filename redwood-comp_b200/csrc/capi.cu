@@ -244,16 +244,28 @@ int rw_tree_im_storage_create_ex(uint32_t n_input, int32_t key_bits,
   const size_t st_b = align(sizeof(rwt::DevStatus));
   im->zero_bytes = ghist_b + skew_b + sdesc_b + udesc_b + cdesc_b + ctr_b + st_b;
 
-  cudaError_t e = cudaMalloc(&im->d_zero, im->zero_bytes);
-  if (e == cudaSuccess) e = cudaMalloc(&im->d_tmp_keys, key_size(key_bits) * n_input);
+  // one allocation: the zero region, the ping-pong keys (and, behind the keys
+  // of a small cloud, the scratch of its one-launch pipeline), the far list
+  bool small = false;
+  cudaError_t e = im->radix_bits == 8 ? rwt::small_prepare(key_bits, &small) : cudaSuccess;
+  const size_t small_at =
+      align(key_size(key_bits) * std::min(n_input, rwt::small_limit(key_bits)));
+  size_t keys_b = key_size(key_bits) * n_input;
+  if (small)
+    keys_b = std::max(keys_b, small_at + rwt::small_scratch_bytes(n_input, key_bits, sms));
+  keys_b = align(keys_b);
   im->tree_far_cap = rwt::div_up(n_input, rwt::kTreeTile) * rwt::kTreeFarPerTile;
-  if (e == cudaSuccess) e = cudaMalloc(&im->d_tree_far, size_t(im->tree_far_cap) * 16);
+  if (e == cudaSuccess)
+    e = cudaMalloc(&im->d_zero, im->zero_bytes + keys_b + size_t(im->tree_far_cap) * 16);
   if (e == cudaSuccess) e = cudaMallocHost(&im->h_status, sizeof(rwt::DevStatus));
   if (e != cudaSuccess) {
     rw_tree_im_storage_destroy(im);
     return cuda_fail(e, "rw_tree_im_storage_create");
   }
   char* z = static_cast<char*>(im->d_zero);
+  im->d_tmp_keys = z + im->zero_bytes;
+  if (small) im->d_small = z + im->zero_bytes + small_at;
+  im->d_tree_far = reinterpret_cast<uint32_t*>(z + im->zero_bytes + keys_b);
   size_t o = 0;
   im->d_ghist = reinterpret_cast<uint32_t*>(z + o); o += ghist_b;
   im->d_skew = reinterpret_cast<uint32_t*>(z + o); o += skew_b;
@@ -303,8 +315,6 @@ int rw_tree_im_storage_set_options(rw_tree_im_storage* im, int32_t options) {
 int rw_tree_im_storage_destroy(rw_tree_im_storage* im) {
   if (!im) return RW_OK;
   if (im->d_zero) cudaFree(im->d_zero);
-  if (im->d_tmp_keys) cudaFree(im->d_tmp_keys);
-  if (im->d_tree_far) cudaFree(im->d_tree_far);
   if (im->h_status) cudaFreeHost(im->h_status);
   delete im;
   return RW_OK;
@@ -482,11 +492,27 @@ int rw_tree_run_stage7(rw_tree_app_data* app, rw_tree_im_storage* im,
 // ---- fused pipeline ----------------------------------------------------------
 namespace {
 
+// The one-launch pipeline takes a small cloud unless the caller chose how
+// stage 2 sorts (a learned sort, another digit width or another variant).
+bool takes_small(const rw_tree_app_data* app, const rw_tree_im_storage* im) {
+  return im->d_small && !im->learned &&
+         im->sort_variant == rwt::default_sort_variant(im->key_bits, im->radix_bits) &&
+         rwt::small_takes(app->n_input, im->key_bits, im->num_sms);
+}
+
 // Enqueues the fused pipeline.  When `ev` is given, an event is recorded
-// before the first launch and after every kernel launch (profiling only).
+// before the first launch and after every kernel launch (profiling only; it
+// takes the general chain of kernels, whose names it reports).
 int enqueue_impl(rw_tree_app_data* app, rw_tree_im_storage* im, cudaStream_t s,
                  cudaEvent_t* ev, int* n_ev) {
   if (int rc = check(app, im, kPoints | kKeys | kAlt | kBrt | kEdge | kOct)) return rc;
+  if (!ev && takes_small(app, im)) {
+    RW_CUDA(rwt::launch_small(bufs_of(*app, im), scratch_of(im), app->n_input, im->n_cap,
+                              app->oct_capacity, geometric_delta(im),
+                              (im->options & RW_TREE_OPT_LINK_LEAVES) != 0, im->d_small,
+                              im->d_tile_ctr + rwt::kCtrSmall, im->h_status, s));
+    return RW_OK;
+  }
   int k = 0;
   auto mark = [&]() -> cudaError_t {
     return ev ? cudaEventRecord(ev[k++], s) : cudaSuccess;
@@ -602,6 +628,8 @@ int rw_tree_pipeline_finish(rw_tree_app_data* app, rw_tree_im_storage* im,
     std::snprintf(buf, sizeof buf, "device error %d at site %u", st.err, st.err_site);
     g_last_error = buf;
     if (st.err != RW_ERR_DEGENERATE) app->n_octree_nodes = st.n_octree_nodes;
+    if (st.err == RW_ERR_TIMEOUT)  // leave the scratch fit for the next run
+      if (int rc = clear_all(im, reinterpret_cast<cudaStream_t>(stream))) return rc;
     return st.err;
   }
   app->n_octree_nodes = st.n_octree_nodes;

@@ -29,7 +29,8 @@ enum : uint32_t {
   kSiteUnique = 2,
   kSiteScan = 3,
   kSiteTree = 4,
-  kSiteOctree = 5
+  kSiteOctree = 5,
+  kSiteSmall = 6
 };
 
 // ~1 s of polling with back-off before a wait gives up.
@@ -38,6 +39,12 @@ constexpr uint32_t kSpinLimit = 1u << 21;
 __device__ __forceinline__ uint32_t ld_relaxed(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 

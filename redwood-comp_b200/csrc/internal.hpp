@@ -43,6 +43,10 @@ struct rw_tree_im_storage {
 
   rwt::DevStatus* h_status = nullptr;  // pinned mirror
 
+  // scratch of the one-launch pipeline of small clouds (inside d_tmp_keys, which
+  // no cloud of that size fills); null when the device cannot hold its blocks
+  char* d_small = nullptr;
+
   // optional learned-CDF sort for stage 2 (32-bit keys); not owned
   rw_tree_learned* learned = nullptr;
   int32_t learned_mode = 0;
@@ -55,7 +59,7 @@ struct rw_tree_im_storage {
 namespace rwt {
 
 enum : int { kCtrUnique = 0, kCtrScan = 1, kCtrTree = 2, kCtrLinks = 3, kCtrSortBase = 4,
-             kCtrSortClassStride = 8, kMaxSortClasses = 4, kCounters = 64 };
+             kCtrSortClassStride = 8, kMaxSortClasses = 4, kCtrSmall = 48, kCounters = 64 };
 
 // Tile sizes of the kernels (points or nodes per tile).
 constexpr uint32_t kPointTile = 4096;  // Morton / histogram
@@ -212,6 +216,25 @@ cudaError_t launch_octree(const Bufs& b, const Scratch& sc, const Plan& pl, cuda
 // The leaf links after stage 7 (RW_TREE_OPT_LINK_LEAVES), single cloud only.
 cudaError_t launch_leaf_links(const Bufs& b, const Scratch& sc, const Plan& pl,
                               cudaStream_t s);
+
+// ---- a small cloud's whole pipeline in one launch (k_small.cu) ----------------
+// It takes clouds up to these sizes, where a bucket still has room for 2.4
+// shares of 148 blocks; it is faster than the general chain of kernels up to
+// there (750,000 points 106 against 134 us, 32-bit keys; 400,000 points 96
+// against 155 us, 64-bit keys).
+constexpr uint32_t kSmallLimit32 = 880000, kSmallLimit64 = 440000;
+// Sets the kernels up on the current device; *usable: a block of them fits an SM.
+cudaError_t small_prepare(int key_bits, bool* usable);
+uint32_t small_limit(int key_bits);
+bool small_takes(uint32_t n, int key_bits, int sms);
+size_t small_scratch_bytes(uint32_t n_cap, int key_bits, int sms);
+// All seven stages for n points: `scratch` of small_scratch_bytes(n_cap),
+// `sync` three zeroed words that only these launches and a clear change.  The
+// counts and the first error go to sc.status and, at the end, to host_status
+// (pinned).
+cudaError_t launch_small(const Bufs& b, const Scratch& sc, uint32_t n, uint32_t n_cap,
+                         uint32_t oct_capacity, bool geometric, bool leaves, char* scratch,
+                         uint32_t* sync, DevStatus* host_status, cudaStream_t s);
 
 // Text returned by rw_tree_last_error (this thread).
 void set_last_error(const std::string& msg);
