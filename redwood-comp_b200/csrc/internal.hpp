@@ -220,7 +220,7 @@ cudaError_t launch_leaf_links(const Bufs& b, const Scratch& sc, const Plan& pl,
 // ---- a small cloud's whole pipeline in one launch (k_small.cu) ----------------
 // It takes clouds up to these sizes, where a bucket still has room for 2.4
 // shares of 148 blocks; it is faster than the general chain of kernels up to
-// there (750,000 points 106 against 134 us, 32-bit keys; 400,000 points 96
+// there (750,000 points 103 against 134 us, 32-bit keys; 400,000 points 82
 // against 155 us, 64-bit keys).
 constexpr uint32_t kSmallLimit32 = 880000, kSmallLimit64 = 440000;
 // Sets the kernels up on the current device; *usable: a block of them fits an SM.

@@ -7,9 +7,9 @@
 // block of 1,024 threads per SM keeps its share of the keys in shared memory,
 // and the steps are separated by barriers over the grid (1.3 us each, 2.3 with
 // stores to drain; none when one block takes the cloud).  A call with its wait,
-// before and now, 32-bit keys: 2,000 points 100 and 45 us, 4,096 100 and 57,
-// 20,000 100 and 61, 307,200 111 and 73, 600,000 128 and 86; 64-bit keys: 4,200
-// points 123 and 70 us, 303,104 143 and 88, 400,000 155 and 96.  What is left is
+// before and now, 32-bit keys: 2,000 points 100 and 43 us, 4,096 100 and 54,
+// 20,000 100 and 57, 303,104 110 and 71, 600,000 126 and 85; 64-bit keys: 4,200
+// points 123 and 58 us, 303,104 143 and 77, 400,000 155 and 82.  What is left is
 // latency: eight barriers, and chains of dependent shared-memory and L2
 // accesses in every step.
 //
@@ -188,6 +188,15 @@ __device__ __forceinline__ void block_digit_pass(const K* a, K* b, int steps, in
 // Sorts a block's c keys in `a` (with `b` as the other half); returns where
 // they end.  Digits that all keys share are left out.  The keys are filled up
 // to whole steps with the largest word, which stays behind them.
+//
+// A few thousand keys rarely share the first kSortBits bits of those in which
+// they differ: only these are sorted by digits (three passes instead of four
+// to eight, 2.1 us each), then every key of a run that shares them finds its
+// place by counting the run's smaller keys: 64-bit keys, 3,001 points 20.0 ->
+// 9.0 us of sorting, 307,200 points 20.2 -> 10.1.  A run beyond kSortRun keys
+// sends the block through all digits.
+constexpr int kSortBits = 24, kSortRun = 32;
+
 template <typename K>
 __device__ K* block_sort(K* a, K* b, int c, uint32_t* hist, uint32_t* next, SmallShared& sh) {
   constexpr int kBits = KeyTraits<K>::kCodeBits;
@@ -210,18 +219,31 @@ __device__ K* block_sort(K* a, K* b, int c, uint32_t* hist, uint32_t* next, Smal
   }
   __syncthreads();
   const K all = sizeof(K) == 8 ? K(uint64_t(sh.diff[1]) << 32 | sh.diff[0]) : K(sh.diff[0]);
-  for (int shift = 0; shift < kBits && (all >> shift); shift += 8) {
-    if (((all >> shift) & K(255)) == 0) continue;
-    if (threadIdx.x < kSortThreads) block_digit_pass<K>(a, b, steps, shift, hist, next, sh);
-    K* t = a;
-    a = b;
-    b = t;
-    uint32_t* h = hist;
-    hist = next;
-    next = h;
+  const int low = max(KeyTraits<K>::kWordBits - KeyTraits<K>::clz(all) - kSortBits, 0);
+  for (int from = low;; from = 0) {
+    for (int shift = from; shift < kBits && (all >> shift); shift += 8) {
+      if (((all >> shift) & K(255)) == 0) continue;
+      if (threadIdx.x < kSortThreads) block_digit_pass<K>(a, b, steps, shift, hist, next, sh);
+      K* t = a;
+      a = b;
+      b = t;
+      uint32_t* h = hist;
+      hist = next;
+      next = h;
+    }
+    __syncthreads();
+    if (from == 0) return a;
+    bool far = false;
+    for (int i = int(threadIdx.x); i < c; i += kSmThreads) {
+      const K k = a[i], p = k >> from;
+      int less = 0, l = i - 1, r = i + 1;
+      while (l >= 0 && i - l <= kSortRun && (a[l] >> from) == p) less += int(a[l--] <= k);
+      while (r < c && r - i <= kSortRun && (a[r] >> from) == p) less += int(a[r++] < k);
+      far |= i - l > kSortRun || r - i > kSortRun;
+      b[l + 1 + less] = k;
+    }
+    if (!__syncthreads_or(int(far))) return b;
   }
-  __syncthreads();
-  return a;
 }
 
 __device__ __forceinline__ uint32_t small_hash(uint32_t x) {  // Wang-style integer mix
@@ -609,7 +631,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
 namespace {
 
 // Blocks for n points: one up to where several with their barriers cost the
-// same (4,096 points in one block 57 us, 4,200 in three 60), then a block per
+// same (4,096 points in one block 54 us, 4,200 in three 58), then a block per
 // kSmShare points, at most one per SM.
 constexpr uint32_t kSmAlone = 4096, kSmShare = 2048;
 
