@@ -97,7 +97,12 @@ def make_points_checker(n, dist, seed):
 
 
 def sort_passes(a):
-    return -(-(30 if a.key_bits == 32 else 63) // (a.radix_bits or 8))
+    """Passes of the sort; 64-bit keys with 8-bit digits take passes over their top 32
+    bits (40 above 2^21 points) and one more sweep that orders runs of equal top bits."""
+    bits = 30 if a.key_bits == 32 else 63
+    if a.key_bits == 64 and (a.radix_bits or 8) == 8:
+        bits = 32 if a.n <= 1 << 21 else 40
+    return -(-bits // (a.radix_bits or 8))
 
 
 def config_of(a):

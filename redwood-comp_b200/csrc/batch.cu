@@ -22,6 +22,7 @@ struct rw_tree_batch {
   int num_sms = 148;
   int radix_bits = 8;
   int passes = 4;
+  int low_bits = 0;  // bits that the passes leave out (sort_low_bits)
   int sort_variant = 0;
 
   std::vector<uint32_t> h_pt_off, h_oct_off;
@@ -51,7 +52,7 @@ struct rw_tree_batch {
   uint32_t tree_far_cap = 0;
   void* d_zero = nullptr;
   size_t zero_bytes = 0;
-  uint32_t *d_ghist = nullptr, *d_skew = nullptr, *d_sort_desc = nullptr,
+  uint32_t *d_ghist = nullptr, *d_skew = nullptr, *d_long_run = nullptr, *d_sort_desc = nullptr,
            *d_unique_desc = nullptr,
            *d_scan_desc = nullptr, *d_tile_ctr = nullptr;
   rwt::DevStatus* d_status = nullptr;
@@ -83,8 +84,6 @@ int fail(cudaError_t e, const char* what) {
     cudaError_t e_ = (call);                             \
     if (e_ != cudaSuccess) return fail(e_, #call);       \
   } while (0)
-
-int code_bits(int32_t key_bits) { return key_bits == 32 ? 30 : 63; }
 
 // tile offsets of a kernel with tile size `tile`
 std::vector<uint32_t> tile_offsets(const std::vector<uint32_t>& pt_off, uint32_t tile) {
@@ -157,6 +156,8 @@ rwt::Scratch scratch_of(const rw_tree_batch* b) {
   sc.sort_variant = b->sort_variant;
   sc.ghist = b->d_ghist;
   sc.skew = b->d_skew;
+  sc.low_bits = b->low_bits;
+  sc.long_run = b->d_long_run;
   sc.sort_desc = b->d_sort_desc;
   sc.sort_rows = b->sort_rows;
   sc.unique_desc = b->d_unique_desc;
@@ -244,7 +245,10 @@ int rw_tree_batch_create(const uint32_t* cloud_sizes, uint32_t n_clouds, int32_t
   cudaGetDevice(&b->device);
   cudaDeviceGetAttribute(&b->num_sms, cudaDevAttrMultiProcessorCount, b->device);
   b->radix_bits = radix_bits ? radix_bits : 8;
-  b->passes = (code_bits(key_bits) + b->radix_bits - 1) / b->radix_bits;
+  uint32_t largest = 0;
+  for (uint32_t c = 0; c < n_clouds; ++c) largest = std::max(largest, cloud_sizes[c]);
+  b->low_bits = rwt::sort_low_bits(key_bits, b->radix_bits, largest);
+  b->passes = rwt::sort_pass_count(key_bits, b->radix_bits, largest);
   b->sort_variant = rwt::default_sort_variant(key_bits, b->radix_bits);
   b->class_variant[0] = b->sort_variant;
 
@@ -282,7 +286,7 @@ int rw_tree_batch_create(const uint32_t* cloud_sizes, uint32_t n_clouds, int32_t
   const size_t ctr_b = align(rwt::kCounters * 4);
   const size_t st_b = align(sizeof(rwt::DevStatus));
   const size_t per_b = align(size_t(n_clouds) * 4);
-  b->zero_bytes = ghist_b + sdesc_b + udesc_b + cdesc_b + ctr_b + st_b + 4 * per_b;
+  b->zero_bytes = ghist_b + sdesc_b + udesc_b + cdesc_b + ctr_b + st_b + 5 * per_b;
 
   const size_t ks = key_bits == 32 ? 4 : 8;
   cudaError_t e = cudaMalloc(&b->d_tables, (8 + rwt::kMaxSortClasses) * tab * 4);
@@ -317,6 +321,7 @@ int rw_tree_batch_create(const uint32_t* cloud_sizes, uint32_t n_clouds, int32_t
   b->d_n_octree = reinterpret_cast<uint32_t*>(z + o); o += per_b;
   b->d_seg_err = reinterpret_cast<int32_t*>(z + o); o += per_b;
   b->d_skew = reinterpret_cast<uint32_t*>(z + o); o += per_b;
+  b->d_long_run = reinterpret_cast<uint32_t*>(z + o); o += per_b;
 
   std::vector<uint32_t> all;
   all.reserve(8 * tab);
@@ -450,7 +455,8 @@ int rw_tree_batch_enqueue(rw_tree_batch* b, const rw_tree_batch_buffers* u, rw_s
     pk.sort_map = rwt::TileMap{b->class_tiles[k], b->d_class_toff + k * (size_t(b->n_clouds) + 1)};
     RWB_CUDA(rwt::launch_sort_passes(x, sk, pk, s));
   }
-  RWB_CUDA(rwt::launch_unique(x, sc, pl, s));
+  RWB_CUDA(rwt::launch_sort_finish(x, sc, pl, s));
+  RWB_CUDA(rwt::launch_unique(x, sc, pl, s, sc.low_bits != 0));
   RWB_CUDA(rwt::launch_radix_tree(x, sc, pl, true, false, s));
   RWB_CUDA(rwt::launch_edge_sums(x, sc, pl, s));
   RWB_CUDA(rwt::launch_octree(x, sc, pl, s, nullptr, true));

@@ -33,8 +33,6 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 
 size_t key_size(int32_t key_bits) { return key_bits == 32 ? 4 : 8; }
 
-int code_bits(int32_t key_bits) { return key_bits == 32 ? 30 : 63; }
-
 // Common argument checks.  `need` lists the buffers a stage touches.
 enum Need : unsigned {
   kPoints = 1, kKeys = 2, kAlt = 4, kBrt = 8, kEdge = 16, kOct = 32
@@ -99,6 +97,8 @@ rwt::Scratch scratch_of(const rw_tree_im_storage* im) {
   sc.sort_variant = im->sort_variant;
   sc.ghist = im->d_ghist;
   sc.skew = im->d_skew;
+  sc.low_bits = im->low_bits;
+  sc.long_run = im->d_long_run;
   sc.sort_desc = im->d_sort_desc;
   sc.sort_rows = im->sort_tiles + 1;
   sc.unique_desc = im->d_unique_desc;
@@ -163,6 +163,7 @@ int sort_enqueue_gated(rw_tree_im_storage* im, const void* keys, void* out, uint
   // sort's kernels load and store keys one at a time, so only the word
   // alignment of the key type is needed
   if (!im || !keys || !out || n < 1 || n > im->n_cap || n >= RW_MAX_POINTS) return RW_ERR_ARG;
+  if (im->low_bits) return RW_ERR_ARG;  // (64-bit keys: what ends their sort is not gated)
   rw_tree_app_data app;
   rw_tree_app_data_init(&app, n, im->key_bits);
   app.u_morton_keys = const_cast<void*>(keys);
@@ -226,7 +227,8 @@ int rw_tree_im_storage_create_ex(uint32_t n_input, int32_t key_bits,
   im->device = device;
   im->num_sms = sms;
   im->radix_bits = radix_bits == 0 ? 8 : radix_bits;
-  im->passes = (code_bits(key_bits) + im->radix_bits - 1) / im->radix_bits;
+  im->low_bits = rwt::sort_low_bits(key_bits, im->radix_bits, n_input);
+  im->passes = rwt::sort_pass_count(key_bits, im->radix_bits, n_input);
   im->sort_variant = rwt::default_sort_variant(key_bits, im->radix_bits);
   im->sort_tile = rwt::sort_tile_for(key_bits, im->radix_bits);
   im->sort_tiles = rwt::div_up(n_input, im->sort_tile);
@@ -234,7 +236,7 @@ int rw_tree_im_storage_create_ex(uint32_t n_input, int32_t key_bits,
 
   auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
   const size_t ghist_b = align(size_t(im->passes) * radix * 4);
-  const size_t skew_b = align(4);
+  const size_t skew_b = align(4), long_b = align(4);
   const size_t sdesc_b = align(size_t(im->passes) * (im->sort_tiles + 1) * radix * 4);
   const size_t udesc_b = align((size_t(rwt::div_up(n_input, rwt::kUniqueTile)) + 1) * 4);
   // stage 6's tiles, or the octree's (smaller) ones in the fused pipeline
@@ -242,7 +244,7 @@ int rw_tree_im_storage_create_ex(uint32_t n_input, int32_t key_bits,
   static_assert(rwt::kOctTile <= rwt::kScanTile, "scan descriptors sized by the octree tiles");
   const size_t ctr_b = align(rwt::kCounters * 4);
   const size_t st_b = align(sizeof(rwt::DevStatus));
-  im->zero_bytes = ghist_b + skew_b + sdesc_b + udesc_b + cdesc_b + ctr_b + st_b;
+  im->zero_bytes = ghist_b + skew_b + long_b + sdesc_b + udesc_b + cdesc_b + ctr_b + st_b;
 
   // one allocation: the zero region, the ping-pong keys (and, behind the keys
   // of a small cloud, the scratch of its one-launch pipeline), the far list
@@ -269,6 +271,7 @@ int rw_tree_im_storage_create_ex(uint32_t n_input, int32_t key_bits,
   size_t o = 0;
   im->d_ghist = reinterpret_cast<uint32_t*>(z + o); o += ghist_b;
   im->d_skew = reinterpret_cast<uint32_t*>(z + o); o += skew_b;
+  im->d_long_run = reinterpret_cast<uint32_t*>(z + o); o += long_b;
   im->d_sort_desc = reinterpret_cast<uint32_t*>(z + o); o += sdesc_b;
   im->d_unique_desc = reinterpret_cast<uint32_t*>(z + o); o += udesc_b;
   im->d_scan_desc = reinterpret_cast<uint32_t*>(z + o); o += cdesc_b;
@@ -354,6 +357,7 @@ int rw_tree_run_stage2(rw_tree_app_data* app, rw_tree_im_storage* im,
   }
   RW_CUDA(rwt::launch_keys(b, sc, pl, false, true, s));
   RW_CUDA(rwt::launch_sort_passes(b, sc, pl, s));
+  RW_CUDA(rwt::launch_sort_finish(b, sc, pl, s));
   return sync_status(im, s);
 }
 
@@ -366,6 +370,7 @@ int rw_tree_sort_enqueue(rw_tree_app_data* app, rw_tree_im_storage* im, rw_strea
   const auto pl = plan_of(*app, im);
   RW_CUDA(rwt::launch_keys(b, sc, pl, false, true, s));
   RW_CUDA(rwt::launch_sort_passes(b, sc, pl, s));
+  RW_CUDA(rwt::launch_sort_finish(b, sc, pl, s));
   return RW_OK;
 }
 
@@ -391,6 +396,10 @@ int rw_tree_sort_profile(rw_tree_app_data* app, rw_tree_im_storage* im, rw_strea
     cudaError_t e = rwt::launch_keys(b, sc, pl, false, true, s);
     cudaEventRecord(ev[1], s);
     if (e == cudaSuccess) e = rwt::launch_sort_passes(b, sc, pl, s, ev + 2);
+    if (e == cudaSuccess && sc.low_bits) {  // counts to the last pass
+      e = rwt::launch_sort_finish(b, sc, pl, s);
+      cudaEventRecord(ev[n_k], s);
+    }
     if (e != cudaSuccess) {
       rc = cuda_fail(e, "rw_tree_sort_profile");
       break;
@@ -537,8 +546,12 @@ int enqueue_impl(rw_tree_app_data* app, rw_tree_im_storage* im, cudaStream_t s,
     RW_CUDA(mark());
     RW_CUDA(rwt::launch_sort_passes(b, sc, pl, s, ev ? ev + k : nullptr));
     if (ev) k += 1 + im->passes;
+    if (sc.low_bits) {
+      RW_CUDA(rwt::launch_sort_finish(b, sc, pl, s));
+      if (ev) RW_CUDA(cudaEventRecord(ev[k - 1], s));  // counts to the last pass
+    }
   }
-  RW_CUDA(rwt::launch_unique(b, sc, pl, s));
+  RW_CUDA(rwt::launch_unique(b, sc, pl, s, sc.low_bits != 0 && !im->learned));
   RW_CUDA(mark());
   RW_CUDA(rwt::launch_radix_tree(b, sc, pl, true, geometric_delta(im), s));
   RW_CUDA(mark());

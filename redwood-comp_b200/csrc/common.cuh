@@ -30,7 +30,7 @@ enum : uint32_t {
   kSiteScan = 3,
   kSiteTree = 4,
   kSiteOctree = 5,
-  kSiteSmall = 6
+  kSiteGrid = 6
 };
 
 // ~1 s of polling with back-off before a wait gives up.

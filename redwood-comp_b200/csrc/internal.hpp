@@ -21,6 +21,7 @@ struct rw_tree_im_storage {
   // sort configuration (radix bits, passes, tile) fixed at creation
   int radix_bits = 8;
   int passes = 4;
+  int low_bits = 0;          // bits that the passes leave out (sort_low_bits)
   int sort_variant = 0;      // index into the onesweep variant menu (k_keys.cu)
   uint32_t sort_tile = 0;
   uint32_t sort_tiles = 0;  // tiles per pass at n_cap
@@ -34,6 +35,7 @@ struct rw_tree_im_storage {
   size_t zero_bytes = 0;
   uint32_t* d_ghist = nullptr;      // [passes][radix]
   uint32_t* d_skew = nullptr;       // [1]: the top sort pass's digits are skewed
+  uint32_t* d_long_run = nullptr;   // [1]: a run was too long for k_sort_fix
   uint32_t* d_sort_desc = nullptr;  // [passes][sort_tiles + 1][radix]
   uint32_t* d_unique_desc = nullptr;
   uint32_t* d_scan_desc = nullptr;
@@ -59,7 +61,7 @@ struct rw_tree_im_storage {
 namespace rwt {
 
 enum : int { kCtrUnique = 0, kCtrScan = 1, kCtrTree = 2, kCtrLinks = 3, kCtrSortBase = 4,
-             kCtrSortClassStride = 8, kMaxSortClasses = 4, kCtrSmall = 48, kCounters = 64 };
+             kMaxPasses = 8, kCtrSortClassStride = kMaxPasses, kMaxSortClasses = 4, kCtrSmall = 48, kCtrLong = 56, kCounters = 64 };
 
 // Tile sizes of the kernels (points or nodes per tile).
 constexpr uint32_t kPointTile = 4096;  // Morton / histogram
@@ -71,6 +73,21 @@ constexpr int kTreeThreads = 256;
 constexpr uint32_t kTreeTile = 2048;  // radix-tree nodes (key gaps) per tile
 constexpr int kOctThreads = 256, kOctNpt = 4;
 constexpr uint32_t kOctTile = kOctThreads * kOctNpt;
+
+// 64-bit keys with 8-bit digits: the passes leave out the low bits, which
+// k_sort_fix puts in order (k_sortfix.cu).  Four passes over the top 32 bits of
+// the 63, five over the top 40 for scratch of more points, where runs of equal
+// top bits get long.
+constexpr int kSplitLow32 = 31, kSplitLow40 = 23;
+constexpr uint32_t kSplitPoints = 1u << 21;
+inline int sort_low_bits(int key_bits, int radix_bits, uint32_t largest) {
+  if (key_bits != 64 || radix_bits != 8) return 0;
+  return largest <= kSplitPoints ? kSplitLow32 : kSplitLow40;
+}
+inline int sort_pass_count(int key_bits, int radix_bits, uint32_t largest) {
+  const int bits = (key_bits == 32 ? 30 : 63) - sort_low_bits(key_bits, radix_bits, largest);
+  return (bits + radix_bits - 1) / radix_bits;
+}
 
 // Boundary MLP of the learned sort: kMlpIn -> kMlpHidden -> kMlpHidden -> 1.
 constexpr int kMlpIn = 16, kMlpHidden = 64;
@@ -119,6 +136,10 @@ struct Scratch {
   // ballots rank them faster than shared-memory atomics (k_sort_init sets it,
   // the kRankMixed variants read it)
   uint32_t* skew = nullptr;
+  // low bits that the passes leave to launch_sort_finish (0: none), and
+  // [segments]: 1 when a run of keys with equal top bits was too long for it
+  int low_bits = 0;
+  uint32_t* long_run = nullptr;
   uint32_t* sort_desc = nullptr;  // [passes][sort_rows][radix]
   uint32_t sort_rows = 0;         // rows per pass: sort tiles + segments
   uint32_t* unique_desc = nullptr;
@@ -168,6 +189,11 @@ cudaError_t launch_keys(const Bufs& b, const Scratch& sc, const Plan& pl, bool e
 // kernel and one after each pass (profiling only).
 cudaError_t launch_sort_passes(const Bufs& b, const Scratch& sc, const Plan& pl,
                                cudaStream_t s, cudaEvent_t* marks = nullptr);
+// After the passes of every segment, when they leave bits out (low_bits): the
+// order within runs of equal top bits, and stage 3's counts per tile
+// (launch_unique's `counted`).
+cudaError_t launch_sort_finish(const Bufs& b, const Scratch& sc, const Plan& pl,
+                               cudaStream_t s);
 // The onesweep sort of keys[0, n) into out on `im`'s scratch, with every
 // kernel gated on *gate (see Scratch::gate); `clear` zeroes the scratch's
 // zero region first (not needed when a pipeline cleared it and has not used
@@ -192,7 +218,9 @@ uint32_t learned_capacity(const rw_tree_learned* L);  // n_max it was created fo
 // spin_limit polls (RW_ERR_TIMEOUT in the status word).  Needs >= 2 tiles.
 cudaError_t launch_sort_lookback_probe(const Bufs& b, const Scratch& sc, const Plan& pl,
                                        uint32_t spin_limit, cudaStream_t s);
-cudaError_t launch_unique(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_t s);
+// counted: the tiles' head counts are in sc.unique_desc already.
+cudaError_t launch_unique(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_t s,
+                          bool counted = false);
 // The unique kernels on caller-given scratch: `counts` holds one word per
 // kUniqueTile keys plus one and, like *status, must be zero.
 cudaError_t launch_unique_raw(const void* sorted, void* out, uint32_t n, int key_bits,

@@ -13,7 +13,8 @@
 // per-warp stable ranking (shared-memory atomic-OR peer masks by default;
 // ballot multi-split and match.any in the variant menu), the tile reordered by
 // digit in shared memory, and a per-digit decoupled look-back.  Digit width is
-// 8, 10 or 11 bits; 32-bit keys take 4, 3 or 3 passes, 64-bit keys 8, 7 or 6.  The
+// 8, 10 or 11 bits; 32-bit keys take 4, 3 or 3 passes, 64-bit keys 4 or 5 (the
+// low bits are put in order afterwards, k_sortfix.cu), 7 or 6.  The
 // default 32-bit variant (384 threads x 24 keys) runs three blocks per SM.
 #include <algorithm>
 
@@ -31,7 +32,8 @@ namespace rwt {
 // each CTA takes a contiguous run of tiles, so with HIST its shared-memory
 // histograms are flushed to the segment's global ones only when the segment
 // changes.  ghist: [segments][passes][RADIX].
-template <typename K, int D, bool HIST, bool ENCODE, bool POW2>
+// LOW: the low bits that the sort's passes leave out.
+template <typename K, int D, int LOW, bool HIST, bool ENCODE, bool POW2>
 __global__ void __launch_bounds__(256)
     k_keys_pass(const float4* __restrict__ pts, K* __restrict__ keys, SegTable seg,
                 TileMap map, uint32_t tiles_per_cta, float min_coord, float range,
@@ -40,8 +42,8 @@ __global__ void __launch_bounds__(256)
   pdl_enter();
   if (gate && *gate == 0) return;  // a gated sort that is not needed this run
   constexpr int RADIX = 1 << D;
-  // the sort's passes: ceil(code bits / D), as the storage computes them
-  constexpr int P = (KeyTraits<K>::kCodeBits + D - 1) / D;
+  // the sort's passes: ceil(sorted bits / D), as the storage computes them
+  constexpr int P = (KeyTraits<K>::kCodeBits - LOW + D - 1) / D;
   extern __shared__ uint32_t s_hist[];  // [P][RADIX] when HIST
   const int nh = P * RADIX;
   if (HIST) {
@@ -73,7 +75,7 @@ __global__ void __launch_bounds__(256)
       if (HIST) {
 #pragma unroll
         for (int ps = 0; ps < P; ++ps)
-          atomicAdd(&s_hist[ps * RADIX + int((k >> (ps * D)) & K(RADIX - 1))], 1u);
+          atomicAdd(&s_hist[ps * RADIX + int((k >> (LOW + ps * D)) & K(RADIX - 1))], 1u);
       }
     };
     if (hi - lo == kPointTile) {
@@ -430,7 +432,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
 
 namespace {
 
-template <typename K, int D>
+template <typename K, int D, int LOW>
 cudaError_t keys_t(const Bufs& b, const Scratch& sc, const Plan& pl, bool encode,
                    bool hist, cudaStream_t s) {
   const uint32_t tiles = pl.point_map.n_tiles;
@@ -438,13 +440,14 @@ cudaError_t keys_t(const Bufs& b, const Scratch& sc, const Plan& pl, bool encode
   const uint32_t ctas = std::max(1u, std::min<uint32_t>(tiles, uint32_t(sc.num_sms) * 8));
   const uint32_t per = div_up(tiles, ctas);
   const uint32_t grid = div_up(tiles, per);
-  if (hist && sc.passes != (KeyTraits<K>::kCodeBits + D - 1) / D) return cudaErrorInvalidValue;
+  if (hist && sc.passes != (KeyTraits<K>::kCodeBits - LOW + D - 1) / D) return cudaErrorInvalidValue;
   const size_t smem = hist ? size_t(sc.passes) * (1u << D) * 4 : 0;
   K* keys = static_cast<K*>(b.keys);
   const float inv = pow2_reciprocal(b.range);
 #define RWT_KEYS_LAUNCH(H, E)                                                        \
   do {                                                                               \
-    auto kern = inv != 0.0f ? k_keys_pass<K, D, H, E, true> : k_keys_pass<K, D, H, E, false>; \
+    auto kern = inv != 0.0f ? k_keys_pass<K, D, LOW, H, E, true>             \
+                            : k_keys_pass<K, D, LOW, H, E, false>; \
     if (smem > 48 * 1024)                                                            \
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)); \
     launch_pdl(kern, grid, 256, smem, s, b.points, keys, pl.seg, pl.point_map, per, b.min_coord, \
@@ -466,10 +469,16 @@ cudaError_t keys_t(const Bufs& b, const Scratch& sc, const Plan& pl, bool encode
 template <typename K, int D, int THREADS, int KPT, int RANK, int MINB>
 cudaError_t passes_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_t s,
                      cudaEvent_t* marks, uint32_t probe_spins) {
-  constexpr int P = (KeyTraits<K>::kCodeBits + D - 1) / D;
+  // with low bits left out the passes end in tmp (launch_sort_finish goes on to alt)
+  const int low = sc.low_bits, P = sc.passes;
+  constexpr int kFull = (KeyTraits<K>::kCodeBits + D - 1) / D;
   constexpr int RB = RANK == kRankMixed ? kRankAtomicOr : RANK;  // passes 0 .. P-2
   constexpr int RT = RANK;                                       // pass P-1
-  constexpr int TB = RANK == kRankMixed ? KeyTraits<K>::kCodeBits - (P - 1) * D : D;
+  // bits of the top digit (left out bits are chosen so that it is a full one)
+  constexpr int TB = RANK == kRankMixed && !(sizeof(K) == 8 && D == 8)
+                         ? KeyTraits<K>::kCodeBits - (kFull - 1) * D
+                         : D;
+  static_assert((63 - kSplitLow32) % 8 == 0 && (63 - kSplitLow40) % 8 == 0, "full digits");
   constexpr int kSkewLog2 = sizeof(K) == 4 ? 5 : 6;
   uint32_t* skew = RANK == kRankMixed ? sc.skew : nullptr;
   using C = BinCfg<K, D, THREADS, KPT, RB>;
@@ -481,7 +490,10 @@ cudaError_t passes_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStrea
   auto kern_top = persist ? k_binning<K, D, THREADS, KPT, RT, MINB, true, TB>
                           : k_binning<K, D, THREADS, KPT, RT, MINB, false, TB>;
   const uint32_t tiles = pl.sort_map.n_tiles;
-  if (tiles + pl.seg.count > sc.sort_rows || sc.passes != P) return cudaErrorInvalidValue;
+  if (tiles + pl.seg.count > sc.sort_rows ||
+      P != (KeyTraits<K>::kCodeBits - low + D - 1) / D || P > kMaxPasses ||
+      (low != 0) != (sizeof(K) == 8 && D == 8))
+    return cudaErrorInvalidValue;
   launch_pdl(k_sort_init<D>, pl.seg.count * sc.passes, 256, 0, s, sc.ghist, sc.sort_desc, pl.seg,
              pl.sort_map, sc.passes, sc.sort_rows, sc.gate, skew, kSkewLog2);
   cudaError_t e = cudaGetLastError();
@@ -503,7 +515,7 @@ cudaError_t passes_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStrea
     e = cudaMemsetAsync(sc.tile_ctr + kCtrSortBase, 0x01, 1, s);
     if (e != cudaSuccess) return e;
     launch_pdl(kern, tiles - 1, THREADS, C::kSmem, s, static_cast<const K*>(keys), alt, pl.seg,
-               pl.sort_map, 0, sc.sort_desc, sc.tile_ctr + kCtrSortBase, sc.status,
+               pl.sort_map, low, sc.sort_desc, sc.tile_ctr + kCtrSortBase, sc.status,
                probe_spins, static_cast<const uint32_t*>(nullptr),
                static_cast<const uint32_t*>(nullptr));
     return cudaGetLastError();
@@ -512,10 +524,10 @@ cudaError_t passes_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStrea
   const uint32_t grid =
       persist ? std::min<uint32_t>(tiles, uint32_t(sc.num_sms) * uint32_t(MINB)) : tiles;
   for (int p = 0; p < P; ++p) {
-    K* dst = ((P - 1 - p) % 2 == 0) ? alt : tmp;
+    K* dst = ((P - 1 - p) % 2 == 0) == (low == 0) ? alt : tmp;
     if (tiles)
       launch_pdl(p == P - 1 ? kern_top : kern, grid, THREADS, p == P - 1 ? CT::kSmem : C::kSmem,
-                 s, src, dst, pl.seg, pl.sort_map, p * D,
+                 s, src, dst, pl.seg, pl.sort_map, low + p * D,
                  sc.sort_desc + size_t(p) * sc.sort_rows * C::RADIX,
                  sc.tile_ctr + kCtrSortBase + p, sc.status, sc.spin_limit, sc.gate,
                  static_cast<const uint32_t*>(p == P - 1 ? skew : nullptr));
@@ -626,13 +638,16 @@ int default_sort_variant(int key_bits, int radix_bits) {
 cudaError_t launch_keys(const Bufs& b, const Scratch& sc, const Plan& pl, bool encode,
                         bool hist, cudaStream_t s) {
   if (b.key_bits == 32) {
-    if (sc.radix_bits == 8) return keys_t<uint32_t, 8>(b, sc, pl, encode, hist, s);
-    if (sc.radix_bits == 10) return keys_t<uint32_t, 10>(b, sc, pl, encode, hist, s);
-    return keys_t<uint32_t, 11>(b, sc, pl, encode, hist, s);
+    if (sc.radix_bits == 8) return keys_t<uint32_t, 8, 0>(b, sc, pl, encode, hist, s);
+    if (sc.radix_bits == 10) return keys_t<uint32_t, 10, 0>(b, sc, pl, encode, hist, s);
+    return keys_t<uint32_t, 11, 0>(b, sc, pl, encode, hist, s);
   }
-  if (sc.radix_bits == 8) return keys_t<uint64_t, 8>(b, sc, pl, encode, hist, s);
-  if (sc.radix_bits == 10) return keys_t<uint64_t, 10>(b, sc, pl, encode, hist, s);
-  return keys_t<uint64_t, 11>(b, sc, pl, encode, hist, s);
+  if (sc.radix_bits == 8)
+    return sc.low_bits == kSplitLow32
+               ? keys_t<uint64_t, 8, kSplitLow32>(b, sc, pl, encode, hist, s)
+               : keys_t<uint64_t, 8, kSplitLow40>(b, sc, pl, encode, hist, s);
+  if (sc.radix_bits == 10) return keys_t<uint64_t, 10, 0>(b, sc, pl, encode, hist, s);
+  return keys_t<uint64_t, 11, 0>(b, sc, pl, encode, hist, s);
 }
 
 cudaError_t launch_sort_passes(const Bufs& b, const Scratch& sc, const Plan& pl,

@@ -27,9 +27,9 @@
 // (tree_tiles.cuh), with each block's tile sized by the cloud.
 #include <algorithm>
 
+#include "block_sort.cuh"
 #include "internal.hpp"
 #include "morton.cuh"
-#include "rank.cuh"
 #include "tree_tiles.cuh"
 
 namespace rwt {
@@ -39,14 +39,15 @@ constexpr int kSmSamples = 32;    // per block: one per warp when they are ranke
 constexpr int kSmEncode = 8;      // points per thread of a block's share
 constexpr int kSmMaxBlocks = 256;
 constexpr int kSmGroups = kSmThreads / kOctThreads;  // octree tiles at a time per block
-constexpr int kSmHist = kSmWarps / 2 * 512;  // words of one set of the local sort's counters
+static_assert(kSmGroups < kSortBarrier, "the groups use the named barriers below");
 constexpr int kSmFill = 32;         // words between two bucket counters: a line each
 constexpr int kSmTreeChunks = 128;  // chunks of 32 gaps per radix-tree tile, at most
 
 template <typename K>
 struct SmallCfg {
   static constexpr int kCap = 57344 / int(sizeof(K));  // keys of a block, sorted in place
-  static constexpr size_t kSort = 2 * size_t(kCap) * sizeof(K) + 2 * size_t(kSmHist) * 4;
+  static constexpr int kKpt = kCap / kSortThreads;
+  static constexpr size_t kSort = 2 * size_t(kCap) * sizeof(K) + 2 * size_t(kSortHist) * 4;
   static constexpr size_t kTree = AnsvCfg<K, kSmTreeChunks>::kSmem;
   static constexpr size_t kOct = kSmGroups * sizeof(OctTileShared<K>);
   static constexpr size_t kSmem = kSort > kTree ? (kSort > kOct ? kSort : kOct)
@@ -71,7 +72,8 @@ struct SmallArgs {
 };
 
 struct SmallShared {
-  uint32_t start[256], place[256];
+  DigitShared digit;
+  uint32_t place[256];
   uint32_t warp[kSmWarps + 1];
   uint32_t hist[kSmMaxBlocks], off[kSmMaxBlocks];
   uint32_t diff[2];
@@ -79,111 +81,6 @@ struct SmallShared {
   unsigned long long gsum[kSmGroups][kOctThreads / 32];
   TreeTileShared tree;
 };
-
-// Barrier over the grid's blocks, which all run (cooperative launch): arrivals
-// only ever grow, the host never resets them between launches.  Bounded: a
-// block whose wait runs out reports RW_ERR_TIMEOUT, marks the scratch (until
-// it is cleared) and leaves.
-struct GridBarrier {
-  uint32_t* word;
-  uint32_t blocks, target;
-  __device__ __forceinline__ bool sync(SmallShared& sh, const SmallArgs& a) {
-    __syncthreads();
-    if (blocks == 1) return true;
-    target += blocks;
-    if (threadIdx.x == 0) {
-      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(word) : "memory");
-      uint32_t spin = 0;
-      while (int32_t(ld_acquire(word) - target) < 0 && ++spin < kSpinLimit) backoff(spin);
-      sh.ok = spin < kSpinLimit;
-      if (!sh.ok) {
-        st_relaxed(a.sync + 2, 1u);
-        report_error(a.status, RW_ERR_TIMEOUT, kSiteSmall);
-        *reinterpret_cast<volatile int32_t*>(&a.host_status->err) = RW_ERR_TIMEOUT;
-      }
-    }
-    __syncthreads();
-    return sh.ok != 0;
-  }
-};
-
-// The local sort runs on half of the block's warps: below a few thousand keys
-// its time is instructions per thread (ranking 32 keys, scanning the 512
-// half-warp counters of every warp), so fewer warps with more keys each are
-// faster (32 warps with 3 steps of 32 keys took 2.3 us a pass at 3,001 keys).
-constexpr int kSortWarps = kSmWarps / 2, kSortThreads = kSortWarps * 32;
-
-__device__ __forceinline__ void sort_sync() {
-  asm volatile("bar.sync %0, %1;" ::"n"(kSmGroups + 1), "n"(kSortThreads) : "memory");
-}
-
-// Stable pass over one 8-bit digit of `steps` x 512 keys, from `a` to `b`, by
-// kSortThreads threads; leaves the digits' first places in sh.start.  A
-// half-warp owns 16 * steps consecutive keys and ranks 16 a step in one word
-// per digit (half_rank, rank.cuh: count << 16 | peer mask).  hist is zero on
-// entry, `next` is left zero for the next pass.
-template <typename K>
-__device__ __forceinline__ void block_digit_pass(const K* a, K* b, int steps, int shift,
-                                                 uint32_t* hist, uint32_t* next,
-                                                 SmallShared& sh) {
-  constexpr int KPT = SmallCfg<K>::kCap / kSortThreads;
-  const int tid = int(threadIdx.x), warp = tid >> 5, lane = tid & 31;
-  const uint32_t l16 = uint32_t(lane) & 15u, lt16 = (1u << l16) - 1u;
-  uint32_t* wp = hist + warp * 512 + (lane >> 4);
-  const int first = (2 * warp + (lane >> 4)) * 16 * steps + int(l16);
-  uint32_t rank2[RankPack<KPT>::kRegs];
-#pragma unroll
-  for (int i = 0; i < KPT; ++i) {
-    if (i >= steps) break;
-    uint32_t* w = wp + 2 * (uint32_t(a[first + 16 * i] >> shift) & 255u);
-    atomicOr(w, 1u << l16);
-    __syncwarp();
-    const uint32_t word = *w, peers = word & 0xffffu, cnt = word >> 16;
-    const uint32_t below = uint32_t(__popc(peers & lt16));
-    __syncwarp();
-    if ((peers >> l16) == 1u) *w = (cnt + below + 1u) << 16;  // the highest peer
-    RankPack<KPT>::set(rank2, i, cnt + below);
-    __syncwarp();
-  }
-  sort_sync();
-  // the counts in the order (digit, warp, half): thread (digit tid / 2, half
-  // tid % 2 of the warps), so one scan over the threads gives every place
-  constexpr int Q = kSortWarps / 2;
-  const int d = tid >> 1, w0 = (tid & 1) * Q;
-  uint2 v[Q];
-  uint32_t sum = 0;
-#pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    v[q] = *reinterpret_cast<const uint2*>(hist + (w0 + q) * 512 + 2 * d);
-    v[q].x >>= 16;
-    v[q].y >>= 16;
-    sum += v[q].x + v[q].y;
-  }
-#pragma unroll
-  for (int q = 0; q < kSmHist / 4 / kSortThreads; ++q)
-    reinterpret_cast<uint4*>(next)[q * kSortThreads + tid] = make_uint4(0, 0, 0, 0);
-  const uint32_t inc = warp_inclusive_scan(sum);
-  if (lane == 31) sh.warp[warp] = inc;
-  sort_sync();
-  uint32_t run = inc - sum;
-#pragma unroll
-  for (int w = 0; w < kSortWarps; ++w) run += w < warp ? sh.warp[w] : 0u;
-  if ((tid & 1) == 0) sh.start[d] = run;
-#pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    const uint2 o = make_uint2(run, run + v[q].x);
-    *reinterpret_cast<uint2*>(hist + (w0 + q) * 512 + 2 * d) = o;
-    run = o.y + v[q].y;
-  }
-  sort_sync();
-#pragma unroll
-  for (int i = 0; i < KPT; ++i) {
-    if (i >= steps) break;
-    const K k = a[first + 16 * i];
-    b[wp[2 * (uint32_t(k >> shift) & 255u)] + RankPack<KPT>::get(rank2, i)] = k;
-  }
-  sort_sync();
-}
 
 // Sorts a block's c keys in `a` (with `b` as the other half); returns where
 // they end.  Digits that all keys share are left out.  The keys are filled up
@@ -223,7 +120,8 @@ __device__ K* block_sort(K* a, K* b, int c, uint32_t* hist, uint32_t* next, Smal
   for (int from = low;; from = 0) {
     for (int shift = from; shift < kBits && (all >> shift); shift += 8) {
       if (((all >> shift) & K(255)) == 0) continue;
-      if (threadIdx.x < kSortThreads) block_digit_pass<K>(a, b, steps, shift, hist, next, sh);
+      if (threadIdx.x < kSortThreads)
+        block_digit_pass<K, SmallCfg<K>::kKpt>(a, b, steps, shift, hist, next, sh.digit);
       K* t = a;
       a = b;
       b = t;
@@ -263,10 +161,10 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
   K* sa = reinterpret_cast<K*>(smem);
   K* sb = sa + C::kCap;
   uint32_t* hist = reinterpret_cast<uint32_t*>(sb + C::kCap);
-  uint32_t* next = hist + kSmHist;
+  uint32_t* next = hist + kSortHist;
   const int tid = int(threadIdx.x), lane = tid & 31, warp = tid >> 5;
   const uint32_t P = gridDim.x, b = blockIdx.x;
-  GridBarrier bar{a.sync, P, ld_relaxed(a.sync + 1)};
+  GridBarrier bar{a.sync, P, ld_relaxed(a.sync + 1), &sh.ok, a.sync + 2, a.status, a.host_status};
   if (ld_relaxed(a.sync + 2)) {  // an earlier wait gave up and nothing cleared the scratch since
     if (b == 0 && tid == 0)
       *reinterpret_cast<volatile int32_t*>(&a.host_status->err) = RW_ERR_TIMEOUT;
@@ -305,7 +203,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
       }
     }
   }
-  for (int i = tid; i < kSmHist / 4; i += kSmThreads)
+  for (int i = tid; i < kSortHist / 4; i += kSmThreads)
     reinterpret_cast<uint4*>(hist)[i] = make_uint4(0, 0, 0, 0);
   __syncthreads();
 
@@ -335,7 +233,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
         }
       samples[b * kSmSamples + lane] = k;
     }
-    if (!bar.sync(sh, a)) return;
+    if (!bar.sync()) return;
     const int ns = int(P) * kSmSamples;
     constexpr int kPitch = kSmSamples + 1;  // a block's samples: lanes in different banks
     K* ss = sb;
@@ -368,7 +266,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
       r = warp_sum(r);
       if (lane == 0 && r && r % kSmSamples == 0) splitters[r / kSmSamples - 1] = my;
     }
-    if (!bar.sync(sh, a)) return;
+    if (!bar.sync()) return;
     const int nspl = int(P) - 1;
     for (int i = tid; i < int(P); i += kSmThreads) {
       if (i < nspl) s_spl[i] = splitters[i];
@@ -416,7 +314,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
         if (at < a.cap) region[size_t(bk) * a.cap + at] = sa[i];
       }
     }
-    if (!bar.sync(sh, a)) return;
+    if (!bar.sync()) return;
     uint32_t f = 0, before = 0, over = 0;
     if (tid < int(P)) {
       f = a.fill[tid * kSmFill];
@@ -443,15 +341,16 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
         const int steps = (c + kSortThreads - 1) / kSortThreads;
         for (int i = c + tid; i < steps * kSortThreads; i += kSmThreads) sa[i] = K(~K(0));
         __syncthreads();
-        if (tid < kSortThreads) block_digit_pass<K>(sa, sb, steps, shift, hist, next, sh);
+        if (tid < kSortThreads)
+          block_digit_pass<K, SmallCfg<K>::kKpt>(sa, sb, steps, shift, hist, next, sh.digit);
         __syncthreads();
         uint32_t* h = hist;
         hist = next;
         next = h;
         // (the filling counts in the last digit: its end is c)
         if (tid < 256)
-          a.mat[b * 256 + tid] = (tid < 255 ? sh.start[tid + 1] : uint32_t(c)) - sh.start[tid];
-        if (!bar.sync(sh, a)) return;
+          a.mat[b * 256 + tid] = (tid < 255 ? sh.digit.start[tid + 1] : uint32_t(c)) - sh.digit.start[tid];
+        if (!bar.sync()) return;
         uint32_t tot = 0, prior = 0;
         if (tid < 256)
           for (uint32_t j = 0; j < P; ++j) {
@@ -461,11 +360,11 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
           }
         uint32_t all;
         const uint32_t ex = block_exclusive_scan<kSmThreads>(tot, sh.warp, &all);
-        if (tid < 256) sh.place[tid] = ex + prior - sh.start[tid];
+        if (tid < 256) sh.place[tid] = ex + prior - sh.digit.start[tid];
         __syncthreads();
         for (int i = tid; i < c; i += kSmThreads)
           tmp[sh.place[uint32_t(sb[i] >> shift) & 255u] + uint32_t(i)] = sb[i];
-        if (!bar.sync(sh, a)) return;
+        if (!bar.sync()) return;
         for (int i = tid; i < c; i += kSmThreads) sa[i] = tmp[p0 + i];
         __syncthreads();
       }
@@ -493,7 +392,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
       last[b] = c ? sorted[c - 1] : K(0);
       a.counts[b] = uint32_t(c);
     }
-    if (!bar.sync(sh, a)) return;
+    if (!bar.sync()) return;
     uint32_t h = 0;
     if (tid < int(P)) {
       // loaded together; an empty block before this one is rare
@@ -522,7 +421,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
   for (int i = i0; i < i1; ++i)
     if ((hm >> (i - i0)) & 1u) keys[pos++] = sorted[i];
   if (b == 0 && tid == 0) a.status->n_unique = u;
-  if (!bar.sync(sh, a)) return;
+  if (!bar.sync()) return;
 
   auto finish = [&](uint32_t m) {  // block 0, one thread: the host's copy of the counts
     if (P > 1) st_relaxed(a.sync + 1, bar.target);
@@ -552,7 +451,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
       __syncthreads();  // the next tile reuses the shared arrays
     }
   }
-  if (!bar.sync(sh, a)) return;
+  if (!bar.sync()) return;
 
   // ---- stage 6: the sums of the octree's tiles ----
   const int group = tid / kOctThreads, gt = tid % kOctThreads;
@@ -582,7 +481,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
     v = uint32_t(group_sum(v));
     if (gt == 0) a.sums[t] = v;
   }
-  if (!bar.sync(sh, a)) return;
+  if (!bar.sync()) return;
 
   // ---- stages 6 and 7: offsets, rows, links inside a tile ----
   uint32_t m = 0;
@@ -606,7 +505,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
                          a.min_coord, a.range, a.o, a.far, a.far_cap, a.far_n);
     gsync();
   }
-  if (!bar.sync(sh, a)) return;
+  if (!bar.sync()) return;
 
   // ---- links that leave their tile, and the leaves ----
   octree_far_links<K>(keys, a.prefix_n, a.parents, a.edge_count, a.edge_offset,
@@ -614,10 +513,10 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
                       &a.status->n_unique, &a.status->n_octree_nodes, &a.status->err, a.o, a.far,
                       a.far_cap, a.far_n);
   if (a.leaves) {
-    if (!bar.sync(sh, a)) return;
+    if (!bar.sync()) return;
     leaf_claim<K>(keys, a.prefix_n, a.hl, a.hr, a.lc, a.parents, a.edge_count, a.edge_offset,
                   a.o.children, a.o.leaf_mask, &a.status->n_unique, a.o.capacity);
-    if (!bar.sync(sh, a)) return;
+    if (!bar.sync()) return;
     leaf_write<K>(keys, a.prefix_n, a.hl, a.hr, a.lc, a.parents, a.edge_count, a.edge_offset,
                   a.o.children, &a.status->n_unique, a.o.capacity);
   }

@@ -570,12 +570,14 @@ namespace {
 
 
 template <typename K>
-cudaError_t unique_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_t s) {
+cudaError_t unique_t(const Bufs& b, const Scratch& sc, const Plan& pl, bool counted,
+                     cudaStream_t s) {
   const uint32_t tiles = pl.unique_map.n_tiles;
   if (!tiles) return cudaSuccess;
   const K* sorted = static_cast<const K*>(b.alt);
-  launch_pdl(k_unique_count<K>, tiles, kUniqueThreads, 0, s, sorted, pl.seg, pl.unique_map,
-                                                     sc.unique_desc);
+  if (!counted)
+    launch_pdl(k_unique_count<K>, tiles, kUniqueThreads, 0, s, sorted, pl.seg, pl.unique_map,
+               sc.unique_desc);
   launch_pdl(k_tile_scan, 1, 1024, 0, s, sc.unique_desc, tiles, pl.seg, pl.unique_map, pl.n_unique);
   launch_pdl(k_unique_write<K>, tiles, kUniqueThreads, 0, s, sorted, static_cast<K*>(b.keys), pl.seg,
                                                      pl.unique_map, sc.unique_desc);
@@ -645,8 +647,10 @@ cudaError_t octree_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStrea
 
 }  // namespace
 
-cudaError_t launch_unique(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_t s) {
-  return b.key_bits == 32 ? unique_t<uint32_t>(b, sc, pl, s) : unique_t<uint64_t>(b, sc, pl, s);
+cudaError_t launch_unique(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_t s,
+                          bool counted) {
+  return b.key_bits == 32 ? unique_t<uint32_t>(b, sc, pl, counted, s)
+                          : unique_t<uint64_t>(b, sc, pl, counted, s);
 }
 
 namespace {
