@@ -234,9 +234,9 @@ cudaError_t launch_radix_tree(const Bufs& b, const Scratch& sc, const Plan& pl, 
 cudaError_t launch_edge_count(const Bufs& b, const Scratch& sc, const Plan& pl,
                               cudaStream_t s);
 cudaError_t launch_edge_scan(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_t s);
-// The first half of stage 6 on the octree's tiles: each tile's count sum,
-// scanned into sc.scan_desc, and the octree row counts.  launch_octree with
-// fused_offsets then makes and writes the offsets itself.
+// The scan of the octree tiles' count sums that stages 4 and 5 in one pass left
+// in sc.scan_desc (zero before them), and the octree row counts.  launch_octree
+// with fused_offsets then makes and writes the offsets itself.
 cudaError_t launch_edge_sums(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_t s);
 cudaError_t launch_octree(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_t s,
                           cudaEvent_t* marks = nullptr, bool fused_offsets = false);

@@ -172,6 +172,8 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
   }
   if (b == 0) {
     for (uint32_t i = uint32_t(tid); i < P; i += kSmThreads) a.fill[i * kSmFill] = 0;
+    for (uint32_t i = uint32_t(tid); i < (a.n + kOctTile - 1) / kOctTile; i += kSmThreads)
+      a.sums[i] = 0;
     if (tid == 0) {
       *a.status = DevStatus{0, 0, 0, 0};
       *a.far_n = 0;
@@ -447,13 +449,12 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
     for (int ch = int(b) * cpb; ch < end; ch += kSmTreeChunks) {
       tree_tile<K, true, LESS, kSmThreads, kSmTreeChunks, true, false>(
           smem, sh.tree, keys, n, ch * 32, min(kSmTreeChunks, end - ch), &a.status->err,
-          a.prefix_n, a.hl, a.hr, a.lc, a.parents, a.edge_count);
+          a.prefix_n, a.hl, a.hr, a.lc, a.parents, a.edge_count, a.sums);
       __syncthreads();  // the next tile reuses the shared arrays
     }
   }
   if (!bar.sync()) return;
 
-  // ---- stage 6: the sums of the octree's tiles ----
   const int group = tid / kOctThreads, gt = tid % kOctThreads;
   auto gsync = [group] {
     asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(kOctThreads) : "memory");
@@ -470,22 +471,10 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
     return t;
   };
   const int tiles = (n + int(kOctTile) - 1) / int(kOctTile);
-  // (tiles go to the blocks in turn, so that few tiles spread over all SMs)
-  for (int t = group * int(P) + int(b); t < tiles; t += int(P) * kSmGroups) {
-    uint32_t v = 0;
-#pragma unroll
-    for (int q = 0; q < kOctNpt; ++q) {
-      const int i = t * int(kOctTile) + q * kOctThreads + gt;
-      if (i < n) v += uint32_t(a.edge_count[i]);
-    }
-    v = uint32_t(group_sum(v));
-    if (gt == 0) a.sums[t] = v;
-  }
-  if (!bar.sync()) return;
-
   // ---- stages 6 and 7: offsets, rows, links inside a tile ----
   uint32_t m = 0;
   OctTileShared<K>* osh = reinterpret_cast<OctTileShared<K>*>(smem) + group;
+  // (tiles go to the blocks in turn, so that few tiles spread over all SMs)
   for (int t = group * int(P) + int(b); t < tiles; t += int(P) * kSmGroups) {
     unsigned long long v = 0;  // all tiles' rows << 32 | those of the tiles before (below 2^32)
     for (int j = gt; j < tiles; j += kOctThreads) {

@@ -286,12 +286,16 @@ __global__ void __launch_bounds__(kUniqueThreads)
 // ---------------------------------------------------------------------------
 
 template <typename K, bool EDGES, int LESS>
-__global__ void __launch_bounds__(kTreeThreads, 8)  // 8 blocks (64 warps) per SM
+// 8 blocks (64 warps) per SM with 32-bit keys; the shared memory holds 5 with
+// 64-bit ones, which then need no more than 48 registers (77.6 against 81.0 us at
+// 5,000,011 points with 32)
+__global__ void __launch_bounds__(kTreeThreads, sizeof(K) == 4 ? 8 : 5)
     k_radix_tree(const K* __restrict__ codes_all, SegTable seg, TileMap map,
                  const uint32_t* __restrict__ n_unique, int32_t* __restrict__ seg_err,
                  uint8_t* __restrict__ prefix_n, uint8_t* __restrict__ hl,
                  uint8_t* __restrict__ hr, int32_t* __restrict__ lc,
-                 int32_t* __restrict__ parents, int32_t* __restrict__ edge_count) {
+                 int32_t* __restrict__ parents, int32_t* __restrict__ edge_count,
+                 TileMap nodes, uint32_t* __restrict__ sums) {
   pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ TreeTileShared sh;
@@ -308,7 +312,8 @@ __global__ void __launch_bounds__(kTreeThreads, 8)  // 8 blocks (64 warps) per S
   if (g0 >= n) return;
   tree_tile<K, EDGES, LESS, kTreeThreads, kTreeTile / 32, false, true>(
       smem_raw, sh, codes_all + sb, n, g0, 0, seg_err + c, prefix_n + sb, hl + sb, hr + sb,
-      lc + sb, parents + sb, EDGES ? edge_count + sb : nullptr);
+      lc + sb, parents + sb, EDGES ? edge_count + sb : nullptr,
+      EDGES ? sums + (nodes.toff ? nodes.toff[c] : 0u) : nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -474,52 +479,6 @@ __launch_bounds__(kOctThreads, sizeof(K) == 4 ? 8 : 6)
       far_cap, far_n);
 }
 
-// Sum of the edge counts of every tile of kOctTile nodes (the tiles of
-// k_octree), for k_tile_scan: stage 6's reduce on the octree's tiles.  A block
-// takes four tiles, 64 threads each; thread j of a tile adds the 16-byte
-// vectors j, j + 64, j + 128 and j + 192 of it (a sum needs no order, so the
-// warps read consecutive vectors).
-__global__ void __launch_bounds__(kOctThreads)
-    k_node_sums(const int32_t* __restrict__ ec_all, SegTable seg, TileMap map,
-                const uint32_t* __restrict__ n_unique, uint32_t* __restrict__ E) {
-  pdl_enter();
-  constexpr int kVecs = int(kOctTile) / 4 / 64;  // 16-byte vectors per thread
-  static_assert(kOctThreads == 256 && kVecs * 4 * 64 == int(kOctTile), "four tiles of 64 threads");
-  __shared__ uint32_t s_warp[kOctThreads / 32];
-  const uint32_t g = threadIdx.x >> 6;  // tile of this thread's group
-  const uint32_t tile = 4 * blockIdx.x + g;
-  uint32_t local = 0;
-  if (tile < map.n_tiles) {
-    uint32_t first;
-    const uint32_t c = tile_segment(seg, map, tile, &first);
-    const uint32_t nu = *reinterpret_cast<const volatile uint32_t*>(n_unique + c);
-    const bool ok = nu >= 3 && nu != RW_COUNT_UNSET && nu <= seg_size(seg, c);
-    const int n = ok ? int(nu - 1) : 0;
-    const int tb = int(tile - first) * int(kOctTile);
-    const int j = int(threadIdx.x & 63u);
-    const int32_t* ec = ec_all + seg_begin(seg, c);
-    if (tb + int(kOctTile) <= n && (reinterpret_cast<uintptr_t>(ec + tb) & 15u) == 0) {
-      int4 x[kVecs];
-#pragma unroll
-      for (int q = 0; q < kVecs; ++q) x[q] = reinterpret_cast<const int4*>(ec + tb)[q * 64 + j];
-#pragma unroll
-      for (int q = 0; q < kVecs; ++q)
-        local += uint32_t(x[q].x) + uint32_t(x[q].y) + uint32_t(x[q].z) + uint32_t(x[q].w);
-    } else {
-      for (int q = 0; q < kVecs; ++q)
-        for (int e = 0; e < 4; ++e) {
-          const int i = tb + (q * 64 + j) * 4 + e;
-          if (i < n) local += uint32_t(ec[i]);
-        }
-    }
-  }
-  local = warp_sum(local);
-  if (lane_id() == 0) s_warp[threadIdx.x >> 5] = local;
-  __syncthreads();
-  if (threadIdx.x < 4 && 4 * blockIdx.x + threadIdx.x < map.n_tiles)
-    E[4 * blockIdx.x + threadIdx.x] = s_warp[2 * threadIdx.x] + s_warp[2 * threadIdx.x + 1];
-}
-
 template <typename K>
 __global__ void __launch_bounds__(256)
     k_octree_far_links(const K* __restrict__ codes_all, const uint8_t* __restrict__ prefix_all,
@@ -599,7 +558,8 @@ cudaError_t tree_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_
   if (e != cudaSuccess) return e;
   launch_pdl(kern, tiles, kTreeThreads, smem, s, static_cast<const K*>(b.keys), pl.seg,
              pl.tree_map, pl.n_unique, pl.seg_err, b.prefix_n, b.hl, b.hr, b.lc, b.parents,
-             EDGES ? b.edge_count : static_cast<int32_t*>(nullptr));
+             EDGES ? b.edge_count : static_cast<int32_t*>(nullptr), pl.node_map,
+             EDGES ? sc.scan_desc : static_cast<uint32_t*>(nullptr));
   return cudaGetLastError();
 }
 
@@ -722,8 +682,6 @@ cudaError_t launch_edge_scan(const Bufs& b, const Scratch& sc, const Plan& pl, c
 cudaError_t launch_edge_sums(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_t s) {
   const uint32_t tiles = pl.node_map.n_tiles;
   if (!tiles) return cudaSuccess;
-  launch_pdl(k_node_sums, div_up(tiles, 4), kOctThreads, 0, s, b.edge_count, pl.seg, pl.node_map,
-                                                      pl.n_unique, sc.scan_desc);
   launch_pdl(k_tile_scan, 1, 1024, 0, s, sc.scan_desc, tiles, pl.seg, pl.node_map, pl.n_octree);
   return cudaGetLastError();
 }

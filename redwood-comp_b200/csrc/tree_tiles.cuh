@@ -198,11 +198,13 @@ __device__ int coop_root_split(const K* __restrict__ codes, int n, int D) {
 // (RW_TREE_OPT_GEOMETRIC_DELTA: the tree's shape depends only on comparisons
 // between deltas, so the clz - 2 tree is the clz - 1 tree with every prefix,
 // at least 1 for distinct 30-bit keys, lowered by one).
+// Returns the node's index; *count gets its edge count (0 without EDGES).
 template <bool EDGES, int LESS>
-__device__ __forceinline__ void write_gap_node_d(int g, int D, int L, int R, int dl, int dr,
-                                                 int root_true_delta, int root_prefix,
-                                                 uint8_t* pn, uint8_t* l8, uint8_t* r8,
-                                                 int32_t* lcs, int32_t* par, int32_t* ec) {
+__device__ __forceinline__ int write_gap_node_d(int g, int D, int L, int R, int dl, int dr,
+                                                int root_true_delta, int root_prefix,
+                                                uint8_t* pn, uint8_t* l8, uint8_t* r8,
+                                                int32_t* lcs, int32_t* par, int32_t* ec,
+                                                int* count) {
   const int i = dr > dl ? R : L + 1;  // left child of R's node, else right child of L's
   const bool leaf_l = g == L + 1, leaf_r = g + 1 == R;
   pn[i] = uint8_t(D - LESS);
@@ -211,27 +213,25 @@ __device__ __forceinline__ void write_gap_node_d(int g, int D, int L, int R, int
   lcs[i] = g;
   if (!leaf_l) par[g] = i;
   if (!leaf_r) par[g + 1] = i;
+  *count = 0;
   if (EDGES) {
     const int pd = max(dl, dr);
     const int pp = pd == root_true_delta ? root_prefix : pd;
-    ec[i] = (D - LESS) / 3 - (pp - LESS) / 3;
+    *count = (D - LESS) / 3 - (pp - LESS) / 3;
+    ec[i] = *count;
   }
+  return i;
 }
 
-template <typename K, bool EDGES, int LESS, typename DAt>
-__device__ __forceinline__ void write_gap_node(int g, int n, int D, int L, int R, const DAt& d_at,
-                                               int root_true_delta, int root_prefix,
-                                               uint8_t* pn, uint8_t* l8, uint8_t* r8,
-                                               int32_t* lcs, int32_t* par, int32_t* ec) {
-  if (L < 0 && R >= n) return;
-  write_gap_node_d<EDGES, LESS>(g, D, L, R, L >= 0 ? d_at(L) : -1, R < n ? d_at(R) : -1,
-                          root_true_delta, root_prefix, pn, l8, r8, lcs, par, ec);
-}
+// Octree tiles that the nodes of a radix-tree tile of up to 4,096 gaps can lie in
+// (a tile of k_small starts anywhere).
+constexpr int kTreeSums = 4096 / int(kOctTile) + 1;
 
 // The shared words of a tile besides the arrays in dynamic shared memory.
 struct TreeTileShared {
   uint32_t far[kTreeFarPerTile];  // the tile's gaps left to phase D
   uint32_t far_n, pend_n;
+  int sum[kTreeSums];  // edge counts of the nodes [g0, ..) by octree tile
   alignas(8) uint64_t bar;
 };
 
@@ -240,14 +240,19 @@ struct TreeTileShared {
 // time number up to TCH, else it is TCH.  BULK: the keys may come by a bulk
 // copy (not in a kernel that wrote them itself: the copy engine would need a
 // proxy fence).  `err` takes the first error.  The tile that starts at 0 also
-// writes node 0.
+// writes node 0.  With EDGES the counts of every kOctTile nodes are also added
+// up in sums (zero before): stage 6's reduction, which as a kernel of its own
+// read every count again (16.8M uniform points, 32-bit keys: tree and scan 205.1
+// -> 198.5 us; gathering the nodes in shared memory to write and sum them in
+// order took more instructions than it saved, 203.4).
 template <typename K, bool EDGES, int LESS, int NT, int TCH, bool DYN, bool BULK>
 __device__ __forceinline__ void tree_tile(unsigned char* smem_raw, TreeTileShared& sh,
                                           const K* __restrict__ codes, int n, int g0,
                                           int tch_arg, int32_t* err, uint8_t* __restrict__ pn,
                                           uint8_t* __restrict__ l8, uint8_t* __restrict__ r8,
                                           int32_t* __restrict__ lcs, int32_t* __restrict__ par,
-                                          int32_t* __restrict__ ec) {
+                                          int32_t* __restrict__ ec,
+                                          uint32_t* __restrict__ sums) {
   using C = AnsvCfg<K, TCH>;
   constexpr int NV = C::NV, VB = C::VB, NW = NT / 32, JN = DYN ? 1 : 2;
   static_assert(kTreeFarPerTile >= 2 * uint32_t(NV), "far gaps of a tile: NV per side");
@@ -285,10 +290,10 @@ __device__ __forceinline__ void tree_tile(unsigned char* smem_raw, TreeTileShare
   };
   if (!DYN && g0 == 0 && threadIdx.x >= NT - 32) root_node();
 
-  if (threadIdx.x == 0) {  // read after the barriers below
-    sh.far_n = 0;
-    sh.pend_n = 0;
-  }
+  // read after the barriers below
+  if (threadIdx.x == 0) sh.far_n = sh.pend_n = 0;
+  if (EDGES && threadIdx.x < kTreeSums) sh.sum[threadIdx.x] = 0;
+  const int t0 = g0 / int(kOctTile);  // the octree tile of sh.sum[0]
 
   // the window's keys [wlo, wlo + kAnsvWin]: one bulk copy when the window
   // lies inside the keys and starts on a 16-byte boundary (every interior
@@ -346,6 +351,7 @@ __device__ __forceinline__ void tree_tile(unsigned char* smem_raw, TreeTileShare
   uint32_t mlane[VB];
 #pragma unroll
   for (int bt = 0; bt < VB; ++bt) mlane[bt] = 0u - ((lane >> bt) & 1u);
+  int acc = 0;  // edge counts of this lane's nodes
   for (int ch0 = kAnsvHalo + int(warp); ch0 < kAnsvHalo + tch; ch0 += JN * NW) {
     int e[JN];
 #pragma unroll
@@ -394,8 +400,9 @@ __device__ __forceinline__ void tree_tile(unsigned char* smem_raw, TreeTileShare
 #pragma unroll
     for (int j = 0; j < JN; ++j) {
       const int ch = ch0 + j * NW;
-      const uint32_t from0 = __shfl_sync(0xffffffffu, lt0[j], e[j] & 31);
-      const uint32_t from1 = NV > 32 ? __shfl_sync(0xffffffffu, lt1[j], e[j] & 31) : 0u;
+      // (the shuffles take the lane index modulo 32)
+      const uint32_t from0 = __shfl_sync(0xffffffffu, lt0[j], e[j]);
+      const uint32_t from1 = NV > 32 ? __shfl_sync(0xffffffffu, lt1[j], e[j]) : 0u;
       const uint32_t lt = (NV > 32 && e[j] >= 32) ? from1 : from0;
       {
         const int tg = (ch - kAnsvHalo) * 32 + int(lane);
@@ -405,15 +412,28 @@ __device__ __forceinline__ void tree_tile(unsigned char* smem_raw, TreeTileShare
         const int rp = __ffs(rm) - 1;
         // E of the two nearest smaller lanes (a wall lane past the last gap
         // has E = 0, so D = -1 there as for the wall at n)
-        const int el = __shfl_sync(0xffffffffu, e[j], lp & 31);
-        const int er = __shfl_sync(0xffffffffu, e[j], rp & 31);
+        const int el = __shfl_sync(0xffffffffu, e[j], lp);
+        const int er = __shfl_sync(0xffffffffu, e[j], rp);
         const int g = g0 + tg;
         const bool real = g < n;
-        const bool here = real && lp >= 0 && rp >= 0;
+        const bool here = real && lm && rm;
+        int count = 0;
         if (here)
-          write_gap_node_d<EDGES, LESS>(g, e[j] - 1, g - int(lane) + lp, g - int(lane) + rp, el - 1,
-                                  er - 1, root_true_delta, root_prefix, pn, l8, r8, lcs, par,
-                                  ec);
+          write_gap_node_d<EDGES, LESS>(g, e[j] - 1, g - int(lane) + lp, g - int(lane) + rp,
+                                        el - 1, er - 1, root_true_delta, root_prefix, pn, l8, r8,
+                                        lcs, par, ec, &count);
+        if (EDGES) {
+          // a chunk's own nodes lie in the chunk, so in one octree tile, and
+          // the chunks of a round in the same one (a sum kept over the rounds
+          // would need a register more than eight blocks leave: 194 us)
+          static_assert(JN == 1 || (JN * NW * 32) <= int(kOctTile), "a round in one octree tile");
+          acc += count;
+          if (j == JN - 1) {
+            acc = __reduce_add_sync(0xffffffffu, acc);
+            if (lane == 0) atomicAdd(&sh.sum[(g0 + (ch - kAnsvHalo) * 32) / int(kOctTile) - t0], acc);
+            acc = 0;
+          }
+        }
         const uint32_t pm = __ballot_sync(0xffffffffu, real && !here);
         if (pm) {
           uint32_t at = 0;
@@ -452,6 +472,24 @@ __device__ __forceinline__ void tree_tile(unsigned char* smem_raw, TreeTileShare
   const int wend = wlo + win - 1;  // last gap of the window
   auto d_at = [&](int p) -> int {       // D of gap p in [0, n)
     return (p >= wlo && p <= wend) ? int(s_e[p - wlo]) - 1 : delta(codes[p], codes[p + 1]);
+  };
+  // writes the node that splits at gap g, given its nearest smaller gaps L and
+  // R (-1 and n for the walls; the root is skipped), and adds its count (to
+  // registers for the octree tiles t0 and t0 + 1, the tile's own but for the
+  // largest of k_small)
+  int sum0 = 0, sum1 = 0;
+  auto put = [&](int g, int D, int L, int R, const auto& d_of) {
+    if (L < 0 && R >= n) return;
+    int count;
+    const int i = write_gap_node_d<EDGES, LESS>(
+        g, D, L, R, L >= 0 ? d_of(L) : -1, R < n ? d_of(R) : -1, root_true_delta, root_prefix, pn,
+        l8, r8, lcs, par, ec, &count);
+    if (EDGES) {
+      const int t = i / int(kOctTile) - t0;
+      if (t == 0) sum0 += count;
+      else if (t == 1) sum1 += count;
+      else if (count) atomicAdd(sums + t0 + t, uint32_t(count));
+    }
   };
   const int np = int(sh.pend_n);
   for (int q = int(threadIdx.x); q < np; q += NT) {
@@ -502,9 +540,7 @@ __device__ __forceinline__ void tree_tile(unsigned char* smem_raw, TreeTileShare
       else atomicCAS(reinterpret_cast<int*>(err), 0, RW_ERR_CAPACITY);  // not reachable, see above
       continue;
     }
-    write_gap_node<K, EDGES, LESS>(g, n, e - 1, max(L, -1), min(R, n), d_at, root_true_delta,
-                             root_prefix, pn, l8, r8, lcs, par,
-                             ec);
+    put(g, e - 1, max(L, -1), min(R, n), d_at);
   }
   __syncthreads();
 
@@ -520,10 +556,18 @@ __device__ __forceinline__ void tree_tile(unsigned char* smem_raw, TreeTileShare
     const int D = delta(codes[g], codes[g + 1]);
     int first_key, last_key;
     coop_node_keys<K>(codes, n, g, D, &first_key, &last_key);
-    if (lane == 0)
-      write_gap_node<K, EDGES, LESS>(g, n, D, first_key - 1, last_key, d_glob, root_true_delta,
-                               root_prefix, pn, l8, r8, lcs, par,
-                               ec);
+    if (lane == 0) put(g, D, first_key - 1, last_key, d_glob);
+  }
+  if (EDGES) {
+    sum0 = __reduce_add_sync(0xffffffffu, sum0);
+    sum1 = __reduce_add_sync(0xffffffffu, sum1);
+    if (lane == 0) {
+      if (sum0) atomicAdd(&sh.sum[0], sum0);
+      if (sum1) atomicAdd(&sh.sum[1], sum1);
+    }
+    __syncthreads();
+    if (threadIdx.x < kTreeSums && sh.sum[threadIdx.x])
+      atomicAdd(sums + t0 + threadIdx.x, uint32_t(sh.sum[threadIdx.x]));
   }
 }
 
