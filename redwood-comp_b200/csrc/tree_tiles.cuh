@@ -571,6 +571,9 @@ __device__ __forceinline__ void tree_tile(unsigned char* smem_raw, TreeTileShare
   }
 }
 
+// x / 3 for 0 <= x < 256.
+__device__ __forceinline__ int third(int x) { return (x * 171) >> 9; }
+
 // ---------------------------------------------------------------------------
 // stage 7: octree rows and links (func_octree.hpp:28-112)
 // ---------------------------------------------------------------------------
@@ -598,11 +601,13 @@ __device__ __forceinline__ OctSeg oct_segment(const SegTable& seg, const OctOut&
                                               const uint32_t* n_octree, int32_t* seg_err,
                                               uint32_t c, bool report) {
   OctSeg r{};
+  // (both loads go out together)
   const uint32_t nu = *reinterpret_cast<const volatile uint32_t*>(n_unique + c);
+  const uint32_t m = *reinterpret_cast<const volatile uint32_t*>(n_octree + c);
   r.ok = nu >= 3 && nu != RW_COUNT_UNSET && nu <= seg_size(seg, c);
   if (!r.ok) return r;
   r.n = int(nu - 1);
-  r.m = *reinterpret_cast<const volatile uint32_t*>(n_octree + c);
+  r.m = m;
   r.row0 = o.oct_off ? o.oct_off[c] : 0u;
   r.cap = o.oct_off ? o.oct_off[c + 1] - o.oct_off[c] : o.capacity;
   r.counts = true;
@@ -674,9 +679,13 @@ constexpr uint32_t kFarFromParent = 0, kFarFromStep = 1, kFarFinal = 2, kFarLoca
 // global atomics; a list that overflows makes the far kernel apply every
 // link again (the atomics are idempotent).
 //
-// Threads take the tile's rows in turn (row r by thread r mod threads), so
-// that every lane has a row; the owner comes from a binary search over the
-// tile's first rows.
+// A thread loads four consecutive nodes as vectors and names itself the owner
+// of their rows in shared memory; then threads take the tile's rows in turn
+// (row r by thread r mod threads), so that every lane has a row.  The kernel is
+// bound by its instructions: with four nodes 256 apart per thread, a scan per
+// group of them and a binary search over the tile's first rows for each row's
+// owner it executed 156M of them instead of 146M and took 183.9 instead of 170.0
+// us at 16.8M uniform points (5,000,011 64-bit keys: 75.7, now 71.8).
 //
 // Node 0 owns no row; tile 0 writes the root initialisation when there is
 // no octree row at all (07_octree.cu:188-198) and clears the spare row m
@@ -691,17 +700,17 @@ struct OctTileShared {
   // k = 0 row of each node: child slot values relative to the tile's first
   // row, plus one (0: no child; the nonzero slots are the node mask)
   uint4 child[kOctTile];  // 8 x u16
-  K code[kOctTile];
+  alignas(16) K code[kOctTile];
   // first row of each node relative to the tile's first row (a tile's rows
   // number at most kTile times the largest count, 21 levels; 0xffff past the
   // tile's nodes); [kOctTile]: end of the tile's rows
-  uint16_t off[kOctTile + 2];
+  alignas(8) uint16_t off[kOctTile + 4];
   // per node: (count class << 12) | tile-relative parent (0xfff: outside);
   // class 0: count 0, 1: count > 0, 2: count < 0
-  uint16_t node[kOctTile];
+  alignas(8) uint16_t node[kOctTile];
   uint16_t owner[kOctTile];  // of the first rows
-  uint8_t level[kOctTile];   // prefix_n / 3
-  uint32_t wsum[4 * (kOctThreads / 32) + 1];
+  alignas(4) uint8_t level[kOctTile];  // prefix_n / 3
+  uint32_t wsum[kOctThreads / 32];
 };
 
 // The tile of nodes from tile0 on, of a segment os (number c) whose arrays are
@@ -718,70 +727,124 @@ __device__ __forceinline__ void octree_tile(
   constexpr int kTile = int(kOctTile);
   constexpr int kRowCap = kTile;  // rows whose owner is kept
   static_assert(kTile < 0xfff && (kTile & (kTile - 1)) == 0, "12-bit parents, 2^k tile");
-  static_assert(kTile == 4 * kOctThreads && 4 * (kOctThreads / 32) == 32,
-                "four groups of 256 nodes, 32 warp sums");
+  static_assert(kTile == 4 * kOctThreads, "four nodes per thread");
   const int n = os.n;
   const uint32_t m = os.m;
   const int tile_end = min(tile0 + kTile, n);
 
-  // thread tid: nodes tile0 + tid + 256 q, q < 4 (coalesced loads)
-  int ev[4], ov[4];
+  // thread tid: nodes tile0 + 4 tid + q, q < 4, as vectors; a tile that ends
+  // early or starts off a 16-byte boundary (a cloud of a batch) goes through
+  // shared memory, in the place of the child slots
+  static_assert(kOctNpt == 4, "four nodes per thread");
+  auto low = [](const void* p) { return uint32_t(reinterpret_cast<uintptr_t>(p)); };
+  const bool vec = tile_end == tile0 + kTile && (low(prefix_n + tile0) & 3u) == 0 &&
+                   ((low(ec + tile0) | low(parents + tile0) | low(off + tile0) |
+                     low(codes + tile0)) & 15u) == 0;
+  const uint32_t base = OFFS ? first_row() : 0u;
+  const int root_level = prefix_n[0] / 3;
+  const int n0 = 4 * tid;  // the thread's first node in the tile
+  int* tmp = reinterpret_cast<int*>(sh.child);
+  int4 e4, p4, o4 = make_int4(0, 0, 0, 0);
+  if (vec) {
+    e4 = reinterpret_cast<const int4*>(ec + tile0)[tid];
+    p4 = reinterpret_cast<const int4*>(parents + tile0)[tid];
+    if (!OFFS) o4 = reinterpret_cast<const int4*>(off + tile0)[tid];
+    const uint32_t pre = reinterpret_cast<const uint32_t*>(prefix_n + tile0)[tid];
+    constexpr int kCodeVecs = int(sizeof(K)) / 4;  // of 16 bytes
+#pragma unroll
+    for (int q = 0; q < kCodeVecs; ++q)
+      reinterpret_cast<uint4*>(sh.code)[tid * kCodeVecs + q] =
+          reinterpret_cast<const uint4*>(codes + tile0)[tid * kCodeVecs + q];
+    *reinterpret_cast<uint32_t*>(sh.level + n0) =
+        uint32_t(third(pre & 255u)) | uint32_t(third(pre >> 8 & 255u)) << 8 |
+        uint32_t(third(pre >> 16 & 255u)) << 16 | uint32_t(third(pre >> 24)) << 24;
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int t = tid + q * kOctThreads;
+      const int i = tile0 + t;
+      const bool valid = i < tile_end;
+      tmp[t] = valid ? ec[i] : 0;
+      tmp[kTile + t] = valid ? parents[i] : -1;
+      if (!OFFS) tmp[2 * kTile + t] = valid ? off[i] : 0;
+      sh.code[t] = valid ? codes[i] : K(0);
+      sh.level[t] = valid ? uint8_t(third(prefix_n[i])) : uint8_t(0);
+    }
+    sync();
+    e4 = reinterpret_cast<const int4*>(tmp)[tid];
+    p4 = reinterpret_cast<const int4*>(tmp + kTile)[tid];
+    if (!OFFS) o4 = reinterpret_cast<const int4*>(tmp + 2 * kTile)[tid];
+    sync();
+  }
+  const int ev[4] = {e4.x, e4.y, e4.z, e4.w}, pa[4] = {p4.x, p4.y, p4.z, p4.w};
+  int ov[4] = {o4.x, o4.y, o4.z, o4.w};
+  uint32_t word[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    const int t = tid + q * kOctThreads;
-    const int i = tile0 + t;
-    const bool valid = i < tile_end;
-    ev[q] = valid ? ec[i] : 0;
-    const int pa = valid ? parents[i] : -1;
-    const int pr = pa >= tile0 && pa < tile_end ? pa - tile0 : 0xfff;
-    sh.node[t] = uint16_t((ev[q] == 0 ? 0 : ev[q] > 0 ? 1 : 2) << 12 | pr);
-    ov[q] = (!OFFS && valid) ? off[i] : 0;
-    sh.code[t] = valid ? codes[i] : K(0);
-    sh.level[t] = valid ? uint8_t(prefix_n[i] / 3) : uint8_t(0);
-    sh.child[t] = make_uint4(0, 0, 0, 0);
+    const uint32_t pr = uint32_t(pa[q] - tile0) < uint32_t(tile_end - tile0)
+                            ? uint32_t(pa[q] - tile0) : 0xfffu;
+    word[q] = (ev[q] == 0 ? 0u : ev[q] > 0 ? 1u : 2u) << 12 | pr;
   }
+  *reinterpret_cast<uint2*>(sh.node + n0) =
+      make_uint2(word[0] | word[1] << 16, word[2] | word[3] << 16);
   uint32_t rows_end = 0;
   int rbase = 0;  // the tile's first row
   if (OFFS) {
-    // exclusive scan of the counts in node order, as stage 6 computes it: a
-    // warp scan per group of 32 nodes, then one warp scans the 32 group sums
+    // exclusive scan of the counts in node order, as stage 6 computes it
     const uint32_t lane = lane_id(), warp = uint32_t(tid) >> 5;
-    uint32_t inc[4];
+    const uint32_t sum = uint32_t(ev[0]) + uint32_t(ev[1]) + uint32_t(ev[2]) + uint32_t(ev[3]);
+    const uint32_t inc = warp_inclusive_scan(sum);
+    if (lane == 31) sh.wsum[warp] = inc;
+    sync();
+    uint32_t run = base + inc - sum;
+    rows_end = base;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      inc[q] = warp_inclusive_scan(uint32_t(ev[q]));
-      if (lane == 31) sh.wsum[q * (kOctThreads / 32) + warp] = inc[q];
+    for (int w = 0; w < kOctThreads / 32; ++w) {
+      const uint32_t x = sh.wsum[w];
+      run += uint32_t(w) < warp ? x : 0u;
+      rows_end += x;
     }
-    sync();
-    if (warp == 0) {
-      const uint32_t v = sh.wsum[lane];
-      const uint32_t wi = warp_inclusive_scan(v);
-      sh.wsum[lane] = wi - v;
-      if (lane == 31) sh.wsum[32] = wi;
-    }
-    sync();
-    const uint32_t base = first_row();
     rbase = int(base);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      ov[q] = int32_t(base + sh.wsum[q * (kOctThreads / 32) + warp] + inc[q] - uint32_t(ev[q]));
-      const int i = tile0 + tid + q * kOctThreads;
-      if (i < tile_end) off[i] = ov[q];
+      ov[q] = int32_t(run);
+      run += uint32_t(ev[q]);
     }
-    rows_end = base + sh.wsum[32];
+    if (vec) {
+      reinterpret_cast<int4*>(off + tile0)[tid] = make_int4(ov[0], ov[1], ov[2], ov[3]);
+    } else {
+      reinterpret_cast<int4*>(tmp)[tid] = make_int4(ov[0], ov[1], ov[2], ov[3]);
+      sync();
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int t = tid + q * kOctThreads;
+        if (tile0 + t < tile_end) off[tile0 + t] = tmp[t];
+      }
+      sync();
+    }
   } else {
     rbase = off[tile0];
+    rows_end = uint32_t(tile_end < n ? off[tile_end] : int(m));
   }
   if (!os.ok) return;  // the whole block: no octree row is written
-  // relative rows kept in [0, 0xfffe] (offsets made by stage 6 stay far inside)
-  auto rel16 = [&](int v) -> uint16_t { return uint16_t(min(max(v - rbase, 0), 0xfffe)); };
+  // relative rows kept in [0, 0xfffe] (offsets made by stage 6 stay far inside);
+  // the entry behind the tile's last node is the end of its rows, 0xffff follows
+  auto rel16 = [&](int v) -> uint32_t { return uint32_t(min(max(v - rbase, 0), 0xfffe)); };
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    const int t = tid + q * kOctThreads;
-    sh.off[t] = tile0 + t < tile_end ? rel16(ov[q]) : uint16_t(0xffff);
+    sh.child[tid + q * kOctThreads] = make_uint4(0, 0, 0, 0);
+    const int i = tile0 + n0 + q;
+    word[q] = i < tile_end ? rel16(ov[q]) : i == tile_end ? rel16(int(rows_end)) : 0xffffu;
+    // the rows' owner
+    if (i < tile_end) {
+      const int r = int(word[q]);
+      for (int k = 0; k < min(ev[q], 32) && r + k < kRowCap; ++k) sh.owner[r + k] = uint16_t(n0 + q);
+    }
   }
+  *reinterpret_cast<uint2*>(sh.off + n0) =
+      make_uint2(word[0] | word[1] << 16, word[2] | word[3] << 16);
   if (tid == 0) {
-    sh.off[kTile] = rel16(OFFS ? int(rows_end) : (tile_end < n ? off[tile_end] : int(m)));
+    sh.off[kTile] = uint16_t(rel16(int(rows_end)));
     if (tile0 == 0) {
       const size_t rm = size_t(os.row0) + m;
       int4* row = reinterpret_cast<int4*>(o.children + 8 * rm);
@@ -790,7 +853,6 @@ __device__ __forceinline__ void octree_tile(
       o.node_mask[rm] = 0;
       o.leaf_mask[rm] = 0;
       if (m == 0) {
-        const int root_level = prefix_n[0] / 3;
         const K pre = codes[0] >> (B - 3 * root_level);
         o.corner[os.row0] = decode<K>(K(pre << (B - 3 * root_level)), min_coord, range);
         o.cell_size[os.row0] = range;
@@ -798,12 +860,10 @@ __device__ __forceinline__ void octree_tile(
     }
   }
   sync();
-  if (tile_end < tile0 + kTile && tid == 0) sh.off[tile_end - tile0] = sh.off[kTile];
-  sync();
 
   const int rend = min(rbase + int(sh.off[kTile]), int(m));  // rows [rbase, rend)
-  const int root_level = prefix_n[0] / 3;
   auto owner_of = [&](int r) -> int {  // last node whose first row is <= rbase + r
+    if (r < kRowCap) return int(sh.owner[r] & (kTile - 1));
     int t = 0;
 #pragma unroll
     for (int step = kTile / 2; step >= 1; step >>= 1)
@@ -821,7 +881,6 @@ __device__ __forceinline__ void octree_tile(
   for (int r = tid; rbase + r < rend; r += kOctThreads) {
     const int p = rbase + r;
     const int t = owner_of(r);
-    if (r < kRowCap) sh.owner[r] = uint16_t(t);
     if (r != int(sh.off[t + 1]) - 1) continue;  // not the top row of its chain
     const int level = int(sh.level[t]) - (r - int(sh.off[t]));  // the top row's level
     const int slot = int((sh.code[t] >> (B - 3 * level)) & K(7));
@@ -881,7 +940,7 @@ __device__ __forceinline__ void octree_tile(
   // rows
   for (int r = tid; rbase + r < rend; r += kOctThreads) {
     const int p = rbase + r;
-    const int t = r < kRowCap ? int(sh.owner[r]) : owner_of(r);
+    const int t = owner_of(r);
     const size_t rp = size_t(os.row0) + uint32_t(p);
     const int k = r - int(sh.off[t]);
     const int level = int(sh.level[t]) - k;
