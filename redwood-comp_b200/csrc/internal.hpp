@@ -246,11 +246,11 @@ cudaError_t launch_leaf_links(const Bufs& b, const Scratch& sc, const Plan& pl,
                               cudaStream_t s);
 
 // ---- a small cloud's whole pipeline in one launch (k_small.cu) ----------------
-// It takes clouds up to these sizes, where a bucket still has room for 2.4
+// It takes clouds up to these sizes, where a bucket still has room for 1.9
 // shares of 148 blocks; it is faster than the general chain of kernels up to
-// there (750,000 points 103 against 134 us, 32-bit keys; 400,000 points 82
-// against 155 us, 64-bit keys).
-constexpr uint32_t kSmallLimit32 = 880000, kSmallLimit64 = 440000;
+// there (a call with 1,000,003 points 123 against 138 us, 32-bit keys; 549,000
+// points 100 against 129 us, 64-bit keys).
+constexpr uint32_t kSmallLimit32 = 1100000, kSmallLimit64 = 550000;
 // Sets the kernels up on the current device; *usable: a block of them fits an SM.
 cudaError_t small_prepare(int key_bits, bool* usable);
 uint32_t small_limit(int key_bits);

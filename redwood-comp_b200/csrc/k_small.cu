@@ -8,13 +8,13 @@
 // and the steps are separated by barriers over the grid (1.3 us each, 2.3 with
 // stores to drain; none when one block takes the cloud).  A call with its wait,
 // before and now, 32-bit keys: 2,000 points 100 and 43 us, 4,096 100 and 54,
-// 20,000 100 and 57, 303,104 110 and 71, 600,000 126 and 85; 64-bit keys: 4,200
-// points 123 and 58 us, 303,104 143 and 77, 400,000 155 and 82.  What is left is
+// 20,000 100 and 59, 303,104 110 and 72, 600,000 126 and 88; 64-bit keys: 4,200
+// points 123 and 57 us, 303,104 143 and 77, 400,000 155 and 83.  What is left is
 // latency: eight barriers, and chains of dependent shared-memory and L2
 // accesses in every step.
 //
-// Sort: one exchange instead of one per digit.  Every block gives 32 sampled
-// keys; the samples' exact ranks yield a splitter per block; every block sends
+// Sort: one exchange instead of one per digit.  Every block gives one or two
+// lists of 32 sampled keys; the samples' exact ranks yield a splitter per block; every block sends
 // its keys to the blocks that own them (bucket regions filled through one
 // atomic counter each) and sorts what it receives in shared memory by 8-bit
 // digits, leaving out the digits that all its keys share.  Keys equal to a
@@ -35,7 +35,7 @@
 namespace rwt {
 
 constexpr int kSmThreads = 1024, kSmWarps = kSmThreads / 32;
-constexpr int kSmSamples = 32;    // per block: one per warp when they are ranked
+constexpr int kSmSamples = 32;    // of a list: one per warp when they are ranked
 constexpr int kSmEncode = 8;      // points per thread of a block's share
 constexpr int kSmMaxBlocks = 256;
 constexpr int kSmGroups = kSmThreads / kOctThreads;  // octree tiles at a time per block
@@ -57,7 +57,8 @@ struct SmallCfg {
 struct SmallArgs {
   const float4* points;
   void *keys, *alt;
-  uint32_t n, chunk, cap;  // points, points per block, keys per bucket region
+  // points, points per block, keys per bucket region, sample lists per block
+  uint32_t n, chunk, cap, lists;
   float min_coord, range, inv_range;
   uint8_t *prefix_n, *hl, *hr;
   int32_t *lc, *parents, *edge_count, *edge_offset;
@@ -86,16 +87,16 @@ struct SmallShared {
 // they end.  Digits that all keys share are left out.  The keys are filled up
 // to whole steps with the largest word, which stays behind them.
 //
-// A few thousand keys rarely share the first kSortBits bits of those in which
-// they differ: only these are sorted by digits (three passes instead of four
-// to eight, 2.1 us each), then every key of a run that shares them finds its
-// place by counting the run's smaller keys: 64-bit keys, 3,001 points 20.0 ->
-// 9.0 us of sorting, 307,200 points 20.2 -> 10.1.  A run beyond kSortRun keys
+// A few thousand keys rarely share the first 24 bits of those in which they
+// differ: with `bits` 24 only these are sorted by digits (three passes instead
+// of four to eight, 2.1 us each), then every key of a run that shares them finds
+// its place by counting the run's smaller keys: 64-bit keys, 3,001 points 20.0
+// -> 9.0 us of sorting, 307,200 points 20.2 -> 10.1.  A run beyond kSortRun keys
 // sends the block through all digits.
-constexpr int kSortBits = 24, kSortRun = 32;
+constexpr int kSortRun = 32;
 
 template <typename K>
-__device__ K* block_sort(K* a, K* b, int c, uint32_t* hist, uint32_t* next, SmallShared& sh) {
+__device__ K* block_sort(K* a, K* b, int c, int bits, uint32_t* hist, uint32_t* next, SmallShared& sh) {
   constexpr int kBits = KeyTraits<K>::kCodeBits;
   if (c < 2) return a;
   const int steps = (c + kSortThreads - 1) / kSortThreads;
@@ -116,7 +117,7 @@ __device__ K* block_sort(K* a, K* b, int c, uint32_t* hist, uint32_t* next, Smal
   }
   __syncthreads();
   const K all = sizeof(K) == 8 ? K(uint64_t(sh.diff[1]) << 32 | sh.diff[0]) : K(sh.diff[0]);
-  const int low = max(KeyTraits<K>::kWordBits - KeyTraits<K>::clz(all) - kSortBits, 0);
+  const int low = max(KeyTraits<K>::kWordBits - KeyTraits<K>::clz(all) - bits, 0);
   for (int from = low;; from = 0) {
     for (int shift = from; shift < kBits && (all >> shift); shift += 8) {
       if (((all >> shift) & K(255)) == 0) continue;
@@ -210,19 +211,26 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
   __syncthreads();
 
   // ---- stage 2 ----
+  // 30-bit codes of a large cloud have such runs wherever it is dense: 899,000
+  // mixture points took 138 us with 24 bits and take 118 with all (uniform ones
+  // 117 and 119; up to 2^18 points 24 bits gain 2 us in both)
+  const int bits = sizeof(K) == 4 && a.n > (1u << 18) ? KeyTraits<K>::kCodeBits : 24;
   K* sorted = nullptr;  // this block's run of the sorted keys, in shared memory
   int c = mine;
   uint32_t base = p0;  // its place among all
   if (P == 1) {
-    sorted = block_sort<K>(sa, sb, c, hist, next, sh);
+    sorted = block_sort<K>(sa, sb, c, bits, hist, next, sh);
   } else {
     K* samples = static_cast<K*>(a.samples);
     K* splitters = static_cast<K*>(a.splitters);
-    if (warp == 0) {
-      // one key of each of 32 strata, sorted within the warp; a share without a
-      // key stands for the largest one
-      const uint32_t lo = uint32_t(uint64_t(mine) * lane / kSmSamples),
-                     hi = uint32_t(uint64_t(mine) * (lane + 1) / kSmSamples);
+    const int R = int(a.lists);
+    if (warp < R) {
+      // one key of each of 32 strata of the share (of 64, the second list the
+      // other half), sorted within the warp; a share without a key stands for
+      // the largest one
+      const int t = warp * kSmSamples + lane, strata = R * kSmSamples;
+      const uint32_t lo = uint32_t(uint64_t(mine) * t / strata),
+                     hi = uint32_t(uint64_t(mine) * (t + 1) / strata);
       static_assert(kSmSamples == 32, "a lane per sample");
       K k = mine == 0 ? K(~K(0)) : sa[hi > lo ? lo + small_hash(p0 + lo) % (hi - lo) : lo];
 #pragma unroll
@@ -233,40 +241,40 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
           const bool up = (lane & size) == 0, low = (lane & st) == 0;
           k = (low == up) == (other < k) ? other : k;
         }
-      samples[b * kSmSamples + lane] = k;
+      samples[(int(b) * R + warp) * kSmSamples + lane] = k;
     }
     if (!bar.sync()) return;
-    const int ns = int(P) * kSmSamples;
-    constexpr int kPitch = kSmSamples + 1;  // a block's samples: lanes in different banks
-    K* ss = sb;
-    for (int i = tid; i < ns; i += kSmThreads)
+    const int nl = int(P) * R;  // lists
+    constexpr int kPitch = kSmSamples + 1;  // a list's samples: lanes in different banks
+    K* ss = sa + mine;  // behind the keys (small_takes: there is room)
+    for (int i = tid; i < nl * kSmSamples; i += kSmThreads)
       ss[i / kSmSamples * kPitch + i % kSmSamples] = samples[i];
     __syncthreads();
-    {
+    for (int own = int(b) * R; own < int(b + 1) * R; ++own) {
       // the exact rank of this warp's sample among all, ties in their order:
-      // a search in every block's sorted samples; every kSmSamples-th is a
-      // splitter
-      static_assert(kSmSamples == kSmWarps, "a warp ranks one sample");
-      const K my = ss[int(b) * kPitch + warp];
+      // a search in every list; every (32 R)-th sample is a splitter
+      static_assert(kSmSamples == kSmWarps, "a warp ranks one sample of a list");
+      const K my = ss[own * kPitch + warp];
       uint32_t r = 0;
-      for (int j = lane; j < int(P); j += 32) {
+      for (int j = lane; j < nl; j += 32) {
         const K* q = ss + j * kPitch;
-        if (j == int(b)) {
+        if (j == own) {
           r += uint32_t(warp);
         } else {
-          // keys of block j below my sample, or not above it if j comes first
+          // keys of list j below my sample, or not above it if j comes first
           uint32_t at = 0;
 #pragma unroll
           for (int st = kSmSamples / 2; st > 0; st >>= 1) {
             const K x = q[at + st - 1];
-            if (x < my || (j < int(b) && x == my)) at += st;
+            if (x < my || (j < own && x == my)) at += st;
           }
           const K x = q[at];
-          r += at + uint32_t(x < my || (j < int(b) && x == my));
+          r += at + uint32_t(x < my || (j < own && x == my));
         }
       }
       r = warp_sum(r);
-      if (lane == 0 && r && r % kSmSamples == 0) splitters[r / kSmSamples - 1] = my;
+      if (lane == 0 && r && r % uint32_t(kSmSamples * R) == 0)
+        splitters[r / uint32_t(kSmSamples * R) - 1] = my;
     }
     if (!bar.sync()) return;
     const int nspl = int(P) - 1;
@@ -334,7 +342,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
       const K* mineq = region + size_t(b) * a.cap;
       for (int i = tid; i < c; i += kSmThreads) sa[i] = mineq[i];
       __syncthreads();
-      sorted = block_sort<K>(sa, sb, c, hist, next, sh);
+      sorted = block_sort<K>(sa, sb, c, bits, hist, next, sh);
     } else {
       // digit by digit over the grid: every block ranks its share, the counts
       // of all blocks give its keys' places
@@ -528,12 +536,24 @@ uint32_t small_blocks(uint32_t n, int sms) {
   return std::min({div_up(n, kSmShare), uint32_t(sms), uint32_t(kSmMaxBlocks)});
 }
 
-// Keys of a bucket region: three times the mean and a little, which a bucket
-// between two splitters of 32 samples each passes with a probability below
-// 1e-8 (the mass between them has a standard deviation of 0.18 means).
+// Keys of a bucket region: three times the mean and a little, at most what a
+// block sorts.
 uint32_t small_cap(uint32_t n, uint32_t blocks, int key_bits) {
   const uint32_t most = key_bits == 32 ? SmallCfg<uint32_t>::kCap : SmallCfg<uint64_t>::kCap;
   return std::min(most, 3 * div_up(n, blocks) + 512);
+}
+
+// Sample lists per block; 0: the cloud is too large.  A bucket between two
+// splitters with 32 samples each holds a mass of standard deviation 0.18 means
+// and more than 2.4 means once in 10^7, one with 64 samples 0.125 and more than
+// 1.9 once in 10^7.
+uint32_t small_lists(uint32_t n, uint32_t blocks, int key_bits) {
+  const uint32_t share = div_up(n, blocks), cap = small_cap(n, blocks, key_bits);
+  if (share > uint32_t(kSmEncode * kSmThreads)) return 0;
+  if (blocks == 1 || 12 * share <= 5 * cap) return 1;
+  // (64 samples of every block fit behind a share's keys)
+  const uint32_t room = 2u * (key_bits == 32 ? SmallCfg<uint32_t>::kCap : SmallCfg<uint64_t>::kCap);
+  return 19 * share <= 10 * cap && share + blocks * 2u * (kSmSamples + 1) <= room ? 2 : 0;
 }
 
 template <typename K, int LESS>
@@ -572,10 +592,7 @@ uint32_t small_limit(int key_bits) { return key_bits == 32 ? kSmallLimit32 : kSm
 
 bool small_takes(uint32_t n, int key_bits, int sms) {
   if (n > small_limit(key_bits)) return false;
-  const uint32_t blocks = small_blocks(n, sms), share = div_up(n, blocks);
-  // a share is encoded in registers, and a bucket has room for 2.4 of them
-  const uint32_t cap = small_cap(n, blocks, key_bits);
-  return share <= uint32_t(kSmEncode * kSmThreads) && (blocks == 1 || 12 * share <= 5 * cap);
+  return small_lists(n, small_blocks(n, sms), key_bits) != 0;
 }
 
 cudaError_t small_prepare(int key_bits, bool* usable) {
@@ -600,7 +617,7 @@ SmallLayout small_layout(uint32_t n_cap, int key_bits, int sms) {
   SmallLayout l{};
   size_t o = 0;
   auto take = [&](size_t bytes) { const size_t at = o; o += up(bytes); return at; };
-  l.samples = take(P * kSmSamples * ks);
+  l.samples = take(P * 2 * kSmSamples * ks);
   l.splitters = take(P * ks);
   l.first = take(P * ks);
   l.last = take(P * ks);
@@ -631,6 +648,7 @@ cudaError_t launch_small(const Bufs& b, const Scratch& sc, uint32_t n, uint32_t 
   a.n = n;
   a.chunk = div_up(n, blocks);
   a.cap = small_cap(n, blocks, b.key_bits);
+  a.lists = small_lists(n, blocks, b.key_bits);
   if (!small_takes(n, b.key_bits, sc.num_sms) || n > n_cap) return cudaErrorInvalidValue;
   a.min_coord = b.min_coord;
   a.range = b.range;

@@ -48,7 +48,8 @@ def test_sizes(rw, oracle, n, kind, key_bits):
 
 
 @pytest.mark.parametrize("key_bits,n", [(32, 148 * SHARE - 1), (32, 148 * SHARE + 1), (32, 879999),
-                                        (32, 880001), (64, 440000), (64, 440001)])
+                                        (32, 890000), (32, 1100000), (32, 1100001),
+                                        (64, 442000), (64, 550000), (64, 550001)])
 def test_largest(rw, oracle, n, key_bits):
     check(rw, oracle, cloud(rw, n, "gauss", 3), key_bits, label=f"{n} {key_bits}")
 
