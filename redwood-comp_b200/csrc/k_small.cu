@@ -512,10 +512,9 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
   if (a.leaves) {
     if (!bar.sync()) return;
     leaf_claim<K>(keys, a.prefix_n, a.hl, a.hr, a.lc, a.parents, a.edge_count, a.edge_offset,
-                  a.o.children, a.o.leaf_mask, &a.status->n_unique, a.o.capacity);
-    if (!bar.sync()) return;
-    leaf_write<K>(keys, a.prefix_n, a.hl, a.hr, a.lc, a.parents, a.edge_count, a.edge_offset,
                   a.o.children, &a.status->n_unique, a.o.capacity);
+    if (!bar.sync()) return;
+    leaf_write(a.lc, a.o.children, &a.status->n_unique, &a.status->n_octree_nodes, a.o.capacity);
   }
   if (b == 0 && tid == 0) finish(m);  // (tile 0 is this thread's)
 }

@@ -503,22 +503,18 @@ __global__ void __launch_bounds__(256)
                  const uint8_t* __restrict__ hl, const uint8_t* __restrict__ hr,
                  const int32_t* __restrict__ lc, const int32_t* __restrict__ par,
                  const int32_t* __restrict__ ec, const int32_t* __restrict__ off,
-                 int32_t* __restrict__ children, int32_t* __restrict__ leaf_mask,
-                 const uint32_t* __restrict__ n_unique, uint32_t rows) {
-  pdl_enter();
-  leaf_claim<K>(codes, pn, hl, hr, lc, par, ec, off, children, leaf_mask, n_unique, rows);
-}
-
-template <typename K>
-__global__ void __launch_bounds__(256)
-    k_leaf_write(const K* __restrict__ codes, const uint8_t* __restrict__ pn,
-                 const uint8_t* __restrict__ hl, const uint8_t* __restrict__ hr,
-                 const int32_t* __restrict__ lc, const int32_t* __restrict__ par,
-                 const int32_t* __restrict__ ec, const int32_t* __restrict__ off,
                  int32_t* __restrict__ children, const uint32_t* __restrict__ n_unique,
                  uint32_t rows) {
   pdl_enter();
-  leaf_write<K>(codes, pn, hl, hr, lc, par, ec, off, children, n_unique, rows);
+  leaf_claim<K>(codes, pn, hl, hr, lc, par, ec, off, children, n_unique, rows);
+}
+
+__global__ void __launch_bounds__(256)
+    k_leaf_write(const int32_t* __restrict__ lc, int32_t* __restrict__ children,
+                 const uint32_t* __restrict__ n_unique, const uint32_t* __restrict__ n_octree,
+                 uint32_t rows) {
+  pdl_enter();
+  leaf_write(lc, children, n_unique, n_octree, rows);
 }
 
 // ---------------------------------------------------------------------------
@@ -617,12 +613,11 @@ namespace {
 template <typename K>
 cudaError_t leaf_links_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_t s) {
   const K* codes = static_cast<const K*>(b.keys);
-  const int grid = std::max(1, sc.num_sms * 4);
+  const int grid = std::max(1, sc.num_sms * 8);
   launch_pdl(k_leaf_claim<K>, grid, 256, 0, s, codes, b.prefix_n, b.hl, b.hr, b.lc, b.parents,
-             b.edge_count, b.edge_offset, b.children, b.leaf_mask, pl.n_unique,
-             pl.oct_capacity);
-  launch_pdl(k_leaf_write<K>, grid, 256, 0, s, codes, b.prefix_n, b.hl, b.hr, b.lc, b.parents,
              b.edge_count, b.edge_offset, b.children, pl.n_unique, pl.oct_capacity);
+  launch_pdl(k_leaf_write, grid, 256, 0, s, b.lc, b.children, pl.n_unique, pl.n_octree,
+             pl.oct_capacity);
   return cudaGetLastError();
 }
 }  // namespace
