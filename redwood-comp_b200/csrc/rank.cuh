@@ -44,7 +44,10 @@ enum RankMode : int {
   // digits, ballots over only the code's remaining bits for the top pass
   // (skewed top digits put many lanes of a warp on one shared word, which the
   // atomics serialise; ballots cost the same whatever the digits)
-  kRankMixed = 4
+  kRankMixed = 4,
+  // a first pass's mode, not a menu mode: keys alone need no stable first pass,
+  // so a key's rank is what a shared counter of the block returns
+  kRankUnordered = 5
 };
 
 // D ballots, one per digit bit (warp-level multi-split).
