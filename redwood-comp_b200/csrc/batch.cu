@@ -460,12 +460,7 @@ int rw_tree_batch_enqueue(rw_tree_batch* b, const rw_tree_batch_buffers* u, rw_s
   RWB_CUDA(rwt::launch_radix_tree(x, sc, pl, true, false, s));
   RWB_CUDA(rwt::launch_edge_sums(x, sc, pl, s));
   RWB_CUDA(rwt::launch_octree(x, sc, pl, s, nullptr, true));
-  const size_t c = b->n_clouds;
-  RWB_CUDA(cudaMemcpyAsync(b->h_results, b->d_n_unique, 4 * c, cudaMemcpyDeviceToHost, s));
-  RWB_CUDA(cudaMemcpyAsync(b->h_results + c, b->d_n_octree, 4 * c, cudaMemcpyDeviceToHost, s));
-  RWB_CUDA(cudaMemcpyAsync(b->h_results + 2 * c, b->d_seg_err, 4 * c, cudaMemcpyDeviceToHost, s));
-  RWB_CUDA(cudaMemcpyAsync(b->h_results + 3 * c, b->d_status, sizeof(rwt::DevStatus),
-                           cudaMemcpyDeviceToHost, s));
+  RWB_CUDA(rwt::launch_results_out(pl, b->d_status, b->h_results, s));
   return RW_OK;
 }
 

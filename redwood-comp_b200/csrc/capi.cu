@@ -118,13 +118,7 @@ rwt::Plan plan_of(const rw_tree_app_data& a, const rw_tree_im_storage* im) {
 // Device status := the host's counts of `app`, error word cleared (for the
 // per-stage calls whose kernels read the counts on the device).
 int upload_counts(const rw_tree_app_data* app, rw_tree_im_storage* im, cudaStream_t s) {
-  RW_CUDA(cudaStreamSynchronize(s));  // the pinned mirror may still be in use
-  im->h_status->n_unique = app->n_unique;
-  im->h_status->n_octree_nodes = app->n_octree_nodes;
-  im->h_status->err = 0;
-  im->h_status->err_site = 0;
-  RW_CUDA(cudaMemcpyAsync(im->d_status, im->h_status, sizeof(rwt::DevStatus),
-                          cudaMemcpyHostToDevice, s));
+  RW_CUDA(rwt::launch_status_in(scratch_of(im), app->n_unique, app->n_octree_nodes, s));
   return RW_OK;
 }
 
@@ -139,8 +133,7 @@ int clear_all(rw_tree_im_storage* im, cudaStream_t s) {
 
 // Waits for the stream, copies the device status and maps its error word.
 int sync_status(rw_tree_im_storage* im, cudaStream_t s) {
-  RW_CUDA(cudaMemcpyAsync(im->h_status, im->d_status, sizeof(rwt::DevStatus),
-                          cudaMemcpyDeviceToHost, s));
+  RW_CUDA(rwt::launch_status_out(im->d_status, im->h_status, s));
   RW_CUDA(cudaStreamSynchronize(s));
   if (im->h_status->err != 0) {
     char buf[96];
@@ -434,7 +427,7 @@ int rw_tree_run_stage3(rw_tree_app_data* app, rw_tree_im_storage* im,
                        rw_stream_t stream) {
   if (int rc = check(app, im, kKeys | kAlt)) return rc;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (int rc = clear_all(im, s)) return rc;
+  RW_CUDA(rwt::launch_status_in(scratch_of(im), 0, 0, s));
   RW_CUDA(rwt::launch_unique(bufs_of(*app, im), scratch_of(im), plan_of(*app, im), s));
   if (int rc = sync_status(im, s)) return rc;
   app->n_unique = im->h_status->n_unique;
@@ -474,7 +467,6 @@ int rw_tree_run_stage6(rw_tree_app_data* app, rw_tree_im_storage* im,
   if (app->n_unique == RW_COUNT_UNSET) return RW_ERR_NOT_READY;
   if (app->n_unique < 3 || app->n_unique > app->n_input) return RW_ERR_DEGENERATE;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (int rc = clear_all(im, s)) return rc;
   if (int rc = upload_counts(app, im, s)) return rc;
   RW_CUDA(rwt::launch_edge_scan(bufs_of(*app, im), scratch_of(im), plan_of(*app, im), s));
   if (int rc = sync_status(im, s)) return rc;
@@ -560,8 +552,7 @@ int enqueue_impl(rw_tree_app_data* app, rw_tree_im_storage* im, cudaStream_t s,
   RW_CUDA(rwt::launch_octree(b, sc, pl, s, ev ? ev + k : nullptr, true));
   if (ev) k += 2;
   if (im->options & RW_TREE_OPT_LINK_LEAVES) RW_CUDA(rwt::launch_leaf_links(b, sc, pl, s));
-  RW_CUDA(cudaMemcpyAsync(im->h_status, im->d_status, sizeof(rwt::DevStatus),
-                          cudaMemcpyDeviceToHost, s));
+  RW_CUDA(rwt::launch_status_out(im->d_status, im->h_status, s));
   if (n_ev) *n_ev = k;
   return RW_OK;
 }

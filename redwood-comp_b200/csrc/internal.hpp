@@ -241,6 +241,15 @@ cudaError_t launch_edge_sums(const Bufs& b, const Scratch& sc, const Plan& pl, c
 cudaError_t launch_octree(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_t s,
                           cudaEvent_t* marks = nullptr, bool fused_offsets = false);
 
+// Device status := the given counts, no error, no far links (before a stage that
+// runs alone); device status -> pinned host memory; a batch's counts, errors and
+// status -> pinned host memory (3 x segments words, then the status).
+cudaError_t launch_status_in(const Scratch& sc, uint32_t n_unique, uint32_t n_octree,
+                             cudaStream_t s);
+cudaError_t launch_status_out(const DevStatus* status, DevStatus* host, cudaStream_t s);
+cudaError_t launch_results_out(const Plan& pl, const DevStatus* status, uint32_t* host,
+                               cudaStream_t s);
+
 // The leaf links after stage 7 (RW_TREE_OPT_LINK_LEAVES), single cloud only.
 cudaError_t launch_leaf_links(const Bufs& b, const Scratch& sc, const Plan& pl,
                               cudaStream_t s);

@@ -518,6 +518,33 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---------------------------------------------------------------------------
+// counts and errors to and from the host
+// ---------------------------------------------------------------------------
+
+// Kernels in the chain of programmatic launches instead of 16-byte copies, which
+// would end it and wait for a copy engine; host memory is pinned.
+__global__ void k_status_in(DevStatus* __restrict__ st, uint32_t n_unique, uint32_t n_octree,
+                            uint32_t* __restrict__ far_n) {
+  pdl_enter();
+  *st = DevStatus{n_unique, n_octree, 0, 0};
+  *far_n = 0;
+}
+
+__global__ void __launch_bounds__(256)
+    k_words_out(const uint32_t* a, const uint32_t* b, const uint32_t* c, uint32_t count,
+                const DevStatus* __restrict__ st, uint32_t* host) {
+  pdl_enter();
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count;
+       i += gridDim.x * blockDim.x) {
+    host[i] = a[i];
+    host[count + i] = b[i];
+    host[2 * count + i] = c[i];
+  }
+  if (blockIdx.x == 0 && threadIdx.x < sizeof(DevStatus) / 4)
+    host[3 * count + threadIdx.x] = reinterpret_cast<const uint32_t*>(st)[threadIdx.x];
+}
+
+// ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
 
@@ -567,15 +594,12 @@ cudaError_t octree_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStrea
   const K* codes = static_cast<const K*>(b.keys);
   const uint32_t tiles = pl.node_map.n_tiles;
   uint32_t* far_n = sc.tile_ctr + kCtrLinks;
-  // the fused pipeline clears every counter when it starts; stage 7 run alone
-  // clears its own (a memset between two kernels would also end the
-  // programmatic launch chain)
-  cudaError_t e = fused_offsets ? cudaSuccess : cudaMemsetAsync(far_n, 0, sizeof(uint32_t), s);
+  // (*far_n is zero: the fused pipeline clears every counter when it starts,
+  // stage 7 run alone brings its counts with launch_status_in)
   // eight blocks of 32-bit keys need nearly all of the SM's shared memory
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(fused_offsets ? k_octree<K, true> : k_octree<K, false>,
-                             cudaFuncAttributePreferredSharedMemoryCarveout,
-                             int(cudaSharedmemCarveoutMaxShared));
+  cudaError_t e = cudaFuncSetAttribute(fused_offsets ? k_octree<K, true> : k_octree<K, false>,
+                                       cudaFuncAttributePreferredSharedMemoryCarveout,
+                                       int(cudaSharedmemCarveoutMaxShared));
   if (e != cudaSuccess) return e;
   if (tiles) {
     if (fused_offsets)
@@ -685,6 +709,25 @@ cudaError_t launch_octree(const Bufs& b, const Scratch& sc, const Plan& pl, cuda
                           cudaEvent_t* marks, bool fused_offsets) {
   return b.key_bits == 32 ? octree_t<uint32_t>(b, sc, pl, s, marks, fused_offsets)
                           : octree_t<uint64_t>(b, sc, pl, s, marks, fused_offsets);
+}
+
+cudaError_t launch_status_in(const Scratch& sc, uint32_t n_unique, uint32_t n_octree,
+                             cudaStream_t s) {
+  launch_pdl(k_status_in, 1, 1, 0, s, sc.status, n_unique, n_octree, sc.tile_ctr + kCtrLinks);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_status_out(const DevStatus* status, DevStatus* host, cudaStream_t s) {
+  launch_pdl(k_words_out, 1, 32, 0, s, nullptr, nullptr, nullptr, 0u, status,
+             reinterpret_cast<uint32_t*>(host));
+  return cudaGetLastError();
+}
+
+cudaError_t launch_results_out(const Plan& pl, const DevStatus* status, uint32_t* host,
+                               cudaStream_t s) {
+  launch_pdl(k_words_out, std::min(32u, div_up(pl.seg.count, 256)), 256, 0, s, pl.n_unique,
+             pl.n_octree, reinterpret_cast<const uint32_t*>(pl.seg_err), pl.seg.count, status, host);
+  return cudaGetLastError();
 }
 
 Plan single_plan(uint32_t n, uint32_t oct_capacity, DevStatus* status, uint32_t sort_tile) {
