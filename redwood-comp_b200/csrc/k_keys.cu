@@ -29,6 +29,20 @@ namespace rwt {
 // stage 1
 // ---------------------------------------------------------------------------
 
+// Digit of pass p of the sort: its lowest bit and its mask.  30-bit codes with
+// 8-bit digits take 8, 8, 7 and 7 bits instead of 8, 8, 8 and 6: the top six bits
+// (a quarter of the box per axis) of a clustered cloud put many lanes of a warp on
+// one counter, the top seven half as many (16.8M mixture points, last two passes
+// 163.8 -> 155.5 us; uniform ones 133.9 -> 134.7).
+template <typename K, int D, int LOW>
+__host__ __device__ constexpr int pass_shift(int p) {
+  return LOW + (sizeof(K) == 4 && D == 8 && p == 3 ? 23 : p * D);
+}
+template <typename K, int D>
+__host__ __device__ constexpr uint32_t pass_mask(int p) {
+  return sizeof(K) == 4 && D == 8 && p == 2 ? 0x7fu : (1u << D) - 1u;
+}
+
 // Points are walked in tiles of kPointTile that never straddle two segments;
 // each CTA takes a contiguous run of tiles, so with HIST its shared-memory
 // histograms are flushed to the segment's global ones only when the segment
@@ -76,7 +90,7 @@ __global__ void __launch_bounds__(256)
       if (HIST) {
 #pragma unroll
         for (int ps = 0; ps < P; ++ps)
-          atomicAdd(&s_hist[ps * RADIX + int((k >> (LOW + ps * D)) & K(RADIX - 1))], 1u);
+          atomicAdd(&s_hist[ps * RADIX + int((k >> pass_shift<K, D, LOW>(ps)) & K(pass_mask<K, D>(ps)))], 1u);
       }
     };
     if (hi - lo == kPointTile) {
@@ -210,7 +224,7 @@ struct BinCfg {
 template <typename K, int D, int THREADS, int KPT, int RANK, int MINB, bool PERSIST, int BB = D>
 __global__ void __launch_bounds__(THREADS, MINB)
     k_binning(const K* __restrict__ in, K* __restrict__ out, SegTable seg, TileMap map,
-              int shift, uint32_t* __restrict__ desc,
+              int shift, uint32_t dmask, uint32_t* __restrict__ desc,
               uint32_t* __restrict__ tile_ctr, DevStatus* __restrict__ st,
               uint32_t spin_limit, const uint32_t* __restrict__ gate,
               const uint32_t* __restrict__ skew) {
@@ -277,7 +291,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
       if (full) {
   #pragma unroll
         for (int i = 0; i < KPT; ++i) {
-          const uint32_t dig = uint32_t(keys[i] >> shift) & (RADIX - 1);
+          const uint32_t dig = uint32_t(keys[i] >> shift) & dmask;
           const uint32_t r = atomicAdd(&s_hist[dig], 1u);
           if (i % 2 == 0) rank16[i / 2] = r;
           else rank16[i / 2] |= r << 16;
@@ -285,7 +299,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
       } else {
   #pragma unroll
         for (int i = 0; i < KPT; ++i) {
-          const uint32_t dig = uint32_t(keys[i] >> shift) & (RADIX - 1);
+          const uint32_t dig = uint32_t(keys[i] >> shift) & dmask;
           const uint32_t r = wbase + 32u * i < n ? atomicAdd(&s_hist[dig], 1u) : 0u;
           if (i % 2 == 0) rank16[i / 2] = r;
           else rank16[i / 2] |= r << 16;
@@ -295,14 +309,14 @@ __global__ void __launch_bounds__(THREADS, MINB)
       if (full) {
   #pragma unroll
         for (int i = 0; i < KPT; ++i) keys[i] = in[hbase + 16u * i];
-        half_rank<D, KPT, true>(keys, rank2, shift, hbase, n, wp);
+        half_rank<D, KPT, true>(keys, rank2, shift, hbase, n, wp, dmask);
       } else {
   #pragma unroll
         for (int i = 0; i < KPT; ++i) {
           const uint32_t idx = hbase + 16u * i;
           keys[i] = idx < n ? in[idx] : K(0);
         }
-        half_rank<D, KPT, false>(keys, rank2, shift, hbase, n, wp);
+        half_rank<D, KPT, false>(keys, rank2, shift, hbase, n, wp, dmask);
       }
     } else if (RANK == kRankMixed) {
       // this segment's digits decide the scheme (block-uniform)
@@ -310,7 +324,8 @@ __global__ void __launch_bounds__(THREADS, MINB)
       if (full) {
   #pragma unroll
         for (int i = 0; i < KPT; ++i) keys[i] = in[wbase + 32u * i];
-        warp_rank<D, KPT, kRankMixed, true, BB>(keys, rank2, shift, wbase, n, wh, wm, KPT, ballots);
+        warp_rank<D, KPT, kRankMixed, true, BB>(keys, rank2, shift, wbase, n, wh, wm, KPT, ballots,
+                                                dmask);
       } else {
   #pragma unroll
         for (int i = 0; i < KPT; ++i) {
@@ -318,19 +333,19 @@ __global__ void __launch_bounds__(THREADS, MINB)
           keys[i] = idx < n ? in[idx] : K(0);
         }
         warp_rank<D, KPT, kRankMixed, false, BB>(keys, rank2, shift, wbase, n, wh, wm, KPT,
-                                                 ballots);
+                                                 ballots, dmask);
       }
     } else if (full) {
   #pragma unroll
       for (int i = 0; i < KPT; ++i) keys[i] = in[wbase + 32u * i];
-      warp_rank<D, KPT, RANK, true, BB>(keys, rank2, shift, wbase, n, wh, wm);
+      warp_rank<D, KPT, RANK, true, BB>(keys, rank2, shift, wbase, n, wh, wm, KPT, false, dmask);
     } else {
   #pragma unroll
       for (int i = 0; i < KPT; ++i) {
         const uint32_t idx = wbase + 32u * i;
         keys[i] = idx < n ? in[idx] : K(0);
       }
-      warp_rank<D, KPT, RANK, false, BB>(keys, rank2, shift, wbase, n, wh, wm);
+      warp_rank<D, KPT, RANK, false, BB>(keys, rank2, shift, wbase, n, wh, wm, KPT, false, dmask);
     }
     __syncthreads();
 
@@ -395,24 +410,24 @@ __global__ void __launch_bounds__(THREADS, MINB)
       if (full) {
   #pragma unroll
         for (int i = 0; i < KPT; ++i) {
-          const uint32_t dig = uint32_t(keys[i] >> shift) & (RADIX - 1);
+          const uint32_t dig = uint32_t(keys[i] >> shift) & dmask;
           s_keys[s_start[dig] + ((rank16[i / 2] >> (16 * (i % 2))) & 0xffffu)] = keys[i];
         }
       } else {
   #pragma unroll
         for (int i = 0; i < KPT; ++i)
           if (wbase + 32u * i < n) {
-            const uint32_t dig = uint32_t(keys[i] >> shift) & (RADIX - 1);
+            const uint32_t dig = uint32_t(keys[i] >> shift) & dmask;
             s_keys[s_start[dig] + ((rank16[i / 2] >> (16 * (i % 2))) & 0xffffu)] = keys[i];
           }
       }
     } else if (RANK == kRankHalfPacked) {
-      if (full) half_place<D, KPT, true>(keys, rank2, shift, hbase, n, wp, s_keys);
-      else half_place<D, KPT, false>(keys, rank2, shift, hbase, n, wp, s_keys);
+      if (full) half_place<D, KPT, true>(keys, rank2, shift, hbase, n, wp, s_keys, dmask);
+      else half_place<D, KPT, false>(keys, rank2, shift, hbase, n, wp, s_keys, dmask);
     } else if (full) {
-      warp_place<D, KPT, true>(keys, rank2, shift, wbase, n, wh, s_keys);
+      warp_place<D, KPT, true>(keys, rank2, shift, wbase, n, wh, s_keys, KPT, dmask);
     } else {
-      warp_place<D, KPT, false>(keys, rank2, shift, wbase, n, wh, s_keys);
+      warp_place<D, KPT, false>(keys, rank2, shift, wbase, n, wh, s_keys, KPT, dmask);
     }
 
     // decoupled look-back, kLookback descriptors per round trip.  The segment's
@@ -462,14 +477,14 @@ __global__ void __launch_bounds__(THREADS, MINB)
       for (int i = 0; i < KPT; ++i) {
         const uint32_t p = tid + uint32_t(i) * THREADS;
         const K k = s_keys[p];
-        const uint32_t dst = s_gofs[uint32_t(k >> shift) & (RADIX - 1)] + p;
+        const uint32_t dst = s_gofs[uint32_t(k >> shift) & dmask] + p;
         if (dst < total) out[dst] = k;
       }
     } else {
       const uint32_t tile_n = n - base;
       for (uint32_t p = tid; p < tile_n; p += THREADS) {
         const K k = s_keys[p];
-        const uint32_t dst = s_gofs[uint32_t(k >> shift) & (RADIX - 1)] + p;
+        const uint32_t dst = s_gofs[uint32_t(k >> shift) & dmask] + p;
         if (dst < total) out[dst] = k;
       }
     }
@@ -528,7 +543,7 @@ cudaError_t passes_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStrea
   constexpr int RT = RANK;                                       // pass P-1
   // bits of the top digit (left out bits are chosen so that it is a full one)
   constexpr int TB = RANK == kRankMixed && !(sizeof(K) == 8 && D == 8)
-                         ? KeyTraits<K>::kCodeBits - (kFull - 1) * D
+                         ? KeyTraits<K>::kCodeBits - pass_shift<K, D, 0>(kFull - 1)
                          : D;
   static_assert((63 - kSplitLow32) % 8 == 0 && (63 - kSplitLow40) % 8 == 0, "full digits");
   constexpr int kSkewLog2 = sizeof(K) == 4 ? 5 : 6;
@@ -581,7 +596,8 @@ cudaError_t passes_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStrea
     e = cudaMemsetAsync(sc.tile_ctr + kCtrSortBase, 0x01, 1, s);
     if (e != cudaSuccess) return e;
     launch_pdl(kern, tiles - 1, THREADS, C::kSmem, s, static_cast<const K*>(keys), alt, pl.seg,
-               pl.sort_map, low, sc.sort_desc, sc.tile_ctr + kCtrSortBase, sc.status,
+               pl.sort_map, low, uint32_t(C::RADIX - 1), sc.sort_desc, sc.tile_ctr + kCtrSortBase,
+               sc.status,
                probe_spins, static_cast<const uint32_t*>(nullptr),
                static_cast<const uint32_t*>(nullptr));
     return cudaGetLastError();
@@ -593,7 +609,7 @@ cudaError_t passes_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStrea
     K* dst = ((P - 1 - p) % 2 == 0) == (low == 0) ? alt : tmp;
     if (tiles)
       launch_pdl(p == P - 1 ? kern_top : p == 0 ? kern_first : kern, grid, THREADS,
-                 p == P - 1 ? CT::kSmem : p == 0 ? smem_first : C::kSmem, s, src, dst, pl.seg, pl.sort_map, low + p * D,
+                 p == P - 1 ? CT::kSmem : p == 0 ? smem_first : C::kSmem, s, src, dst, pl.seg, pl.sort_map, low + pass_shift<K, D, 0>(p), pass_mask<K, D>(p),
                  sc.sort_desc + size_t(p) * sc.sort_rows * C::RADIX,
                  sc.tile_ctr + kCtrSortBase + p, sc.status, sc.spin_limit, sc.gate,
                  static_cast<const uint32_t*>(p == P - 1 ? skew : nullptr));

@@ -83,6 +83,7 @@ struct RankPack {
 // Stable ranks of one warp's 32*KPT keys among the warp's keys of the same
 // digit (order: step, then lane); the warp's digit counters `wh` advance.
 // FULL: every key is in range, so no per-key checks are made.
+// dmask: the digit's bits (a pass may use fewer than D).
 // BB: the digit bits the ballot scheme compares (the bits above them are zero
 // in every key of this pass).
 // RANK kRankMixed: `ballots` (block-uniform) picks the ballot scheme, else
@@ -91,15 +92,15 @@ template <int D, int KPT, int RANK, bool FULL, int BB = D, typename K>
 __device__ __forceinline__ void warp_rank(const K (&keys)[KPT],
                                           uint32_t (&rank2)[RankPack<KPT>::kRegs],
                                           int shift, uint32_t wbase, uint32_t n, uint32_t* wh,
-                                          uint32_t* wm, int steps = KPT, bool ballots = false) {
+                                          uint32_t* wm, int steps = KPT, bool ballots = false,
+                                          uint32_t dmask = (1u << D) - 1) {
   const bool by_ballot = RANK == kRankBallot || (RANK == kRankMixed && ballots);
-  constexpr uint32_t RADIX = 1u << D;
   const uint32_t lane = lane_id();
 #pragma unroll
   for (int i = 0; i < KPT; ++i) {
     if (!FULL && i >= steps) break;  // warp-uniform: the warp's keys end here
     const bool valid = FULL || wbase + 32u * i < n;
-    const uint32_t dig = uint32_t(keys[i] >> shift) & (RADIX - 1);
+    const uint32_t dig = uint32_t(keys[i] >> shift) & dmask;
     uint32_t peers;
     static_assert(BB >= 1 && BB <= D, "ballot bits within the digit");
     if (by_ballot) {
@@ -132,13 +133,13 @@ template <int D, int KPT, bool FULL, typename K>
 __device__ __forceinline__ void warp_place(const K (&keys)[KPT],
                                            const uint32_t (&rank2)[RankPack<KPT>::kRegs], int shift,
                                            uint32_t wbase, uint32_t n, const uint32_t* wh,
-                                           K* s_keys, int steps = KPT) {
-  constexpr uint32_t RADIX = 1u << D;
+                                           K* s_keys, int steps = KPT,
+                                           uint32_t dmask = (1u << D) - 1) {
 #pragma unroll
   for (int i = 0; i < KPT; ++i) {
     if (!FULL && i >= steps) break;
     if (FULL || wbase + 32u * i < n) {
-      const uint32_t dig = uint32_t(keys[i] >> shift) & (RADIX - 1);
+      const uint32_t dig = uint32_t(keys[i] >> shift) & dmask;
       s_keys[wh[dig] + RankPack<KPT>::get(rank2, i)] = keys[i];
     }
   }
@@ -162,14 +163,14 @@ __device__ __forceinline__ uint32_t half_slot(uint32_t dig) {
 template <int D, int KPT, bool FULL, typename K>
 __device__ __forceinline__ void half_rank(const K (&keys)[KPT],
                                           uint32_t (&rank2)[RankPack<KPT>::kRegs], int shift,
-                                          uint32_t hbase, uint32_t n, uint32_t* wp) {
-  constexpr uint32_t RADIX = 1u << D;
+                                          uint32_t hbase, uint32_t n, uint32_t* wp,
+                                          uint32_t dmask) {
   const uint32_t l16 = lane_id() & 15u;
   const uint32_t lt16 = (1u << l16) - 1u;
 #pragma unroll
   for (int i = 0; i < KPT; ++i) {
     const bool valid = FULL || hbase + 16u * i < n;
-    const uint32_t dig = uint32_t(keys[i] >> shift) & (RADIX - 1);
+    const uint32_t dig = uint32_t(keys[i] >> shift) & dmask;
     uint32_t* w = wp + half_slot(dig);
     if (valid) atomicOr(w, 1u << l16);
     __syncwarp();
@@ -193,12 +194,11 @@ template <int D, int KPT, bool FULL, typename K>
 __device__ __forceinline__ void half_place(const K (&keys)[KPT],
                                            const uint32_t (&rank2)[RankPack<KPT>::kRegs],
                                            int shift, uint32_t hbase, uint32_t n,
-                                           const uint32_t* wp, K* s_keys) {
-  constexpr uint32_t RADIX = 1u << D;
+                                           const uint32_t* wp, K* s_keys, uint32_t dmask) {
 #pragma unroll
   for (int i = 0; i < KPT; ++i) {
     if (FULL || hbase + 16u * i < n) {
-      const uint32_t dig = uint32_t(keys[i] >> shift) & (RADIX - 1);
+      const uint32_t dig = uint32_t(keys[i] >> shift) & dmask;
       s_keys[wp[half_slot(dig)] + RankPack<KPT>::get(rank2, i)] = keys[i];
     }
   }
