@@ -29,15 +29,6 @@ struct KeyTraits<uint32_t> {
     v = (v | (v << 2)) & 0x09249249u;
     return v;
   }
-  // Inverse of spread: gather bits 0, 3, 6, ... into the low 10 bits.
-  __device__ __forceinline__ static uint32_t gather(uint32_t v) {
-    v &= 0x09249249u;
-    v = (v ^ (v >> 2)) & 0x030c30c3u;
-    v = (v ^ (v >> 4)) & 0x0300f00fu;
-    v = (v ^ (v >> 8)) & 0x030000ffu;
-    v = (v ^ (v >> 16)) & 0x3ffu;
-    return v;
-  }
   __device__ __forceinline__ static int clz(uint32_t v) { return __clz(v); }
 };
 
@@ -55,15 +46,6 @@ struct KeyTraits<uint64_t> {
     v = (v | (v << 8)) & 0x100f00f00f00f00full;
     v = (v | (v << 4)) & 0x10c30c30c30c30c3ull;
     v = (v | (v << 2)) & 0x1249249249249249ull;
-    return v;
-  }
-  __device__ __forceinline__ static uint64_t gather(uint64_t v) {
-    v &= 0x1249249249249249ull;
-    v = (v ^ (v >> 2)) & 0x10c30c30c30c30c3ull;
-    v = (v ^ (v >> 4)) & 0x100f00f00f00f00full;
-    v = (v ^ (v >> 8)) & 0x001f0000ff0000ffull;
-    v = (v ^ (v >> 16)) & 0x001f00000000ffffull;
-    v = (v ^ (v >> 32)) & 0x1fffffull;
     return v;
   }
   __device__ __forceinline__ static int clz(uint64_t v) { return __clzll(v); }
@@ -109,22 +91,47 @@ inline float pow2_reciprocal(float range) {
   return out;
 }
 
+// Bits A, A + 3, ..., A + 27 of v, gathered in order into bits 18 + A .. 27 + A
+// (the other bits are not cleared).  Each step doubles the groups' size: a
+// multiplication by 1 + 2^s sets a copy s bits higher, which no other group
+// overlaps, and the mask keeps the half that has moved of each pair.
+template <int A>
+__device__ __forceinline__ uint32_t gather_high(uint32_t v) {
+  v &= 0x09249249u << A;
+  v = (v * 5u) & (0x0c30c30cu << A);
+  v = (v * 17u) & (0x0f00f00cu << A);
+  v = (v * 257u) & (0x0ff0000cu << A);
+  return v * 65537u;
+}
+
+// Axis A of a code as a fraction of the axis in [0, 1), exactly: the axis's
+// bits become the mantissa of 1.x, less 1.
+template <int A>
+__device__ __forceinline__ float axis_fraction(uint32_t code) {
+  const uint32_t m = (gather_high<A>(code) >> (5 + A)) & 0x007fe000u;
+  return __fadd_rn(__uint_as_float(0x3f800000u | m), -1.0f);
+}
+template <int A>
+__device__ __forceinline__ float axis_fraction(uint64_t code) {
+  // the axis's bits 0-9, 10-19 and 20 from 30, 30 and 3 bits of the code
+  const uint32_t lo = gather_high<A>(uint32_t(code) & 0x3fffffffu);
+  const uint32_t mid = gather_high<A>(uint32_t(code >> 30) & 0x3fffffffu);
+  const uint32_t top = uint32_t(code >> (60 + A)) & 1u;
+  const uint32_t m = ((lo >> (16 + A)) & 0xffcu) | ((mid >> (6 + A)) & 0x3ff000u) | top << 22;
+  return __fadd_rn(__uint_as_float(0x3f800000u | m), -1.0f);
+}
+
 // morton32_to_xyz (func_morton.hpp:60-80): float(d) / scale * range + min,
-// w = 1.
+// w = 1.  Dividing by the scale, a power of two, is exact, and so is the
+// fraction made from the bits.  Octree rows are bound by their integer
+// instructions: multiplications and additions of floats in place of half of
+// the shifts, and no conversions.
 template <typename K>
 __device__ __forceinline__ float4 decode(K code, float min_coord, float range) {
-  using T = KeyTraits<K>;
-  constexpr float kScale = float(1u << T::kAxisBits);
-  const float fx = __uint2float_rn(uint32_t(T::gather(code)));
-  const float fy = __uint2float_rn(uint32_t(T::gather(code >> 1)));
-  const float fz = __uint2float_rn(uint32_t(T::gather(code >> 2)));
   float4 r;
-  // kScale is a power of two: dividing by it is multiplying by its exact
-  // reciprocal (the same correctly rounded value)
-  constexpr float kInv = 1.0f / kScale;
-  r.x = __fadd_rn(__fmul_rn(__fmul_rn(fx, kInv), range), min_coord);
-  r.y = __fadd_rn(__fmul_rn(__fmul_rn(fy, kInv), range), min_coord);
-  r.z = __fadd_rn(__fmul_rn(__fmul_rn(fz, kInv), range), min_coord);
+  r.x = __fadd_rn(__fmul_rn(axis_fraction<0>(code), range), min_coord);
+  r.y = __fadd_rn(__fmul_rn(axis_fraction<1>(code), range), min_coord);
+  r.z = __fadd_rn(__fmul_rn(axis_fraction<2>(code), range), min_coord);
   r.w = 1.0f;
   return r;
 }

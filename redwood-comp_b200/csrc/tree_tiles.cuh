@@ -692,7 +692,9 @@ constexpr uint32_t kFarFromParent = 0, kFarFromStep = 1, kFarFinal = 2, kFarLoca
 // bound by its instructions: with four nodes 256 apart per thread, a scan per
 // group of them and a binary search over the tile's first rows for each row's
 // owner it executed 156M of them instead of 146M and took 183.9 instead of 170.0
-// us at 16.8M uniform points (5,000,011 64-bit keys: 75.7, now 71.8).
+// us at 16.8M uniform points (5,000,011 64-bit keys: 75.7, then 71.8).  Corners
+// decoded by multiplications (decode) and one expansion of the child slots for
+// first and later rows of a chain alike: 164.0 us (64-bit keys 69.7).
 //
 // Node 0 owns no row; tile 0 writes the root initialisation when there is
 // no octree row at all (07_octree.cu:188-198) and clears the spare row m
@@ -700,7 +702,7 @@ constexpr uint32_t kFarFromParent = 0, kFarFromStep = 1, kFarFinal = 2, kFarLoca
 //
 // With OFFS the offsets are not read but made here (stage 6's write folded
 // into stage 7): tile_prefix holds the exclusive scan of every tile's count
-// sum (k_node_sums, k_tile_scan), the block scans its tile's counts on top
+// sum (tree_tile, k_tile_scan), the block scans its tile's counts on top
 // of it and writes them to off_all.
 template <typename K>
 struct OctTileShared {
@@ -959,28 +961,28 @@ __device__ __forceinline__ void octree_tile(
     o.cell_size[rp] =
         __fmul_rn(range, __uint_as_float(uint32_t(127 - (level - root_level)) << 23));
     int4* row = reinterpret_cast<int4*>(o.children + 8 * rp);
+    // the children as slots of 16 bits, relative to the tile's first row, plus one
+    uint4 a;
     if (k == 0) {
-      const uint4 a = sh.child[t];
-      const uint32_t wv[4] = {a.x, a.y, a.z, a.w};
-      int32_t child[8];
-      uint32_t mask = 0;
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const uint32_t v = (wv[q >> 1] >> (16 * (q & 1))) & 0xffffu;
-        child[q] = v ? int32_t(v) - 1 + rbase : 0;
-        mask |= uint32_t(v != 0) << q;
-      }
-      row[0] = make_int4(child[0], child[1], child[2], child[3]);
-      row[1] = make_int4(child[4], child[5], child[6], child[7]);
-      o.node_mask[rp] = int32_t(mask);
-    } else {
-      int32_t child[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      const int slot = int((code >> (B - 3 * (level + 1))) & K(7));
-      child[slot] = p - 1;
-      row[0] = make_int4(child[0], child[1], child[2], child[3]);
-      row[1] = make_int4(child[4], child[5], child[6], child[7]);
-      o.node_mask[rp] = 1 << slot;
+      a = sh.child[t];
+    } else {  // the chain's row before this one
+      const uint32_t slot = uint32_t(code >> (B - 3 * (level + 1))) & 7u;
+      const uint32_t w = uint32_t(r) << (16 * (slot & 1u));
+      a = make_uint4(slot >> 1 == 0 ? w : 0u, slot >> 1 == 1 ? w : 0u, slot >> 1 == 2 ? w : 0u,
+                     slot >> 1 == 3 ? w : 0u);
     }
+    const uint32_t wv[4] = {a.x, a.y, a.z, a.w};
+    int32_t child[8];
+    uint32_t mask = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const uint32_t v = (wv[q >> 1] >> (16 * (q & 1))) & 0xffffu;
+      child[q] = v ? int32_t(v) - 1 + rbase : 0;
+      mask |= uint32_t(v != 0) << q;
+    }
+    row[0] = make_int4(child[0], child[1], child[2], child[3]);
+    row[1] = make_int4(child[4], child[5], child[6], child[7]);
+    o.node_mask[rp] = int32_t(mask);
     o.leaf_mask[rp] = 0;
   }
 }
