@@ -8,6 +8,12 @@
 
 namespace rwt {
 
+// Highest set bit of x, -1 for 0.
+__device__ __forceinline__ int highest_bit(uint32_t x) {
+  int r;
+  asm("bfind.u32 %0, %1;" : "=r"(r) : "r"(x));
+  return r;
+}
 // x / 3 for 0 <= x < 256.
 __device__ __forceinline__ int third(int x) { return (x * 171) >> 9; }
 
@@ -307,7 +313,10 @@ __device__ __forceinline__ void tree_tile(unsigned char* smem_raw, TreeTileShare
 
   // the window's keys [wlo, wlo + kAnsvWin]: one bulk copy when the window
   // lies inside the keys and starts on a 16-byte boundary (every interior
-  // tile of a plain run), else key by key with zeros outside [0, n]
+  // tile of a plain run), else key by key; outside [0, n] the key word's top
+  // bit, clear in every key, changes from each key to the next, so that the
+  // gaps there come out as E = 0 without a check (16.8M 32-bit keys 179.6 ->
+  // 173.8 us together with highest_bit)
   static_assert((size_t(C::kWin) * sizeof(K)) % 16 == 0, "bulk copies move 16-byte units");
   const bool bulk = BULK && wlo >= 0 && wlo + win <= n &&
                     (reinterpret_cast<uintptr_t>(codes + wlo) & 15u) == 0;
@@ -328,7 +337,7 @@ __device__ __forceinline__ void tree_tile(unsigned char* smem_raw, TreeTileShare
   } else {
     for (int j = threadIdx.x; j <= win; j += NT) {
       const int k = wlo + j;
-      s_key[j] = (k >= 0 && k <= n) ? codes[k] : K(0);
+      s_key[j] = (k >= 0 && k <= n) ? codes[k] : K((k > n ? k - n : -k) & 1) << (8 * sizeof(K) - 1);
     }
   }
   __syncthreads();
@@ -346,8 +355,7 @@ __device__ __forceinline__ void tree_tile(unsigned char* smem_raw, TreeTileShare
   for (int hc = int(warp); hc < 2 * kAnsvHalo; hc += NW) {
     const int ch = hc < kAnsvHalo ? hc : hc + tch;
     const int w = ch * 32 + int(lane);
-    const int g = wlo + w;
-    const int e = uint32_t(g) < uint32_t(n) ? KeyTraits<K>::clz(s_key[w] ^ s_key[w + 1]) : 0;
+    const int e = KeyTraits<K>::clz(s_key[w] ^ s_key[w + 1]);
     s_e[w] = uint8_t(e);
     const uint32_t cmin = __reduce_min_sync(0xffffffffu, uint32_t(e));
     if (lane == 0) s_cmin[ch] = uint8_t(cmin);
@@ -368,11 +376,9 @@ __device__ __forceinline__ void tree_tile(unsigned char* smem_raw, TreeTileShare
     for (int j = 0; j < JN; ++j) {
       const int ch = ch0 + j * NW;
       const int w = ch * 32 + int(lane);  // window index of this lane's gap
-      const int g = wlo + w;
-      const bool real = uint32_t(g) < uint32_t(n);
       // distinct keys whose top bit is clear: E = delta + 1 = clz of the xor,
       // at least 1 for a real gap, so 0 marks walls only
-      e[j] = real ? KeyTraits<K>::clz(s_key[w] ^ s_key[w + 1]) : 0;
+      e[j] = KeyTraits<K>::clz(s_key[w] ^ s_key[w + 1]);
       s_e[w] = uint8_t(e[j]);
       const uint32_t cmin = __reduce_min_sync(0xffffffffu, uint32_t(e[j]));
       if (lane == 0) s_cmin[ch] = uint8_t(cmin);
@@ -418,15 +424,16 @@ __device__ __forceinline__ void tree_tile(unsigned char* smem_raw, TreeTileShare
         const int tg = (ch - kAnsvHalo) * 32 + int(lane);
         // lt never holds the lane itself; clz(0) = 32 and ffs(0) = 0 give -1
         const uint32_t lm = lt & lanemask_lt(), rm = lt & ~lm;
-        const int lp = 31 - __clz(lm);
+        // (the one instruction is the faster form with the 64-bit kernel's
+        // registers only: 75.1 against 76.0 us, 32-bit 176.2 against 173.8)
+        const int lp = NV > 32 ? highest_bit(lm) : 31 - __clz(lm);
         const int rp = __ffs(rm) - 1;
         // E of the two nearest smaller lanes (a wall lane past the last gap
         // has E = 0, so D = -1 there as for the wall at n)
         const int el = __shfl_sync(0xffffffffu, e[j], lp);
         const int er = __shfl_sync(0xffffffffu, e[j], rp);
         const int g = g0 + tg;
-        const bool real = g < n;
-        const bool here = real && lm && rm;
+        const bool here = lm && rm;  // (no lane lies below a wall)
         int count = 0;
         if (here)
           write_gap_node_d<EDGES, LESS>(g, e[j] - 1, g - int(lane) + lp, g - int(lane) + rp,
@@ -444,21 +451,21 @@ __device__ __forceinline__ void tree_tile(unsigned char* smem_raw, TreeTileShare
             acc = 0;
           }
         }
-        const uint32_t pm = __ballot_sync(0xffffffffu, real && !here);
+        const uint32_t pm = __ballot_sync(0xffffffffu, e[j] != 0 && !here);
         if (pm) {
           uint32_t at = 0;
           if (lane == uint32_t(__ffs(pm) - 1)) at = atomicAdd(&sh.pend_n, uint32_t(__popc(pm)));
           at = __shfl_sync(0xffffffffu, at, __ffs(pm) - 1) + __popc(pm & lanemask_lt());
-          if (real && !here)
+          if (e[j] != 0 && !here)
             s_pend[at] = uint32_t(tg) | uint32_t(lp & 0xff) << 16 | uint32_t(rp & 0xff) << 24;
         }
       }
       // an empty mask gives 0xff (none) by itself: 31 - clz(0) = ffs(0) - 1 = -1
       const int tc = ch - kAnsvHalo;  // the chunk's column among the tile's
-      s_last[int(lane) * C::kRow + tc] = uint8_t(31 - __clz(lt0[j]));
+      s_last[int(lane) * C::kRow + tc] = uint8_t(highest_bit(lt0[j]));
       s_first[int(lane) * C::kRow + tc] = uint8_t(__ffs(lt0[j]) - 1);
       if (NV > 32) {
-        s_last[(int(lane) + 32) * C::kRow + tc] = uint8_t(31 - __clz(lt1[j]));
+        s_last[(int(lane) + 32) * C::kRow + tc] = uint8_t(highest_bit(lt1[j]));
         s_first[(int(lane) + 32) * C::kRow + tc] = uint8_t(__ffs(lt1[j]) - 1);
       }
     }
