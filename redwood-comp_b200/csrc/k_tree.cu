@@ -522,7 +522,8 @@ __global__ void __launch_bounds__(256)
 // ---------------------------------------------------------------------------
 
 // Kernels in the chain of programmatic launches instead of 16-byte copies, which
-// would end it and wait for a copy engine; host memory is pinned.
+// would end it and wait for a copy engine (2,000,003 points, the stages called one by
+// one: 349 -> 289 us; a batch of 256 clouds 707 -> 689); host memory is pinned.
 __global__ void k_status_in(DevStatus* __restrict__ st, uint32_t n_unique, uint32_t n_octree,
                             uint32_t* __restrict__ far_n) {
   pdl_enter();
