@@ -55,25 +55,47 @@ __global__ void __launch_bounds__(1024)
     k_tile_scan(uint32_t* __restrict__ E, uint32_t tiles, SegTable seg, TileMap map,
                 uint32_t* __restrict__ seg_total) {
   pdl_enter();
-  // rounds of 1,024 x J tiles; warp w scans its contiguous 32 x J slice with
-  // coalesced loads (J warp scans with a running carry), then one warp scans
-  // the 32 warp sums
-  constexpr int J = 16;
+  // Rounds of up to 1,024 x 4 J tiles, a contiguous slice of 128 q per warp: a
+  // lane takes four consecutive tiles at a time as a vector and adds them up, so
+  // that a warp scan serves 128 tiles, then one warp scans the 32 warp sums.
+  // One block: its shuffles are what counts (J scans of single words for every
+  // warp, whether it had tiles or not: unique and edge scan of
+  // 16.8M points 60.8 -> 56.7 us, of 5M 64-bit keys 31.6 -> 26.4)
+  constexpr int J = 4;
   __shared__ uint32_t s_warp[33];
   const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+  const bool vec = (reinterpret_cast<uintptr_t>(E) & 15u) == 0;
   uint32_t carry = 0;
-  for (uint32_t c0 = 0; c0 < tiles; c0 += 1024u * J) {
-    const uint32_t wb = c0 + warp * 32u * J + lane;
-    uint32_t v[J];
+  for (uint32_t c0 = 0; c0 < tiles; c0 += 4096u * J) {
+    const uint32_t q = min(uint32_t(J), (tiles - c0 + 4095u) / 4096u);
+    const uint32_t wb = c0 + warp * 128u * q + 4u * lane;
+    uint4 v[J];
 #pragma unroll
-    for (int j = 0; j < J; ++j) v[j] = wb + 32u * j < tiles ? E[wb + 32u * j] : 0u;
+    for (int j = 0; j < J; ++j) {
+      const uint32_t i = wb + 128u * j;
+      v[j] = make_uint4(0, 0, 0, 0);
+      if (uint32_t(j) < q) {
+        if (vec && i + 4u <= tiles) {
+          v[j] = *reinterpret_cast<const uint4*>(E + i);
+        } else {
+          if (i < tiles) v[j].x = E[i];
+          if (i + 1u < tiles) v[j].y = E[i + 1u];
+          if (i + 2u < tiles) v[j].z = E[i + 2u];
+          if (i + 3u < tiles) v[j].w = E[i + 3u];
+        }
+      }
+    }
     uint32_t run = 0;
 #pragma unroll
     for (int j = 0; j < J; ++j) {
-      const uint32_t inc = warp_inclusive_scan(v[j]);
-      const uint32_t x = v[j];
-      v[j] = run + inc - x;  // exclusive within the warp's slice
-      run += __shfl_sync(0xffffffffu, inc, 31);
+      if (uint32_t(j) < q) {
+        const uint4 x = v[j];
+        const uint32_t sum = x.x + x.y + x.z + x.w;
+        const uint32_t inc = warp_inclusive_scan(sum);
+        const uint32_t at = run + inc - sum;  // exclusive within the warp's slice
+        v[j] = make_uint4(at, at + x.x, at + x.x + x.y, at + x.x + x.y + x.z);
+        run += __shfl_sync(0xffffffffu, inc, 31);
+      }
     }
     if (lane == 0) s_warp[warp] = run;
     __syncthreads();
@@ -86,8 +108,20 @@ __global__ void __launch_bounds__(1024)
     __syncthreads();
     const uint32_t wofs = carry + s_warp[warp];
 #pragma unroll
-    for (int j = 0; j < J; ++j)
-      if (wb + 32u * j < tiles) E[wb + 32u * j] = wofs + v[j];
+    for (int j = 0; j < J; ++j) {
+      const uint32_t i = wb + 128u * j;
+      if (uint32_t(j) < q) {
+        const uint4 x = make_uint4(wofs + v[j].x, wofs + v[j].y, wofs + v[j].z, wofs + v[j].w);
+        if (vec && i + 4u <= tiles) {
+          *reinterpret_cast<uint4*>(E + i) = x;
+        } else {
+          if (i < tiles) E[i] = x.x;
+          if (i + 1u < tiles) E[i + 1u] = x.y;
+          if (i + 2u < tiles) E[i + 2u] = x.z;
+          if (i + 3u < tiles) E[i + 3u] = x.w;
+        }
+      }
+    }
     carry += s_warp[32];
     __syncthreads();  // s_warp is reused by the next round
   }
