@@ -325,7 +325,8 @@ int rw_tree_batch_finish(rw_tree_batch* batch, rw_stream_t stream, uint32_t* n_u
 
 /* Stage 2 alone, asynchronous on `stream` (no synchronisation, capturable):
  * sorts app->u_morton_keys[0, n) into app->u_morton_keys_alt with the onesweep
- * sort.  Only the two key buffers of `app` are used. */
+ * sort, by every bit of the words (with 8- and 11-bit digits; 10-bit digits sort
+ * 32-bit keys by their low 30 bits).  Only the two key buffers of `app` are used. */
 int rw_tree_sort_enqueue(rw_tree_app_data* app, rw_tree_im_storage* im, rw_stream_t stream);
 /* The same sort `reps` times with CUDA events between its kernels; mean
  * device milliseconds of the digit histogram, the pass set-up and each pass

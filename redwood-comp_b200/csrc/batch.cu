@@ -157,6 +157,7 @@ rwt::Scratch scratch_of(const rw_tree_batch* b) {
   sc.ghist = b->d_ghist;
   sc.skew = b->d_skew;
   sc.low_bits = b->low_bits;
+  sc.codes = true;
   sc.long_run = b->d_long_run;
   sc.sort_desc = b->d_sort_desc;
   sc.sort_rows = b->sort_rows;

@@ -520,7 +520,8 @@ int enqueue_impl(rw_tree_app_data* app, rw_tree_im_storage* im, cudaStream_t s,
   };
   if (int rc = clear_all(im, s)) return rc;
   const auto b = bufs_of(*app, im);
-  const auto sc = scratch_of(im);
+  auto sc = scratch_of(im);
+  sc.codes = true;
   const auto pl = plan_of(*app, im);
   RW_CUDA(mark());
   if (im->learned) {

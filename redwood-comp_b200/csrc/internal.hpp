@@ -77,7 +77,8 @@ constexpr uint32_t kOctTile = kOctThreads * kOctNpt;
 // 64-bit keys with 8-bit digits: the passes leave out the low bits, which
 // k_sort_fix puts in order (k_sortfix.cu).  Four passes over the top 32 bits of
 // the 63, five over the top 40 for scratch of more points, where runs of equal
-// top bits get long.
+// top bits get long.  A caller's keys may have the top bit of the word set as
+// well: one bit more is then left out (sorted_low_bits).
 constexpr int kSplitLow32 = 31, kSplitLow40 = 23;
 constexpr uint32_t kSplitPoints = 1u << 21;
 inline int sort_low_bits(int key_bits, int radix_bits, uint32_t largest) {
@@ -140,6 +141,9 @@ struct Scratch {
   // [segments]: 1 when a run of keys with equal top bits was too long for it
   int low_bits = 0;
   uint32_t* long_run = nullptr;
+  // the keys are codes that stage 1 makes in the same chain, whose top bits are
+  // clear; else a caller's, which are sorted by the whole word
+  bool codes = false;
   uint32_t* sort_desc = nullptr;  // [passes][sort_rows][radix]
   uint32_t sort_rows = 0;         // rows per pass: sort tiles + segments
   uint32_t* unique_desc = nullptr;
@@ -156,6 +160,10 @@ struct Scratch {
   uint32_t* tree_far = nullptr;
   uint32_t tree_far_cap = 0;
 };
+
+inline int sorted_low_bits(const Scratch& sc) {
+  return sc.low_bits && !sc.codes ? sc.low_bits + 1 : sc.low_bits;
+}
 
 // Entries of the radix tree's far-search list per tile: the gaps of a tile
 // with no smaller gap inside its window have strictly decreasing (left side)

@@ -29,18 +29,20 @@ namespace rwt {
 // stage 1
 // ---------------------------------------------------------------------------
 
-// Digit of pass p of the sort: its lowest bit and its mask.  30-bit codes with
-// 8-bit digits take 8, 8, 7 and 7 bits instead of 8, 8, 8 and 6: the top six bits
-// (a quarter of the box per axis) of a clustered cloud put many lanes of a warp on
-// one counter, the top seven half as many (16.8M mixture points, last two passes
-// 163.8 -> 155.5 us; uniform ones 133.9 -> 134.7).
-template <typename K, int D, int LOW>
+// Digit of pass p of the sort: its lowest bit and its mask.  CODES: the keys are
+// codes that stage 1 has just made, else a caller's, of which every bit of the
+// word may be set.  30-bit codes with 8-bit digits take 8, 8, 7 and 7 bits instead
+// of a word's 8, 8, 8 and 8: the top six bits (a quarter of the box per axis) of a
+// clustered cloud put many lanes of a warp on one counter, the top seven half as
+// many (16.8M mixture points, last two passes 163.8 -> 155.5 us; uniform ones
+// 133.9 -> 134.7).
+template <typename K, int D, bool CODES>
 __host__ __device__ constexpr int pass_shift(int p) {
-  return LOW + (sizeof(K) == 4 && D == 8 && p == 3 ? 23 : p * D);
+  return CODES && sizeof(K) == 4 && D == 8 && p == 3 ? 23 : p * D;
 }
-template <typename K, int D>
+template <typename K, int D, bool CODES>
 __host__ __device__ constexpr uint32_t pass_mask(int p) {
-  return sizeof(K) == 4 && D == 8 && p == 2 ? 0x7fu : (1u << D) - 1u;
+  return CODES && sizeof(K) == 4 && D == 8 && p == 2 ? 0x7fu : (1u << D) - 1u;
 }
 
 // Points are walked in tiles of kPointTile that never straddle two segments;
@@ -90,7 +92,8 @@ __global__ void __launch_bounds__(256)
       if (HIST) {
 #pragma unroll
         for (int ps = 0; ps < P; ++ps)
-          atomicAdd(&s_hist[ps * RADIX + int((k >> pass_shift<K, D, LOW>(ps)) & K(pass_mask<K, D>(ps)))], 1u);
+          atomicAdd(&s_hist[ps * RADIX + int((k >> (LOW + pass_shift<K, D, ENCODE>(ps))) &
+                                             K(pass_mask<K, D, ENCODE>(ps)))], 1u);
       }
     };
     if (hi - lo == kPointTile) {
@@ -507,14 +510,17 @@ cudaError_t keys_t(const Bufs& b, const Scratch& sc, const Plan& pl, bool encode
   const uint32_t ctas = std::max(1u, std::min<uint32_t>(tiles, uint32_t(sc.num_sms) * 8));
   const uint32_t per = div_up(tiles, ctas);
   const uint32_t grid = div_up(tiles, per);
-  if (hist && sc.passes != (KeyTraits<K>::kCodeBits - LOW + D - 1) / D) return cudaErrorInvalidValue;
+  if (hist && (sc.passes != (KeyTraits<K>::kCodeBits - LOW + D - 1) / D || sc.codes != encode))
+    return cudaErrorInvalidValue;
+  constexpr int kWordLow = LOW ? LOW + 1 : 0;  // the top bit belongs to a digit of a word
   const size_t smem = hist ? size_t(sc.passes) * (1u << D) * 4 : 0;
   K* keys = static_cast<K*>(b.keys);
   const float inv = pow2_reciprocal(b.range);
 #define RWT_KEYS_LAUNCH(H, E)                                                        \
   do {                                                                               \
-    auto kern = inv != 0.0f ? k_keys_pass<K, D, LOW, H, E, true>             \
-                            : k_keys_pass<K, D, LOW, H, E, false>; \
+    constexpr int kLow = E ? LOW : kWordLow;                                         \
+    auto kern = inv != 0.0f ? k_keys_pass<K, D, kLow, H, E, true>                    \
+                            : k_keys_pass<K, D, kLow, H, E, false>;                  \
     if (smem > 48 * 1024)                                                            \
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)); \
     launch_pdl(kern, grid, 256, smem, s, b.points, keys, pl.seg, pl.point_map, per, b.min_coord, \
@@ -537,15 +543,22 @@ template <typename K, int D, int THREADS, int KPT, int RANK, int MINB>
 cudaError_t passes_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_t s,
                      cudaEvent_t* marks, uint32_t probe_spins) {
   // with low bits left out the passes end in tmp (launch_sort_finish goes on to alt)
-  const int low = sc.low_bits, P = sc.passes;
+  const int low = sorted_low_bits(sc), P = sc.passes;
   constexpr int kFull = (KeyTraits<K>::kCodeBits + D - 1) / D;
   constexpr int RB = RANK == kRankMixed ? kRankAtomicOr : RANK;  // passes 0 .. P-2
   constexpr int RT = RANK;                                       // pass P-1
-  // bits of the top digit (left out bits are chosen so that it is a full one)
+  // bits of a code's top digit (left out bits are chosen so that it is a full one;
+  // so is a word's)
   constexpr int TB = RANK == kRankMixed && !(sizeof(K) == 8 && D == 8)
-                         ? KeyTraits<K>::kCodeBits - pass_shift<K, D, 0>(kFull - 1)
+                         ? KeyTraits<K>::kCodeBits - pass_shift<K, D, true>(kFull - 1)
                          : D;
   static_assert((63 - kSplitLow32) % 8 == 0 && (63 - kSplitLow40) % 8 == 0, "full digits");
+  const auto shift = [&](int p) {
+    return low + (sc.codes ? pass_shift<K, D, true>(p) : pass_shift<K, D, false>(p));
+  };
+  const auto mask = [&](int p) {
+    return sc.codes ? pass_mask<K, D, true>(p) : pass_mask<K, D, false>(p);
+  };
   constexpr int kSkewLog2 = sizeof(K) == 4 ? 5 : 6;
   uint32_t* skew = RANK == kRankMixed ? sc.skew : nullptr;
   using C = BinCfg<K, D, THREADS, KPT, RB>;
@@ -556,6 +569,9 @@ cudaError_t passes_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStrea
                       : k_binning<K, D, THREADS, KPT, RB, MINB, false>;
   auto kern_top = persist ? k_binning<K, D, THREADS, KPT, RT, MINB, true, TB>
                           : k_binning<K, D, THREADS, KPT, RT, MINB, false, TB>;
+  if (!sc.codes)
+    kern_top = persist ? k_binning<K, D, THREADS, KPT, RT, MINB, true, D>
+                       : k_binning<K, D, THREADS, KPT, RT, MINB, false, D>;
   // the first pass need not be stable (a gated sort, which rarely runs, keeps to
   // the other kernel, and so do the wider digits)
   using CF = BinCfg<K, D, THREADS, KPT, D == 8 ? kRankUnordered : RB>;
@@ -609,7 +625,8 @@ cudaError_t passes_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStrea
     K* dst = ((P - 1 - p) % 2 == 0) == (low == 0) ? alt : tmp;
     if (tiles)
       launch_pdl(p == P - 1 ? kern_top : p == 0 ? kern_first : kern, grid, THREADS,
-                 p == P - 1 ? CT::kSmem : p == 0 ? smem_first : C::kSmem, s, src, dst, pl.seg, pl.sort_map, low + pass_shift<K, D, 0>(p), pass_mask<K, D>(p),
+                 p == P - 1 ? CT::kSmem : p == 0 ? smem_first : C::kSmem, s, src, dst, pl.seg,
+                 pl.sort_map, shift(p), mask(p),
                  sc.sort_desc + size_t(p) * sc.sort_rows * C::RADIX,
                  sc.tile_ctr + kCtrSortBase + p, sc.status, sc.spin_limit, sc.gate,
                  static_cast<const uint32_t*>(p == P - 1 ? skew : nullptr));

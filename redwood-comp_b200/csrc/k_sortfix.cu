@@ -34,9 +34,10 @@ constexpr int kFixWin = kFixTile + 2 * kFixRun;
 // at 5,000,011 points (80 MB: 3.2 TB/s), where plain loads took 27.8, looking at
 // both neighbours key by key 33.6 and gathering the sorted tile in a second
 // buffer 26.1.  The last of two waves of tiles is what is left.
-template <typename K, int LOW>
+template <typename K>
 __global__ void __launch_bounds__(kFixThreads, 6)
-    k_sort_fix(const K* __restrict__ in, K* __restrict__ out, SegTable seg, TileMap map,
+    k_sort_fix(const K* __restrict__ in, K* __restrict__ out, uint32_t top, SegTable seg,
+               TileMap map,
                uint32_t* __restrict__ heads, uint32_t* __restrict__ long_run,
                DevStatus* __restrict__ st) {
   pdl_enter();
@@ -77,10 +78,10 @@ __global__ void __launch_bounds__(kFixThreads, 6)
     for (int i = int(threadIdx.x); i < m; i += kFixThreads) s[i] = in[lo + uint32_t(i)];
   }
   __syncthreads();
-  // equal top bits: the upper words and the bits from LOW on
-  static_assert(LOW < 32 && sizeof(K) == 8, "the bits left out lie in the lower word");
-  auto same = [](K x, K y) {
-    return uint32_t(x >> 32) == uint32_t(y >> 32) && (uint32_t(x) ^ uint32_t(y)) < (1u << LOW);
+  // equal top bits: the upper words and the bits of `top` in the lower one
+  static_assert(sizeof(K) == 8, "the bits left out lie in the lower word");
+  auto same = [top](K x, K y) {
+    return uint32_t(x >> 32) == uint32_t(y >> 32) && ((uint32_t(x) ^ uint32_t(y)) & top) == 0;
   };
   bool far = false;
   uint32_t count = 0;
@@ -195,7 +196,7 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_sort_long(LongArgs a) {
     const uint32_t s0 = seg_begin(a.seg, c), n = seg_size(a.seg, c);
     const uint32_t share = (n + P - 1) / P;
     const uint32_t p0 = min(b * share, n), p1 = min(p0 + share, n);
-    constexpr int kDigits = (KeyTraits<K>::kCodeBits + 7) / 8;
+    constexpr int kDigits = int(sizeof(K));
     static_assert(kDigits % 2 == 0, "the last pass ends in alt");
     for (int q = 0; q < kDigits; ++q) {
       const K* src = static_cast<const K*>(q == 0 ? a.keys : (q & 1) ? a.tmp : a.alt) + s0;
@@ -257,10 +258,10 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_sort_long(LongArgs a) {
 
 namespace {
 
-template <typename K, int LOW>
+template <typename K>
 cudaError_t fix_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_t s) {
   // six blocks need nearly all of the SM's shared memory
-  cudaError_t e = cudaFuncSetAttribute(k_sort_fix<K, LOW>,
+  cudaError_t e = cudaFuncSetAttribute(k_sort_fix<K>,
                                        cudaFuncAttributePreferredSharedMemoryCarveout,
                                        int(cudaSharedmemCarveoutMaxShared));
   if (e == cudaSuccess)
@@ -268,8 +269,10 @@ cudaError_t fix_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_t
                              int(long_smem<K>()));
   if (e != cudaSuccess) return e;
   if (!pl.unique_map.n_tiles) return cudaSuccess;
-  launch_pdl(k_sort_fix<K, LOW>, pl.unique_map.n_tiles, kFixThreads, 0, s,
-             static_cast<const K*>(b.tmp), static_cast<K*>(b.alt), pl.seg, pl.unique_map,
+  const int low = sorted_low_bits(sc);  // at most 32
+  const uint32_t top = low < 32 ? ~0u << low : 0u;
+  launch_pdl(k_sort_fix<K>, pl.unique_map.n_tiles, kFixThreads, 0, s,
+             static_cast<const K*>(b.tmp), static_cast<K*>(b.alt), top, pl.seg, pl.unique_map,
              sc.unique_desc, sc.long_run, sc.status);
   LongArgs a{b.keys, b.tmp, b.alt, pl.seg, pl.unique_map, sc.unique_desc, sc.long_run,
              sc.sort_desc, sc.tile_ctr + kCtrLong, sc.status};
@@ -292,12 +295,8 @@ cudaError_t fix_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_t
 
 cudaError_t launch_sort_finish(const Bufs& b, const Scratch& sc, const Plan& pl,
                                cudaStream_t s) {
-  switch (sc.low_bits) {
-    case 0: return cudaSuccess;
-    case kSplitLow32: return fix_t<uint64_t, kSplitLow32>(b, sc, pl, s);
-    case kSplitLow40: return fix_t<uint64_t, kSplitLow40>(b, sc, pl, s);
-    default: return cudaErrorInvalidValue;
-  }
+  if (!sc.low_bits) return cudaSuccess;
+  return fix_t<uint64_t>(b, sc, pl, s);
 }
 
 }  // namespace rwt
