@@ -313,10 +313,10 @@ __device__ __forceinline__ void tree_tile(unsigned char* smem_raw, TreeTileShare
 
   // the window's keys [wlo, wlo + kAnsvWin]: one bulk copy when the window
   // lies inside the keys and starts on a 16-byte boundary (every interior
-  // tile of a plain run), else key by key; outside [0, n] the key word's top
-  // bit, clear in every key, changes from each key to the next, so that the
-  // gaps there come out as E = 0 without a check (16.8M 32-bit keys 179.6 ->
-  // 173.8 us together with highest_bit)
+  // tile of a plain run), else key by key; outside [0, n] the first and the last
+  // key go on with their top bit changing from each key to the next, so that
+  // the gaps there come out as E = 0 without a check, whatever the keys (16.8M
+  // 32-bit keys 179.6 -> 173.8 us together with highest_bit)
   static_assert((size_t(C::kWin) * sizeof(K)) % 16 == 0, "bulk copies move 16-byte units");
   const bool bulk = BULK && wlo >= 0 && wlo + win <= n &&
                     (reinterpret_cast<uintptr_t>(codes + wlo) & 15u) == 0;
@@ -337,7 +337,8 @@ __device__ __forceinline__ void tree_tile(unsigned char* smem_raw, TreeTileShare
   } else {
     for (int j = threadIdx.x; j <= win; j += NT) {
       const int k = wlo + j;
-      s_key[j] = (k >= 0 && k <= n) ? codes[k] : K((k > n ? k - n : -k) & 1) << (8 * sizeof(K) - 1);
+      const int out = k < 0 ? -k : k > n ? k - n : 0;  // how far outside
+      s_key[j] = codes[min(max(k, 0), n)] ^ K(out & 1) << (8 * sizeof(K) - 1);
     }
   }
   __syncthreads();
