@@ -52,7 +52,7 @@ struct rw_tree_batch {
   uint32_t tree_far_cap = 0;
   void* d_zero = nullptr;
   size_t zero_bytes = 0;
-  uint32_t *d_ghist = nullptr, *d_skew = nullptr, *d_long_run = nullptr, *d_sort_desc = nullptr,
+  uint32_t *d_ghist = nullptr, *d_skew = nullptr, *d_dense = nullptr, *d_rest_ctr = nullptr, *d_rest = nullptr, *d_sort_desc = nullptr,
            *d_unique_desc = nullptr,
            *d_scan_desc = nullptr, *d_tile_ctr = nullptr;
   rwt::DevStatus* d_status = nullptr;
@@ -158,7 +158,9 @@ rwt::Scratch scratch_of(const rw_tree_batch* b) {
   sc.skew = b->d_skew;
   sc.low_bits = b->low_bits;
   sc.codes = true;
-  sc.long_run = b->d_long_run;
+  sc.dense = b->d_dense;
+  sc.rest = b->d_rest;
+  sc.rest_ctr = b->d_rest_ctr;
   sc.sort_desc = b->d_sort_desc;
   sc.sort_rows = b->sort_rows;
   sc.unique_desc = b->d_unique_desc;
@@ -287,13 +289,16 @@ int rw_tree_batch_create(const uint32_t* cloud_sizes, uint32_t n_clouds, int32_t
   const size_t ctr_b = align(rwt::kCounters * 4);
   const size_t st_b = align(sizeof(rwt::DevStatus));
   const size_t per_b = align(size_t(n_clouds) * 4);
-  b->zero_bytes = ghist_b + sdesc_b + udesc_b + cdesc_b + ctr_b + st_b + 5 * per_b;
+  b->zero_bytes = ghist_b + sdesc_b + udesc_b + cdesc_b + ctr_b + st_b + 6 * per_b +
+                  align(rwt::kRestWords * 4);
 
   const size_t ks = key_bits == 32 ? 4 : 8;
   cudaError_t e = cudaMalloc(&b->d_tables, (8 + rwt::kMaxSortClasses) * tab * 4);
   if (e == cudaSuccess) e = cudaMalloc(&b->d_tmp_keys, ks * total);
   b->tree_far_cap = b->tree_tiles * rwt::kTreeFarPerTile;
   if (e == cudaSuccess) e = cudaMalloc(&b->d_tree_far, size_t(b->tree_far_cap) * 16);
+  if (e == cudaSuccess && b->low_bits)
+    e = cudaMalloc(&b->d_rest, rwt::rest_words(n_clouds, b->n_total) * 4);
   if (e == cudaSuccess) e = cudaMalloc(&b->d_zero, b->zero_bytes);
   if (e == cudaSuccess) e = cudaMallocHost(&b->h_results, (3 * size_t(n_clouds) + 4) * 4);
   if (e != cudaSuccess) {
@@ -322,7 +327,8 @@ int rw_tree_batch_create(const uint32_t* cloud_sizes, uint32_t n_clouds, int32_t
   b->d_n_octree = reinterpret_cast<uint32_t*>(z + o); o += per_b;
   b->d_seg_err = reinterpret_cast<int32_t*>(z + o); o += per_b;
   b->d_skew = reinterpret_cast<uint32_t*>(z + o); o += per_b;
-  b->d_long_run = reinterpret_cast<uint32_t*>(z + o); o += per_b;
+  b->d_dense = reinterpret_cast<uint32_t*>(z + o); o += 2 * per_b;
+  b->d_rest_ctr = reinterpret_cast<uint32_t*>(z + o);
 
   std::vector<uint32_t> all;
   all.reserve(8 * tab);
@@ -346,6 +352,7 @@ int rw_tree_batch_destroy(rw_tree_batch* b) {
   if (b->d_tables) cudaFree(b->d_tables);
   if (b->d_tmp_keys) cudaFree(b->d_tmp_keys);
   if (b->d_tree_far) cudaFree(b->d_tree_far);
+  if (b->d_rest) cudaFree(b->d_rest);
   if (b->d_zero) cudaFree(b->d_zero);
   if (b->h_results) cudaFreeHost(b->h_results);
   delete b;

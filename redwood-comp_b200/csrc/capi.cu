@@ -98,7 +98,9 @@ rwt::Scratch scratch_of(const rw_tree_im_storage* im) {
   sc.ghist = im->d_ghist;
   sc.skew = im->d_skew;
   sc.low_bits = im->low_bits;
-  sc.long_run = im->d_long_run;
+  sc.dense = im->d_dense;
+  sc.rest = im->d_rest;
+  sc.rest_ctr = im->d_rest_ctr;
   sc.sort_desc = im->d_sort_desc;
   sc.sort_rows = im->sort_tiles + 1;
   sc.unique_desc = im->d_unique_desc;
@@ -229,7 +231,7 @@ int rw_tree_im_storage_create_ex(uint32_t n_input, int32_t key_bits,
 
   auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
   const size_t ghist_b = align(size_t(im->passes) * radix * 4);
-  const size_t skew_b = align(4), long_b = align(4);
+  const size_t skew_b = align(4), dense_b = align(2 * 4);
   const size_t sdesc_b = align(size_t(im->passes) * (im->sort_tiles + 1) * radix * 4);
   const size_t udesc_b = align((size_t(rwt::div_up(n_input, rwt::kUniqueTile)) + 1) * 4);
   // stage 6's tiles, or the octree's (smaller) ones in the fused pipeline
@@ -237,7 +239,8 @@ int rw_tree_im_storage_create_ex(uint32_t n_input, int32_t key_bits,
   static_assert(rwt::kOctTile <= rwt::kScanTile, "scan descriptors sized by the octree tiles");
   const size_t ctr_b = align(rwt::kCounters * 4);
   const size_t st_b = align(sizeof(rwt::DevStatus));
-  im->zero_bytes = ghist_b + skew_b + long_b + sdesc_b + udesc_b + cdesc_b + ctr_b + st_b;
+  const size_t rctr_b = im->low_bits ? align(rwt::kRestWords * 4) : 0;
+  im->zero_bytes = ghist_b + skew_b + dense_b + sdesc_b + udesc_b + cdesc_b + ctr_b + st_b + rctr_b;
 
   // one allocation: the zero region, the ping-pong keys (and, behind the keys
   // of a small cloud, the scratch of its one-launch pipeline), the far list
@@ -250,8 +253,9 @@ int rw_tree_im_storage_create_ex(uint32_t n_input, int32_t key_bits,
     keys_b = std::max(keys_b, small_at + rwt::small_scratch_bytes(n_input, key_bits, sms));
   keys_b = align(keys_b);
   im->tree_far_cap = rwt::div_up(n_input, rwt::kTreeTile) * rwt::kTreeFarPerTile;
-  if (e == cudaSuccess)
-    e = cudaMalloc(&im->d_zero, im->zero_bytes + keys_b + size_t(im->tree_far_cap) * 16);
+  const size_t far_b = size_t(im->tree_far_cap) * 16;
+  const size_t rest_b = im->low_bits ? rwt::rest_words(1, n_input) * 4 : 0;
+  if (e == cudaSuccess) e = cudaMalloc(&im->d_zero, im->zero_bytes + keys_b + far_b + rest_b);
   if (e == cudaSuccess) e = cudaMallocHost(&im->h_status, sizeof(rwt::DevStatus));
   if (e != cudaSuccess) {
     rw_tree_im_storage_destroy(im);
@@ -261,15 +265,17 @@ int rw_tree_im_storage_create_ex(uint32_t n_input, int32_t key_bits,
   im->d_tmp_keys = z + im->zero_bytes;
   if (small) im->d_small = z + im->zero_bytes + small_at;
   im->d_tree_far = reinterpret_cast<uint32_t*>(z + im->zero_bytes + keys_b);
+  if (rest_b) im->d_rest = reinterpret_cast<uint32_t*>(z + im->zero_bytes + keys_b + far_b);
   size_t o = 0;
   im->d_ghist = reinterpret_cast<uint32_t*>(z + o); o += ghist_b;
   im->d_skew = reinterpret_cast<uint32_t*>(z + o); o += skew_b;
-  im->d_long_run = reinterpret_cast<uint32_t*>(z + o); o += long_b;
+  im->d_dense = reinterpret_cast<uint32_t*>(z + o); o += dense_b;
   im->d_sort_desc = reinterpret_cast<uint32_t*>(z + o); o += sdesc_b;
   im->d_unique_desc = reinterpret_cast<uint32_t*>(z + o); o += udesc_b;
   im->d_scan_desc = reinterpret_cast<uint32_t*>(z + o); o += cdesc_b;
   im->d_tile_ctr = reinterpret_cast<uint32_t*>(z + o); o += ctr_b;
-  im->d_status = reinterpret_cast<rwt::DevStatus*>(z + o);
+  im->d_status = reinterpret_cast<rwt::DevStatus*>(z + o); o += st_b;
+  if (rctr_b) im->d_rest_ctr = reinterpret_cast<uint32_t*>(z + o);
   std::memset(im->h_status, 0, sizeof(rwt::DevStatus));
   e = cudaMemset(im->d_zero, 0, im->zero_bytes);
   if (e != cudaSuccess) {

@@ -27,6 +27,8 @@ struct rw_tree_im_storage {
   uint32_t sort_tiles = 0;  // tiles per pass at n_cap
 
   void* d_tmp_keys = nullptr;  // [n_cap] ping-pong buffer of the sort
+  uint32_t* d_rest_ctr = nullptr;   // [kRestWords] (64-bit keys)
+  uint32_t* d_rest = nullptr;       // [rest_words], not zeroed (64-bit keys)
   uint32_t* d_tree_far = nullptr;  // far links of the octree
   uint32_t tree_far_cap = 0;       // entries (16 bytes each)
 
@@ -35,7 +37,7 @@ struct rw_tree_im_storage {
   size_t zero_bytes = 0;
   uint32_t* d_ghist = nullptr;      // [passes][radix]
   uint32_t* d_skew = nullptr;       // [1]: the top sort pass's digits are skewed
-  uint32_t* d_long_run = nullptr;   // [1]: a run was too long for k_sort_fix
+  uint32_t* d_dense = nullptr;      // [2]: Scratch::dense
   uint32_t* d_sort_desc = nullptr;  // [passes][sort_tiles + 1][radix]
   uint32_t* d_unique_desc = nullptr;
   uint32_t* d_scan_desc = nullptr;
@@ -61,7 +63,7 @@ struct rw_tree_im_storage {
 namespace rwt {
 
 enum : int { kCtrUnique = 0, kCtrScan = 1, kCtrTree = 2, kCtrLinks = 3, kCtrSortBase = 4,
-             kMaxPasses = 8, kCtrSortClassStride = kMaxPasses, kMaxSortClasses = 4, kCtrSmall = 48, kCtrLong = 56, kCounters = 64 };
+             kMaxPasses = 8, kCtrSortClassStride = kMaxPasses, kMaxSortClasses = 4, kCtrSmall = 48, kCounters = 64 };
 
 // Tile sizes of the kernels (points or nodes per tile).
 constexpr uint32_t kPointTile = 4096;  // Morton / histogram
@@ -85,6 +87,11 @@ inline int sort_low_bits(int key_bits, int radix_bits, uint32_t largest) {
   if (key_bits != 64 || radix_bits != 8) return 0;
   return largest <= kSplitPoints ? kSplitLow32 : kSplitLow40;
 }
+// k_sort_rest's counters: dense segments, listed runs, passes over dense segments,
+// then tickets and jobs done of each of its phases; a listed run has more than 256 keys.
+enum : int { kRestDense = 0, kRestRuns = 1, kRestPasses = 2, kRestTickets = 3, kRestWords = 32 };
+inline uint32_t rest_runs(uint32_t n) { return n / 257u + 1u; }
+size_t rest_words(uint32_t segments, uint32_t n);
 inline int sort_pass_count(int key_bits, int radix_bits, uint32_t largest) {
   const int bits = (key_bits == 32 ? 30 : 63) - sort_low_bits(key_bits, radix_bits, largest);
   return (bits + radix_bits - 1) / radix_bits;
@@ -138,9 +145,12 @@ struct Scratch {
   // the kRankMixed variants read it)
   uint32_t* skew = nullptr;
   // low bits that the passes leave to launch_sort_finish (0: none), and
-  // [segments]: 1 when a run of keys with equal top bits was too long for it
+  // [segments]: 1 when the segment is dense and the passes leave it alone, then
+  // [segments]: pairs of its samples with equal top bits (k_keys.cu)
   int low_bits = 0;
-  uint32_t* long_run = nullptr;
+  uint32_t* dense = nullptr;
+  uint32_t* rest_ctr = nullptr;  // [kRestWords], zeroed
+  uint32_t* rest = nullptr;      // [rest_words]
   // the keys are codes that stage 1 makes in the same chain, whose top bits are
   // clear; else a caller's, which are sorted by the whole word
   bool codes = false;
@@ -198,8 +208,8 @@ cudaError_t launch_keys(const Bufs& b, const Scratch& sc, const Plan& pl, bool e
 cudaError_t launch_sort_passes(const Bufs& b, const Scratch& sc, const Plan& pl,
                                cudaStream_t s, cudaEvent_t* marks = nullptr);
 // After the passes of every segment, when they leave bits out (low_bits): the
-// order within runs of equal top bits, and stage 3's counts per tile
-// (launch_unique's `counted`).
+// order within runs of equal top bits, the dense segments, and stage 3's counts
+// per tile (launch_unique's `counted`).
 cudaError_t launch_sort_finish(const Bufs& b, const Scratch& sc, const Plan& pl,
                                cudaStream_t s);
 // The onesweep sort of keys[0, n) into out on `im`'s scratch, with every

@@ -19,9 +19,9 @@
 // default 32-bit variant (384 threads x 24 keys) runs three blocks per SM.
 #include <algorithm>
 
+#include "binning.cuh"
 #include "internal.hpp"
 #include "morton.cuh"
-#include "rank.cuh"
 
 namespace rwt {
 
@@ -45,19 +45,96 @@ __host__ __device__ constexpr uint32_t pass_mask(int p) {
   return CODES && sizeof(K) == 4 && D == 8 && p == 2 ? 0x7fu : (1u << D) - 1u;
 }
 
+// Keys that share their top bits are counted against one another at the end of a
+// sort that leaves low bits out (k_sort_fix), in time proportional to their
+// number.  Segments where a key shares them with kDenseRun - 1 others on average
+// take all digits instead: of 2,000,000 points, runs of 36 keys take 269 us by
+// counting and 293 by all digits, runs of 9 keys 238 and 293.  That is decided from samples, which blocks of stage
+// 1 take beside their others (in a block of k_sort_init they were 10 us that all
+// waited for): of S keys, S^2 / 2 * r / n pairs share their top bits when a key's
+// run has r keys on average.  The keys are those at random places, not every
+// (n / S)-th: neighbours in the input may be neighbours in space.  Sorted either
+// way the result is the same; a sample that misses costs time only.
+constexpr int kDenseSamples = 1024, kDenseSlots = 2 * kDenseSamples;
+constexpr uint32_t kDenseRun = 48, kDenseFrom = 4096;
+
+__host__ __device__ __forceinline__ uint32_t dense_blocks(uint32_t segments) {
+  return segments == 1 ? 4u : 1u;  // per segment
+}
+__device__ __forceinline__ bool is_dense(uint32_t pairs, uint32_t n, uint32_t segments) {
+  constexpr unsigned long long kAll = (kDenseSamples / 2) * kDenseSamples;
+  return n > kDenseFrom && pairs > 2 && pairs * (unsigned long long)n >
+                                            kDenseRun * kAll * dense_blocks(segments);
+}
+
+// One block's samples: the pairs among kDenseSamples of n keys, which key(i) gives
+// without their low bits, added to *pairs.
+template <typename KeyAt>
+__device__ __forceinline__ void dense_sample(uint32_t n, const KeyAt& key, uint32_t* pairs) {
+  // a slot: the top bits (41 at most) << 20 | how many samples had them
+  __shared__ unsigned long long s_slot[kDenseSlots];
+  if (n <= kDenseFrom) return;
+  uint64_t k[kDenseSamples / 256];
+#pragma unroll
+  for (int q = 0; q < kDenseSamples / 256; ++q) {
+    uint32_t x = (blockIdx.x * kDenseSamples + 256u * q + threadIdx.x) * 0x9e3779b9u + n;
+    x = (x ^ (x >> 16)) * 0x85ebca6bu;  // murmur3's finisher
+    x = (x ^ (x >> 13)) * 0xc2b2ae35u;
+    k[q] = key(__umulhi(x ^ (x >> 16), n));
+  }
+  for (int i = int(threadIdx.x); i < kDenseSlots; i += 256) s_slot[i] = 0;
+  __syncthreads();
+  uint32_t found = 0;
+#pragma unroll
+  for (int q = 0; q < kDenseSamples / 256; ++q) {
+    const unsigned long long top = (unsigned long long)k[q] << 20;
+    uint32_t at = uint32_t((k[q] * 0x9e3779b97f4a7c15ull) >> 53);
+    static_assert(kDenseSlots == 1 << 11, "11 bits of the hash");
+    for (int probe = 0; probe < kDenseSlots; ++probe, at = (at + 1) % kDenseSlots) {
+      unsigned long long old = s_slot[at];
+      if (old == 0) old = atomicCAS(&s_slot[at], 0ull, top | 1ull);
+      if (old == 0) break;
+      if ((old ^ top) >> 20 == 0) {
+        found += atomicAdd(reinterpret_cast<uint32_t*>(&s_slot[at]), 1u) & 0xfffffu;
+        break;
+      }
+    }
+  }
+  found = warp_sum(found);
+  if (lane_id() == 0 && found) atomicAdd(pairs, found);
+}
+
 // Points are walked in tiles of kPointTile that never straddle two segments;
 // each CTA takes a contiguous run of tiles, so with HIST its shared-memory
 // histograms are flushed to the segment's global ones only when the segment
 // changes.  ghist: [segments][passes][RADIX].
-// LOW: the low bits that the sort's passes leave out.
+// LOW: the low bits that the sort's passes leave out; then the first blocks
+// (dense_blocks per segment) take samples, if pairs [segments] is given.
 template <typename K, int D, int LOW, bool HIST, bool ENCODE, bool POW2>
 __global__ void __launch_bounds__(256)
     k_keys_pass(const float4* __restrict__ pts, K* __restrict__ keys, SegTable seg,
                 TileMap map, uint32_t tiles_per_cta, float min_coord, float range,
                 float inv_range, uint32_t* __restrict__ ghist,
-                const uint32_t* __restrict__ gate) {
+                const uint32_t* __restrict__ gate, uint32_t* __restrict__ pairs) {
   pdl_enter();
   if (gate && *gate == 0) return;  // a gated sort that is not needed this run
+  uint32_t block = blockIdx.x;
+  if constexpr (HIST && LOW > 0) {
+    const uint32_t per = pairs ? dense_blocks(seg.count) : 0u;
+    if (block < per * seg.count) {
+      const uint32_t c = block / per, sb = seg_begin(seg, c);
+      dense_sample(seg_size(seg, c), [&](uint32_t i) -> uint64_t {
+        if constexpr (ENCODE) {
+          const float4 p = pts[sb + i];
+          return encode<K, POW2>(p.x, p.y, p.z, min_coord, range, inv_range) >> LOW;
+        } else {
+          return keys[sb + i] >> LOW;
+        }
+      }, pairs + c);
+      return;
+    }
+    block -= per * seg.count;
+  }
   constexpr int RADIX = 1 << D;
   // the sort's passes: ceil(sorted bits / D), as the storage computes them
   constexpr int P = (KeyTraits<K>::kCodeBits - LOW + D - 1) / D;
@@ -67,7 +144,7 @@ __global__ void __launch_bounds__(256)
     for (int i = threadIdx.x; i < nh; i += blockDim.x) s_hist[i] = 0;
     __syncthreads();
   }
-  const uint32_t t0 = blockIdx.x * tiles_per_cta;
+  const uint32_t t0 = block * tiles_per_cta;
   const uint32_t t1 = min(t0 + tiles_per_cta, map.n_tiles);
   uint32_t cur = 0xffffffffu;
   auto flush = [&](uint32_t c) {
@@ -143,11 +220,14 @@ __global__ void __launch_bounds__(256)
 // chance that two keys share a digit, sum over digits of (count / n)^2, above
 // 2^-skew_log2 (many lanes of a warp on one digit then serialise the
 // atomic-OR ranking, which the ballot ranking does not).
-template <int D>
+// DENSE: it also decides which segments are dense, by the pairs that stage 1's
+// samples found (all: every one is).
+template <int D, bool DENSE>
 __global__ void __launch_bounds__(256)
     k_sort_init(const uint32_t* __restrict__ ghist, uint32_t* __restrict__ desc,
                 SegTable seg, TileMap map, int passes, uint32_t rows_per_pass,
-                const uint32_t* __restrict__ gate, uint32_t* __restrict__ skew, int skew_log2) {
+                const uint32_t* __restrict__ gate, uint32_t* __restrict__ skew, int skew_log2,
+                uint32_t* __restrict__ dense, uint32_t* __restrict__ dense_n, bool all) {
   pdl_enter();
   if (gate && *gate == 0) return;
   constexpr int RADIX = 1 << D;
@@ -157,6 +237,11 @@ __global__ void __launch_bounds__(256)
   const uint32_t c = blockIdx.x / passes;
   const int pass = int(blockIdx.x % passes);
   if (map.toff && map.toff[c + 1] == map.toff[c]) return;  // no tile in this map
+  if (DENSE && dense && pass == 0 && threadIdx.x == 0 &&
+      (all || is_dense(dense[seg.count + c], seg_size(seg, c), seg.count))) {
+    dense[c] = 1u;
+    atomicAdd(dense_n, 1u);
+  }
   const uint32_t* h = ghist + (size_t(c) * passes + pass) * RADIX;
   const uint32_t init_row = (map.toff ? map.toff[c] : 0u) + c;
   uint32_t* row0 = desc + (size_t(pass) * rows_per_pass + init_row) * RADIX;
@@ -196,26 +281,6 @@ __global__ void __launch_bounds__(256)
 // ---------------------------------------------------------------------------
 
 
-// Descriptors a look-back reads per round trip.
-constexpr int kLookback = 8;
-
-template <typename K, int D, int THREADS, int KPT, int RANK>
-struct BinCfg {
-  static constexpr int RADIX = 1 << D;
-  static constexpr int NW = THREADS / 32;
-  static constexpr int TILE = THREADS * KPT;
-  static constexpr size_t kKeysBytes = size_t(TILE) * sizeof(K);
-  // one set of counters per warp; the unordered scheme has one per block
-  static constexpr size_t kHistBytes = size_t(RANK == kRankUnordered ? 1 : NW) * RADIX * 4;
-  // the two-array scheme keeps a match-mask array beside the counters; the
-  // half-warp scheme has two words per digit and warp (one per half-warp)
-  static constexpr size_t kMatchBytes =
-      (RANK == kRankAtomicOr || RANK == kRankHalfPacked || RANK == kRankMixed) ? kHistBytes : 0;
-  static constexpr size_t kSmem =
-      kKeysBytes + kHistBytes + kMatchBytes + 3 * size_t(RADIX) * 4 + 64 * 4;
-  static_assert(kSmem <= 227 * 1024, "onesweep variant exceeds shared memory per CTA");
-};
-
 // One onesweep pass over `n` keys: digit `shift`..`shift+D-1`, stable.
 // desc: [(tiles + 1) x RADIX] descriptors, row 0 prefilled with the global
 // exclusive digit offsets (k_sort_init), rows 1.. zero.
@@ -224,273 +289,47 @@ struct BinCfg {
 // that a pass that is not needed costs one short wave of CTAs.  A CTA holds a
 // ticket only while it runs, so every look-back still waits only on running
 // tiles, whatever the grid.
+// skip (64-bit keys): [segments] those that the pass leaves alone.
 template <typename K, int D, int THREADS, int KPT, int RANK, int MINB, bool PERSIST, int BB = D>
 __global__ void __launch_bounds__(THREADS, MINB)
     k_binning(const K* __restrict__ in, K* __restrict__ out, SegTable seg, TileMap map,
               int shift, uint32_t dmask, uint32_t* __restrict__ desc,
               uint32_t* __restrict__ tile_ctr, DevStatus* __restrict__ st,
               uint32_t spin_limit, const uint32_t* __restrict__ gate,
-              const uint32_t* __restrict__ skew) {
+              const uint32_t* __restrict__ skew, const uint32_t* __restrict__ skip) {
   pdl_enter();
   if (gate && *gate == 0) return;  // every tile of the pass returns: no look-back waits
   using C = BinCfg<K, D, THREADS, KPT, RANK>;
-  constexpr int RADIX = C::RADIX, NW = C::NW, TILE = C::TILE;
   extern __shared__ __align__(16) unsigned char smem[];
-  K* s_keys = reinterpret_cast<K*>(smem);
-  uint32_t* s_hist = reinterpret_cast<uint32_t*>(smem + C::kKeysBytes);
-  uint32_t* s_match = s_hist + NW * RADIX;  // only with kRankAtomicOr / kRankMixed
-  uint32_t* s_cnt = reinterpret_cast<uint32_t*>(smem + C::kKeysBytes + C::kHistBytes +
-                                                C::kMatchBytes);
-  uint32_t* s_start = s_cnt + RADIX;
-  uint32_t* s_gofs = s_start + RADIX;
-  uint32_t* s_misc = s_gofs + RADIX;  // [0] tile, [1..] warp scan scratch
-
-  const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+  uint32_t* s_tile = reinterpret_cast<uint32_t*>(smem + C::kSmem - 64 * 4);
+  uint32_t off = 0;
+  if (sizeof(K) == 8 && skip && !map.toff) off = skip[0];
   for (;;) {
-    if (tid == 0) s_misc[0] = atomicAdd(tile_ctr, 1u);
-    {
-      static_assert(RADIX % 4 == 0 && C::kKeysBytes % 16 == 0, "16-byte zeroing");
-      const uint4 z = make_uint4(0, 0, 0, 0);
-      constexpr int kWords =
-          (RANK == kRankAtomicOr || RANK == kRankHalfPacked || RANK == kRankMixed ? 2 : 1) *
-          (RANK == kRankUnordered ? 1 : NW) * RADIX;
-      for (int i = tid; i < kWords / 4; i += THREADS) reinterpret_cast<uint4*>(s_hist)[i] = z;
-    }
+    if (threadIdx.x == 0) *s_tile = atomicAdd(tile_ctr, 1u);
+    bin_zero<K, D, THREADS, KPT, RANK>(smem);
     __syncthreads();
-    const uint32_t tile = s_misc[0];
+    const uint32_t tile = *s_tile;
     if (PERSIST && tile >= map.n_tiles) break;  // block-uniform
+    if (sizeof(K) == 8 && off) return;
     uint32_t first_tile;
     const uint32_t segc = tile_segment(seg, map, tile, &first_tile);
-    const uint32_t base = seg_begin(seg, segc) + (tile - first_tile) * TILE;
+    const uint32_t base = seg_begin(seg, segc) + (tile - first_tile) * C::TILE;
     const uint32_t n = seg_begin(seg, segc) + seg_size(seg, segc);  // end of the segment
-    const int row = int(tile + segc + 1);       // this tile's descriptor row
+    const int row = int(tile + segc + 1);         // this tile's descriptor row
     const int init_row = int(first_tile + segc);  // the segment's inclusive row
-    const bool full = base + TILE <= n;
-
-    // load: warp w owns [w*32*KPT, (w+1)*32*KPT) of the tile, 32 keys per step
-    // (half-warp scheme: half h of warp w owns [w*32*KPT + h*16*KPT, +16*KPT),
-    // 16 keys per step)
-    K keys[KPT];
-    uint32_t rank2[RankPack<KPT>::kRegs];  // packed warp ranks
-    uint32_t rank16[(KPT + 1) / 2];        // unordered: the block's ranks
-    const uint32_t wbase = base + warp * 32u * KPT + lane;
-    const uint32_t hbase = base + warp * 32u * KPT + (lane >> 4) * 16u * KPT + (lane & 15u);
-    uint32_t* wh = s_hist + warp * RADIX;
-    uint32_t* wm = s_match + warp * RADIX;
-    uint32_t* wp = s_hist + warp * 2u * RADIX;  // half-warp scheme: [2 RADIX] per warp
-    if (RANK == kRankUnordered) {
-      // any order within a digit will do, so ranks come straight from the
-      // block's counters: one shared atomic per key instead of four accesses, a
-      // shuffle and two population counts (16.8M 32-bit keys 71.7 -> 55.5 us,
-      // 5,000,011 64-bit keys 36.8 -> 30.7)
-      static_assert(TILE <= 65536, "16-bit ranks");
-      if (full) {
-  #pragma unroll
-        for (int i = 0; i < KPT; ++i) keys[i] = in[wbase + 32u * i];
-      } else {
-  #pragma unroll
-        for (int i = 0; i < KPT; ++i) keys[i] = wbase + 32u * i < n ? in[wbase + 32u * i] : K(0);
-      }
-      if (full) {
-  #pragma unroll
-        for (int i = 0; i < KPT; ++i) {
-          const uint32_t dig = uint32_t(keys[i] >> shift) & dmask;
-          const uint32_t r = atomicAdd(&s_hist[dig], 1u);
-          if (i % 2 == 0) rank16[i / 2] = r;
-          else rank16[i / 2] |= r << 16;
-        }
-      } else {
-  #pragma unroll
-        for (int i = 0; i < KPT; ++i) {
-          const uint32_t dig = uint32_t(keys[i] >> shift) & dmask;
-          const uint32_t r = wbase + 32u * i < n ? atomicAdd(&s_hist[dig], 1u) : 0u;
-          if (i % 2 == 0) rank16[i / 2] = r;
-          else rank16[i / 2] |= r << 16;
-        }
-      }
-    } else if (RANK == kRankHalfPacked) {
-      if (full) {
-  #pragma unroll
-        for (int i = 0; i < KPT; ++i) keys[i] = in[hbase + 16u * i];
-        half_rank<D, KPT, true>(keys, rank2, shift, hbase, n, wp, dmask);
-      } else {
-  #pragma unroll
-        for (int i = 0; i < KPT; ++i) {
-          const uint32_t idx = hbase + 16u * i;
-          keys[i] = idx < n ? in[idx] : K(0);
-        }
-        half_rank<D, KPT, false>(keys, rank2, shift, hbase, n, wp, dmask);
-      }
-    } else if (RANK == kRankMixed) {
-      // this segment's digits decide the scheme (block-uniform)
-      const bool ballots = skew != nullptr && skew[segc] != 0u;
-      if (full) {
-  #pragma unroll
-        for (int i = 0; i < KPT; ++i) keys[i] = in[wbase + 32u * i];
-        warp_rank<D, KPT, kRankMixed, true, BB>(keys, rank2, shift, wbase, n, wh, wm, KPT, ballots,
-                                                dmask);
-      } else {
-  #pragma unroll
-        for (int i = 0; i < KPT; ++i) {
-          const uint32_t idx = wbase + 32u * i;
-          keys[i] = idx < n ? in[idx] : K(0);
-        }
-        warp_rank<D, KPT, kRankMixed, false, BB>(keys, rank2, shift, wbase, n, wh, wm, KPT,
-                                                 ballots, dmask);
-      }
-    } else if (full) {
-  #pragma unroll
-      for (int i = 0; i < KPT; ++i) keys[i] = in[wbase + 32u * i];
-      warp_rank<D, KPT, RANK, true, BB>(keys, rank2, shift, wbase, n, wh, wm, KPT, false, dmask);
-    } else {
-  #pragma unroll
-      for (int i = 0; i < KPT; ++i) {
-        const uint32_t idx = wbase + 32u * i;
-        keys[i] = idx < n ? in[idx] : K(0);
-      }
-      warp_rank<D, KPT, RANK, false, BB>(keys, rank2, shift, wbase, n, wh, wm, KPT, false, dmask);
-    }
-    __syncthreads();
-
-    // per digit: exclusive scan over warps (half-warps) and publish the tile
-    // aggregate
-    uint32_t* drow = desc + size_t(row) * RADIX;
-    if (RANK == kRankHalfPacked) {
-      // lane pairs own a digit: the even lane its half-warp-0 words, the odd
-      // lane its half-warp-1 words (consecutive addresses, no bank conflicts);
-      // units run in the order (warp, half), the partner's count by a shuffle
-      static_assert((2 * RADIX) % 32 == 0 && THREADS % 32 == 0, "whole warps per pass");
-      for (int x = tid; x < 2 * RADIX; x += THREADS) {
-        const uint32_t h = uint32_t(x) & 1u;
-        uint32_t run = 0;
-  #pragma unroll
-        for (int w = 0; w < NW; ++w) {
-          uint32_t* p = s_hist + w * 2 * RADIX + x;
-          const uint32_t mine = *p >> 16;
-          const uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 1);
-          *p = run + (h ? other : 0u);
-          run += mine + other;
-        }
-        if (!h) {
-          s_cnt[x >> 1] = run;
-          st_relaxed(drow + (x >> 1), kFlagAgg | (run << 2));
-        }
-      }
-    } else {
-      for (int d = tid; d < RADIX; d += THREADS) {
-        uint32_t run = 0;
-        if (RANK == kRankUnordered) {
-          run = s_hist[d];
-        } else {
-  #pragma unroll
-          for (int w = 0; w < NW; ++w) {
-            const uint32_t c = s_hist[w * RADIX + d];
-            s_hist[w * RADIX + d] = run;
-            run += c;
-          }
-        }
-        s_cnt[d] = run;
-        st_relaxed(drow + d, kFlagAgg | (run << 2));
-      }
-    }
-    __syncthreads();
-    digit_exclusive_scan<D, THREADS>(s_cnt, s_start, s_misc + 1);
-    __syncthreads();
-    // fold the digit starts into the per-warp offsets once per tile, so that
-    // placing a key below reads one shared-memory word instead of two
-    if (RANK == kRankHalfPacked) {
-      for (int i = tid; i < 2 * NW * RADIX; i += THREADS)
-        s_hist[i] += s_start[(i >> 1) & (RADIX - 1)];
-    } else if (RANK != kRankUnordered) {
-      for (int i = tid; i < NW * RADIX; i += THREADS) s_hist[i] += s_start[i & (RADIX - 1)];
-    }
-    if (RANK != kRankUnordered) __syncthreads();
-
-    // reorder the tile by digit in shared memory first: it needs only the
-    // tile's own counts, and gives the predecessors time to publish their
-    // inclusive prefixes before the look-back below reads them
-    if (RANK == kRankUnordered) {
-      if (full) {
-  #pragma unroll
-        for (int i = 0; i < KPT; ++i) {
-          const uint32_t dig = uint32_t(keys[i] >> shift) & dmask;
-          s_keys[s_start[dig] + ((rank16[i / 2] >> (16 * (i % 2))) & 0xffffu)] = keys[i];
-        }
-      } else {
-  #pragma unroll
-        for (int i = 0; i < KPT; ++i)
-          if (wbase + 32u * i < n) {
-            const uint32_t dig = uint32_t(keys[i] >> shift) & dmask;
-            s_keys[s_start[dig] + ((rank16[i / 2] >> (16 * (i % 2))) & 0xffffu)] = keys[i];
-          }
-      }
-    } else if (RANK == kRankHalfPacked) {
-      if (full) half_place<D, KPT, true>(keys, rank2, shift, hbase, n, wp, s_keys, dmask);
-      else half_place<D, KPT, false>(keys, rank2, shift, hbase, n, wp, s_keys, dmask);
-    } else if (full) {
-      warp_place<D, KPT, true>(keys, rank2, shift, wbase, n, wh, s_keys, KPT, dmask);
-    } else {
-      warp_place<D, KPT, false>(keys, rank2, shift, wbase, n, wh, s_keys, KPT, dmask);
-    }
-
-    // decoupled look-back, kLookback descriptors per round trip.  The segment's
-    // first row is always inclusive, so rows are read clamped to it and the
-    // walk stops there at the latest.
-    for (int d = tid; d < RADIX; d += THREADS) {
-      uint32_t excl = 0;
-      int k = row - 1;
-      uint32_t spin = 0;
-      while (true) {
-        uint32_t v[kLookback];
-  #pragma unroll
-        for (int q = 0; q < kLookback; ++q)
-          v[q] = ld_relaxed(desc + size_t(max(k - q, init_row)) * RADIX + d);
-        int used = 0;
-        bool done = false;
-  #pragma unroll
-        for (int q = 0; q < kLookback; ++q) {
-          const uint32_t f = v[q] & kFlagMask;
-          if (done || f == 0 || used != q) break;
-          excl += v[q] >> 2;
-          ++used;
-          done = f == kFlagInc;
-        }
-        if (done) break;
-        if (used) {
-          k -= used;
-          spin = 0;
-          continue;
-        }
-        if (++spin > spin_limit || device_failed(st)) {
-          report_error(st, RW_ERR_TIMEOUT, kSiteSort);
-          break;
-        }
-        backoff(spin);
-      }
-      st_relaxed(drow + d, kFlagInc | ((excl + s_cnt[d]) << 2));
-      s_gofs[d] = excl - s_start[d];
-    }
-    __syncthreads();
-
-    // write runs of equal digits to their global positions (a destination is
-    // out of range only if a look-back gave up)
-    const uint32_t total = seg.total;
-    if (full) {
-  #pragma unroll 4
-      for (int i = 0; i < KPT; ++i) {
-        const uint32_t p = tid + uint32_t(i) * THREADS;
-        const K k = s_keys[p];
-        const uint32_t dst = s_gofs[uint32_t(k >> shift) & dmask] + p;
-        if (dst < total) out[dst] = k;
-      }
-    } else {
-      const uint32_t tile_n = n - base;
-      for (uint32_t p = tid; p < tile_n; p += THREADS) {
-        const K k = s_keys[p];
-        const uint32_t dst = s_gofs[uint32_t(k >> shift) & dmask] + p;
-        if (dst < total) out[dst] = k;
-      }
-    }
+    uint32_t* drow = desc + size_t(row) * C::RADIX;
+    uint32_t seg_off = 0;
+    if (sizeof(K) == 8 && skip && map.toff) seg_off = skip[segc];
+    // this segment's digits decide the ranking scheme (block-uniform)
+    const bool ballots = RANK == kRankMixed && skew != nullptr && skew[segc] != 0u;
+    bin_tile<K, D, THREADS, KPT, RANK, BB>(
+        smem, in, out, base, n, seg.total, shift, dmask, ballots, seg_off,
+        [&](uint32_t d, uint32_t count) { st_relaxed(drow + d, kFlagAgg | (count << 2)); },
+        [&](uint32_t d, uint32_t count) {
+          const uint32_t excl = look_back<C::RADIX>(desc, d, row, init_row, spin_limit, st);
+          st_relaxed(drow + d, kFlagInc | ((excl + count) << 2));
+          return excl;
+        });
     if (!PERSIST) break;
     __syncthreads();  // the next tile reuses every shared array
   }
@@ -516,6 +355,7 @@ cudaError_t keys_t(const Bufs& b, const Scratch& sc, const Plan& pl, bool encode
   const size_t smem = hist ? size_t(sc.passes) * (1u << D) * 4 : 0;
   K* keys = static_cast<K*>(b.keys);
   const float inv = pow2_reciprocal(b.range);
+  const uint32_t samples = LOW ? dense_blocks(pl.seg.count) * pl.seg.count : 0u;
 #define RWT_KEYS_LAUNCH(H, E)                                                        \
   do {                                                                               \
     constexpr int kLow = E ? LOW : kWordLow;                                         \
@@ -523,8 +363,9 @@ cudaError_t keys_t(const Bufs& b, const Scratch& sc, const Plan& pl, bool encode
                             : k_keys_pass<K, D, kLow, H, E, false>;                  \
     if (smem > 48 * 1024)                                                            \
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)); \
-    launch_pdl(kern, grid, 256, smem, s, b.points, keys, pl.seg, pl.point_map, per, b.min_coord, \
-                                 b.range, inv, sc.ghist, sc.gate);                   \
+    launch_pdl(kern, grid + (H ? samples : 0u), 256, smem, s, b.points, keys, pl.seg,       \
+               pl.point_map, per, b.min_coord, b.range, inv, sc.ghist, sc.gate,             \
+               samples ? sc.dense + pl.seg.count : static_cast<uint32_t*>(nullptr));        \
   } while (0)
   if (encode && hist) RWT_KEYS_LAUNCH(true, true);
   else if (encode) RWT_KEYS_LAUNCH(false, true);
@@ -588,8 +429,12 @@ cudaError_t passes_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStrea
       P != (KeyTraits<K>::kCodeBits - low + D - 1) / D || P > kMaxPasses ||
       (low != 0) != (sizeof(K) == 8 && D == 8))
     return cudaErrorInvalidValue;
-  launch_pdl(k_sort_init<D>, pl.seg.count * sc.passes, 256, 0, s, sc.ghist, sc.sort_desc, pl.seg,
-             pl.sort_map, sc.passes, sc.sort_rows, sc.gate, skew, kSkewLog2);
+  // (the first of several passes would overwrite keys that are sorted in place)
+  const bool rest = low != 0 && !probe_spins;
+  launch_pdl(k_sort_init<D, sizeof(K) == 8 && D == 8>, pl.seg.count * sc.passes, 256, 0, s,
+             sc.ghist, sc.sort_desc, pl.seg, pl.sort_map, sc.passes, sc.sort_rows, sc.gate, skew,
+             kSkewLog2, rest ? sc.dense : static_cast<uint32_t*>(nullptr),
+             sc.rest_ctr + kRestDense, b.keys == b.alt);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (marks) cudaEventRecord(marks[0], s);
@@ -615,7 +460,7 @@ cudaError_t passes_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStrea
                pl.sort_map, low, uint32_t(C::RADIX - 1), sc.sort_desc, sc.tile_ctr + kCtrSortBase,
                sc.status,
                probe_spins, static_cast<const uint32_t*>(nullptr),
-               static_cast<const uint32_t*>(nullptr));
+               static_cast<const uint32_t*>(nullptr), static_cast<const uint32_t*>(nullptr));
     return cudaGetLastError();
   }
   const K* src = keys;
@@ -629,7 +474,8 @@ cudaError_t passes_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStrea
                  pl.sort_map, shift(p), mask(p),
                  sc.sort_desc + size_t(p) * sc.sort_rows * C::RADIX,
                  sc.tile_ctr + kCtrSortBase + p, sc.status, sc.spin_limit, sc.gate,
-                 static_cast<const uint32_t*>(p == P - 1 ? skew : nullptr));
+                 static_cast<const uint32_t*>(p == P - 1 ? skew : nullptr),
+                 static_cast<const uint32_t*>(rest ? sc.dense : nullptr));
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (marks) cudaEventRecord(marks[1 + p], s);

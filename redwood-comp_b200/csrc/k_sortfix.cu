@@ -5,15 +5,19 @@
 // over the low bits (37 us each at 5,000,011 points) are left out, and every
 // key of a run that shares its top bits finds its place by counting the run's
 // smaller keys (k_sort_fix).  The clouds that this is for have runs of a few
-// keys (uniform) or a few tens (mixtures of sigma 4 and more in a box of 1,024;
-// the densest places, edges of the box that points were clamped to, grow with
-// the cloud to about 130 keys at 2^21 points, hence the line there).  A run
-// beyond kFixRun keys that is not in order sets its cloud's flag, and
-// k_sort_long, launched behind in any case, sorts the flagged clouds by all
-// digits from the unsorted keys.
+// keys (uniform) or a few tens (mixtures of sigma 4 and more in a box of 1,024).
+//
+// Two other kinds of keys go to k_sort_rest, one launch behind, which costs 2 us
+// when there is nothing for it:
+//   - Segments dense everywhere: k_sort_init looks at a sample before the passes,
+//     which then leave a dense segment alone (dense_sample below).  It is
+//     sorted by all eight digits, as many passes as without the low bits left
+//     out, in one launch.
+//   - Runs of more than kFixRun keys among sparse ones: each is sorted by itself,
+//     by the digits left out, by one block.
 #include <algorithm>
 
-#include "block_sort.cuh"
+#include "binning.cuh"
 #include "internal.hpp"
 #include "morton.cuh"
 
@@ -28,24 +32,28 @@ constexpr int kFixWin = kFixTile + 2 * kFixRun;
 // inside the segment, so that every run that touches the tile is in the
 // window, whole.  Also counts the tile's heads (keys with no equal key before
 // them) for stage 3, whose counting pass over the keys it replaces.  Each key
-// is read and written once.  A warp takes 32 keys at a time whose flags "same
-// top bits as the key before" are one ballot, and a group without any (nearly
-// all of them) is stored as it is; the window comes by one bulk copy: 25.4 us
-// at 5,000,011 points (80 MB: 3.2 TB/s), where plain loads took 27.8, looking at
-// both neighbours key by key 33.6 and gathering the sorted tile in a second
-// buffer 26.1.  The last of two waves of tiles is what is left.
+// is read and written once.  A warp takes 32 keys at a time, and a group without
+// any that share their top bits (nearly all of them) is stored as it is; the
+// others find their run's ends in the window's flags ("same top bits as the key
+// before", a bit each).  The window comes by one bulk copy: 25.4 us at 5,000,011
+// points (80 MB: 3.2 TB/s), where plain loads took 27.8 and gathering the sorted
+// tile in a second buffer 26.1.  The last of two waves of tiles is what is left.
+// Where it is dense, a block's time is what counts: 2,000,000 points in a cube of
+// side 24 (runs of 36) took 381 us in all when each key walked its run from
+// neighbour to neighbour, 269 now; with 1 % of them in a cube of side 4 447 and 248.
 template <typename K>
 __global__ void __launch_bounds__(kFixThreads, 6)
     k_sort_fix(const K* __restrict__ in, K* __restrict__ out, uint32_t top, SegTable seg,
-               TileMap map,
-               uint32_t* __restrict__ heads, uint32_t* __restrict__ long_run,
+               TileMap map, uint32_t* __restrict__ heads, const uint32_t* __restrict__ dense,
+               uint2* __restrict__ runs, uint32_t* __restrict__ runs_n, uint32_t runs_cap,
                DevStatus* __restrict__ st) {
   pdl_enter();
   __shared__ __align__(16) K s_raw[kFixWin + 2];
   __shared__ __align__(8) uint64_t s_bar;
-  __shared__ uint32_t s_warp[kFixThreads / 32];
+  __shared__ uint32_t s_warp[kFixThreads / 32], s_flag[kFixWin / 32 + 1];
   uint32_t first;
   const uint32_t c = tile_segment(seg, map, blockIdx.x, &first);
+  if (dense[c]) return;  // the passes have left it to k_sort_rest
   const uint32_t sb = seg_begin(seg, c), se = sb + seg_size(seg, c);
   const uint32_t t0 = sb + (blockIdx.x - first) * uint32_t(kFixTile);
   const uint32_t t1 = min(t0 + uint32_t(kFixTile), se);
@@ -83,176 +91,428 @@ __global__ void __launch_bounds__(kFixThreads, 6)
   auto same = [top](K x, K y) {
     return uint32_t(x >> 32) == uint32_t(y >> 32) && ((uint32_t(x) ^ uint32_t(y)) & top) == 0;
   };
-  bool far = false;
+  // bit i of the flags: key i shares its top bits with the key before it
+  const int lane = int(lane_id()), warp = int(threadIdx.x >> 5);
+  const int groups = (m + 31) / 32;
+  for (int g = warp; g < groups; g += kWarps) {
+    const int i = 32 * g + lane;
+    const uint32_t w = __ballot_sync(0xffffffffu, i > 0 && i < m && same(s[max(i - 1, 0)], s[i]));
+    if (lane == 0) s_flag[g] = w;
+  }
+  if (threadIdx.x == 0) s_flag[groups] = 0;
+  __syncthreads();
+  auto flag = [&](int i) { return i < m && ((s_flag[i >> 5] >> (i & 31)) & 1u); };
+  // a key of the halo matters only if its run reaches into the tile
+  const int g0 = flag(a0) ? 0 : a0 / 32, g1 = flag(a1) ? groups : (a1 + 31) / 32;
+  const uint32_t upto = (2u << lane) - 1u;  // the lanes up to this one
   uint32_t count = 0;
-  // key i, which shares its top bits with a neighbour
-  auto place = [&](int i, K k) {
-    // a key of the halo matters only if its run reaches into the tile
-    if (i < a0 ? !same(s[a0], k) : i >= a1 && !same(s[a1 - 1], k)) return;
-    int at = i, l = i - 1, r = i + 1, less = 0;
+#pragma unroll 2
+  for (int g = g0 + warp; g < g1; g += kWarps) {
+    const uint32_t word = s_flag[g], next = s_flag[g + 1];
+    const int i = 32 * g + lane;
+    const uint32_t either = word | word >> 1 | next << 31;  // same as the key before or after
+    if (i >= m) continue;
+    const K k = s[i];
+    int at = i;
     bool head = true;
-    for (K x; l >= 0 && i - l <= kFixRun && same(x = s[l], k); --l) {
-      less += int(uint32_t(x) <= uint32_t(k));
-      head &= uint32_t(x) != uint32_t(k);
-    }
-    for (K x; r < m && r - i <= kFixRun && same(x = s[r], k); ++r)
-      less += int(uint32_t(x) < uint32_t(k));
-    if (r - l - 1 <= kFixRun) {
-      at = l + 1 + less;
-    } else if (i > 0 && same(s[i - 1], k)) {
-      // every key of a longer run that reaches into the tile sees that it is
-      // longer (257 of its keys are in the window): the run stays as it is,
-      // which is right if it is in order (copies of one key, say)
-      far |= s[i - 1] > k;
-      head = s[i - 1] != k;
+    if ((either >> lane) & 1u) {
+      // the run [l, r), at most nine words of flags to either side
+      int l, r, q = g;
+      uint32_t z = ~word & upto;
+      while (!z && q > g - 9) z = ~s_flag[--q];
+      l = z ? 32 * q + 31 - __clz(z) : 32 * q;
+      z = ~word & ~upto;
+      q = g;
+      while (!z && q < g + 9) z = ~s_flag[++q];
+      r = z ? 32 * q + __ffs(z) - 1 : 32 * q + 32;
+      if (i < a0 ? r <= a0 : i >= a1 && l >= a1) continue;
+      if (r - l > kFixRun) {
+        // every key of a longer run that reaches into the tile sees that it is
+        // longer (257 of its keys are in the window); the tile where it starts
+        // enters it in the list
+        if (l == i && i >= a0 && i < a1) {
+          const uint32_t e = atomicAdd(runs_n, 1u);
+          if (e < runs_cap) runs[e] = make_uint2(lo + uint32_t(i), blockIdx.x);
+        }
+        continue;
+      }
+      // (with the ends known, and the same for all lanes of a run, the loads of the
+      // loop are in flight together)
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(s);  // the lower words
+      const uint32_t kw = uint32_t(k);
+      int less = 0, most = 0;
+#pragma unroll 8
+      for (int j = l; j < r; ++j) {
+        const uint32_t x = w[2 * j];
+        less += int(x < kw);
+        most += int(x <= kw);
+      }
+      if (most - less > 1) {  // copies: in the order in which they stand
+        const int first_copy = less;
+        for (int j = l; j < i; ++j) less += int(w[2 * j] == kw);
+        head = less == first_copy;
+      }
+      at = l + less;
     }
     if (at >= a0 && at < a1) {
       out[lo + uint32_t(at)] = k;
       count += uint32_t(head);
     }
-  };
-  if (full) {
-    static_assert(kFixRun == kFixThreads, "a halo key per thread");
-    const int lane = int(lane_id()), i0 = kFixRun + int(threadIdx.x >> 5) * (kFixTile / kWarps) + lane;
-    constexpr int kGroups = kFixTile / kWarps / 32;
-    K k = s[i0];
-    uint32_t flags = __ballot_sync(0xffffffffu, same(s[i0 - 1], k));
-    K* o = out + lo + uint32_t(i0);
-#pragma unroll 4
-    for (int q = 0; q < kGroups; ++q) {
-      const int i = i0 + 32 * q;
-      const K nk = s[i + 32];
-      const uint32_t nf = __ballot_sync(0xffffffffu, same(s[i + 31], nk));
-      const uint32_t either = flags | flags >> 1 | nf << 31;  // same as the key before or after
-      if (either == 0) {
-        o[32 * q] = k;
-        ++count;
-      } else if ((either >> lane) & 1u) {
-        place(i, k);
-      } else {
-        o[32 * q] = k;
-        ++count;
-      }
-      k = nk;
-      flags = nf;
-    }
-    if (same(s[a0 - 1], s[a0])) place(int(threadIdx.x), s[threadIdx.x]);
-    if (same(s[a1 - 1], s[a1])) place(a1 + int(threadIdx.x), s[a1 + int(threadIdx.x)]);
-  } else {
-    for (int i = int(threadIdx.x); i < m; i += kFixThreads) place(i, s[i]);
   }
   count = warp_sum(count);
   if (lane_id() == 0) s_warp[threadIdx.x >> 5] = count;
-  const bool any = __syncthreads_or(int(far)) != 0;
+  __syncthreads();
   if (threadIdx.x == 0) {
     uint32_t t = 0;
     for (int w = 0; w < kFixThreads / 32; ++w) t += s_warp[w];
     heads[blockIdx.x] = t;
-    if (any) long_run[c] = 1u;
   }
 }
 
-constexpr int kLongThreads = 1024, kLongKpt = 7;
-constexpr int kLongTile = kLongKpt * kSortThreads;
+// Tiles of 4,096 keys; a tile's ranking goes by ballots where its first digit
+// holds a quarter of the segment's keys (in a dense segment the top digits are
+// skewed, which serialises the atomics), and a digit that all keys share is left
+// out.
+constexpr int kRestThreads = 256, kRestKpt = 16, kRestBlocks = 4;
+constexpr int kRestTile = kRestThreads * kRestKpt;
+constexpr int kRestDigits = 8, kRestHistTiles = 4;
+static_assert(kRestTile == int(kUniqueTile) && kRestTile == kFixTile, "stage 3's tiles");
+// zero, histogram, which digits, passes (one more for a copy), heads
+enum : int { kPhaseZero = 0, kPhaseHist = 1, kPhasePlan = 2, kPhasePass = 3,
+             kPhaseHeads = kPhasePass + kRestDigits + 1, kPhases };
+static_assert(kRestWords >= kRestTickets + 2 * kPhases, "counters of the phases");
 
-template <typename K>
-constexpr size_t long_smem() {
-  return 2 * size_t(kLongTile) * sizeof(K) + 2 * size_t(kSortHist) * 4;
-}
-
-struct LongArgs {
+struct RestArgs {
   const void* keys;
   void *tmp, *alt;
   SegTable seg;
-  TileMap map;  // stage 3's tiles
-  uint32_t *heads, *long_run, *mat, *sync;
+  TileMap map;
+  const uint32_t* dense;
+  uint32_t *heads, *desc, *hist, *ctr;
+  uint32_t* digits;  // [segments]: the digits that differ, a bit each
+  const uint2* runs;
+  uint32_t runs_cap, top;
+  int low;
+  uint32_t spin_limit;
   DevStatus* status;
 };
 
-// Sorts the flagged segments by all their digits, keys -> alt, and counts
-// their heads: a cooperative launch of up to one block per SM, each block a
-// share of the segment, two barriers per digit.  It is for correctness, not
-// for speed (about four times the time of the onesweep passes); with no flag
-// set it costs its launch.
+// One run of keys [r0, r1) with equal top bits, out of order in tmp: sorted by the
+// digits of its low bits (stable passes by one block, tmp -> alt -> tmp ..), and
+// its heads added to their tiles'.
 template <typename K>
-__global__ void __launch_bounds__(kLongThreads, 1) k_sort_long(LongArgs a) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  K* sa = reinterpret_cast<K*>(smem);
-  K* sb = sa + kLongTile;
-  uint32_t* hist = reinterpret_cast<uint32_t*>(sb + kLongTile);
-  uint32_t* next = hist + kSortHist;
-  __shared__ DigitShared sd;
-  __shared__ uint32_t s_cnt[256], s_off[256], s_warp[kLongThreads / 32 + 1], s_ok;
+__device__ __forceinline__ void sort_run(const RestArgs& a, unsigned char* smem, uint32_t* s_base,
+                                         uint32_t r0, uint32_t r1, uint32_t sb, uint32_t first) {
+  using C = BinCfg<K, 8, kRestThreads, kRestKpt, kRankMixed>;
   const int tid = int(threadIdx.x);
-  bool mine = false;
-  for (uint32_t c = uint32_t(tid); c < a.seg.count; c += kLongThreads) mine |= a.long_run[c] != 0;
-  if (!__syncthreads_or(int(mine))) return;  // the whole grid: the flags are final
-  const uint32_t P = gridDim.x, b = blockIdx.x;
-  GridBarrier bar{a.sync, P, 0u, &s_ok, a.sync + 1, a.status, nullptr};
-  for (int i = tid; i < 2 * kSortHist / 4; i += kLongThreads)
-    reinterpret_cast<uint4*>(hist)[i] = make_uint4(0, 0, 0, 0);
-  for (uint32_t c = 0; c < a.seg.count; ++c) {
-    if (!a.long_run[c]) continue;
-    const uint32_t s0 = seg_begin(a.seg, c), n = seg_size(a.seg, c);
-    const uint32_t share = (n + P - 1) / P;
-    const uint32_t p0 = min(b * share, n), p1 = min(p0 + share, n);
-    constexpr int kDigits = int(sizeof(K));
-    static_assert(kDigits % 2 == 0, "the last pass ends in alt");
-    for (int q = 0; q < kDigits; ++q) {
-      const K* src = static_cast<const K*>(q == 0 ? a.keys : (q & 1) ? a.tmp : a.alt) + s0;
-      K* dst = static_cast<K*>((q & 1) ? a.alt : a.tmp) + s0;
-      const int shift = 8 * q;
-      if (tid < 256) s_cnt[tid] = 0;
-      __syncthreads();
-      for (uint32_t i = p0 + uint32_t(tid); i < p1; i += kLongThreads)
-        atomicAdd(&s_cnt[uint32_t(src[i] >> shift) & 255u], 1u);
-      __syncthreads();
-      if (tid < 256) a.mat[b * 256 + uint32_t(tid)] = s_cnt[tid];
-      if (!bar.sync()) return;
-      uint32_t tot = 0, prior = 0, all;
-      if (tid < 256)
-        for (uint32_t j = 0; j < P; ++j) {
-          const uint32_t v = a.mat[j * 256 + uint32_t(tid)];
-          prior += j < b ? v : 0u;
-          tot += v;
-        }
-      const uint32_t ex = block_exclusive_scan<kLongThreads>(tot, s_warp, &all);
-      if (tid < 256) s_off[tid] = ex + prior;
-      for (uint32_t t = p0; t < p1; t += kLongTile) {
-        const int cnt = int(min(uint32_t(kLongTile), p1 - t));
-        const int steps = (cnt + kSortThreads - 1) / kSortThreads;
-        for (int i = tid; i < steps * kSortThreads; i += kLongThreads)
-          sa[i] = i < cnt ? src[t + uint32_t(i)] : K(~K(0));
-        __syncthreads();
-        if (tid < kSortThreads)
-          block_digit_pass<K, kLongKpt>(sa, sb, steps, shift, hist, next, sd);
-        uint32_t* h = hist;
-        hist = next;
-        next = h;
-        __syncthreads();
-        for (int i = tid; i < cnt; i += kLongThreads) {
-          const K k = sb[i];
-          const uint32_t g = uint32_t(k >> shift) & 255u;
-          dst[s_off[g] + uint32_t(i) - sd.start[g]] = k;
-        }
-        __syncthreads();
-        // (the filling counts in the last digit: its end is cnt)
-        if (tid < 256) s_off[tid] += (tid < 255 ? sd.start[tid + 1] : uint32_t(cnt)) - sd.start[tid];
+  uint32_t* s_cnt = s_base + 256;
+  uint32_t* s_warp = s_base + 512;
+  K* buf[2] = {static_cast<K*>(a.tmp), static_cast<K*>(a.alt)};
+  const int digits = (a.low + 7) / 8;
+  for (int q = 0; q < digits; ++q) {
+    const K* src = buf[q & 1];
+    K* dst = buf[~q & 1];
+    s_cnt[tid] = 0;
+    __syncthreads();
+    for (uint32_t t = r0 + uint32_t(tid); t < r1; t += 8 * kRestThreads) {
+      uint32_t d[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t i = t + uint32_t(j) * kRestThreads;
+        d[j] = i < r1 ? uint32_t(src[i] >> (8 * q)) & 255u : 256u;
       }
-      if (!bar.sync()) return;
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (d[j] < 256u) atomicAdd(&s_cnt[d[j]], 1u);
     }
-    // stage 3's counts
-    const K* sorted = static_cast<const K*>(a.alt) + s0;
-    const uint32_t f0 = a.map.toff ? a.map.toff[c] : 0u;
-    const uint32_t tiles = (n + uint32_t(kFixTile) - 1) / uint32_t(kFixTile);
-    for (uint32_t t = b; t < tiles; t += P) {
-      uint32_t count = 0, sum;
-      const uint32_t e = min((t + 1) * uint32_t(kFixTile), n);
-      for (uint32_t i = t * uint32_t(kFixTile) + uint32_t(tid); i < e; i += kLongThreads)
-        count += uint32_t(i == 0 || sorted[i] != sorted[i - 1]);
-      block_exclusive_scan<kLongThreads>(count, s_warp, &sum);
-      if (tid == 0) a.heads[f0 + t] = sum;
+    __syncthreads();
+    digit_exclusive_scan<8, kRestThreads>(s_cnt, s_base, s_warp);
+    for (uint32_t t = r0; t < r1; t += uint32_t(kRestTile)) {
+      bin_zero<K, 8, kRestThreads, kRestKpt, kRankMixed>(smem);
+      __syncthreads();
+      bin_tile<K, 8, kRestThreads, kRestKpt, kRankMixed, 8>(
+          smem, src, dst, t, r1, a.seg.total, 8 * q, 255u, false, 0u, [](uint32_t, uint32_t) {},
+          [&](uint32_t d, uint32_t count) {
+            const uint32_t at = s_base[d];
+            s_base[d] = at + count;
+            return r0 + at;
+          });
+      __syncthreads();
     }
+  }
+  const K* src = buf[digits & 1];
+  K* alt = buf[1];
+  // 32 keys at a time that lie in one tile of stage 3
+  const uint32_t g0 = (r0 - sb) & ~31u;
+  for (uint32_t g = g0 + uint32_t(tid); g < ((r1 - sb + 31u) & ~31u); g += kRestThreads) {
+    const uint32_t i = sb + g;
+    bool head = false;
+    if (i >= r0 && i < r1) {
+      const K k = src[i];
+      head = i == r0 || src[i - 1] != k;
+      if (src != alt) alt[i] = k;
+    }
+    const uint32_t m = __ballot_sync(0xffffffffu, head);
+    if (m && lane_id() == 0) atomicAdd(a.heads + first + g / uint32_t(kFixTile), uint32_t(__popc(m)));
+  }
+  __syncthreads();
+  static_assert(C::TILE == kRestTile, "bin_tile's tile");
+}
+
+// What the passes and k_sort_fix have left: the listed runs, then the dense
+// segments' keys -> alt by all digits, with their head counts.
+//
+// The steps of a dense segment (zero, histogram, passes, heads) are phases
+// of jobs that blocks take by ticket; a block that has a job of a phase waits
+// until every job of the phase before is done, and a tile's look-back for the
+// tiles before it.  Both wait only for jobs with earlier tickets, whose blocks are
+// running, so the launch needs no more blocks than happen to run.  Waits are
+// bounded (RW_ERR_TIMEOUT).
+//
+// Whole calls, 64-bit keys in a cube of side 2 (all dense), with eight onesweep
+// passes, with the sorted top bits first and then everything again, and now:
+// 2,000,000 points 310, 1,629 and 295 us, 5,000,011 points 545, 2,332 and 579;
+// 256 clouds of 30,000 points 872 us, 23.8 ms and 808 us.  Four blocks per SM with
+// 64 registers: with three and 80 5,000,011 points took 544 us, but 2,000,000
+// (488 tiles, then more than a wave) 316.
+template <typename K>
+__global__ void __launch_bounds__(kRestThreads, kRestBlocks) k_sort_rest(const RestArgs a) {
+  pdl_enter();
+  const uint32_t listed = min(a.ctr[kRestRuns], a.runs_cap), dense_n = a.ctr[kRestDense];
+  if (listed == 0 && dense_n == 0) return;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ uint32_t s_base[512 + kRestThreads / 32 + 1], s_job, s_end;
+  const int tid = int(threadIdx.x);
+  K* const keys = static_cast<K*>(const_cast<void*>(a.keys));
+  K* const tmp = static_cast<K*>(a.tmp);
+  K* const alt = static_cast<K*>(a.alt);
+
+  for (uint32_t e = blockIdx.x; e < listed; e += gridDim.x) {
+    const uint2 run = a.runs[e];
+    uint32_t first;
+    const uint32_t c = tile_segment(a.seg, a.map, run.y, &first);
+    const uint32_t sb = seg_begin(a.seg, c), se = sb + seg_size(a.seg, c);
+    // the run's end: 256 probes 16 keys apart at a time, then key by key
+    const K k = tmp[run.x];
+    auto same = [&](uint32_t i) {
+      const K x = tmp[i];
+      return uint32_t(x >> 32) == uint32_t(k >> 32) && ((uint32_t(x) ^ uint32_t(k)) & a.top) == 0;
+    };
+    uint32_t from = run.x;
+    for (;; from += 16 * kRestThreads) {
+      const uint32_t i = from + 16 * uint32_t(tid);
+      if (tid == 0) s_end = ~0u;
+      __syncthreads();
+      if (i >= se || !same(i)) atomicMin(&s_end, i);
+      __syncthreads();
+      if (s_end != ~0u) break;
+      __syncthreads();
+    }
+    const uint32_t beyond = s_end;  // not of the run, the key 16 before it is
+    __syncthreads();
+    if (tid == 0) s_end = min(beyond, se);
+    __syncthreads();
+    if (tid < 16) {
+      const uint32_t i = beyond - 16 + uint32_t(tid);
+      if (i >= se || !same(i)) atomicMin(&s_end, i);
+    }
+    __syncthreads();
+    const uint32_t end = s_end;
+    sort_run<K>(a, smem, s_base, run.x, end, sb, first);
+  }
+  if (dense_n == 0) return;
+
+  const uint32_t tiles = a.map.n_tiles;
+  uint32_t* tickets = a.ctr + kRestTickets;
+  uint32_t* done = tickets + kPhases;
+  auto jobs_of = [&](int ph) {
+    return ph == kPhaseHist   ? (tiles + kRestHistTiles - 1) / kRestHistTiles
+           : ph == kPhasePlan ? a.seg.count
+                              : tiles;
+  };
+  // waits until all jobs of a phase are done (block-uniform: false if it gave up)
+  auto wait = [&](int ph) {
+    __syncthreads();  // the last wait's answer has been read
+    if (tid == 0) {
+      s_end = 1u;
+      for (uint32_t spin = 0; ld_acquire(done + ph) != jobs_of(ph);) {
+        if (++spin > a.spin_limit || device_failed(a.status)) {
+          report_error(a.status, RW_ERR_TIMEOUT, kSiteSort);
+          s_end = 0u;
+          break;
+        }
+        backoff(spin);
+      }
+    }
+    __syncthreads();
+    return s_end != 0u;
+  };
+  // passes over a segment in which `digits` of its digits differ: in place an even
+  // number (the last one a copy), so that the first leaves the keys alone
+  auto passes_of = [&](uint32_t digits) {
+    return keys == alt ? (digits + 1u) & ~1u : max(digits, 1u);
+  };
+  auto histogram = [&](uint32_t job) {
+    // digit counts of four tiles, added to their segments'
+    uint32_t* h = reinterpret_cast<uint32_t*>(smem);
+    uint32_t cur = ~0u;
+    auto flush = [&] {
+      __syncthreads();
+      for (int i = tid; i < kRestDigits * 256; i += kRestThreads) {
+        const uint32_t v = h[i];
+        if (v) atomicAdd(a.hist + size_t(cur) * kRestDigits * 256 + uint32_t(i), v);
+      }
+      __syncthreads();
+    };
+    for (uint32_t t = job * kRestHistTiles; t < min((job + 1) * kRestHistTiles, tiles); ++t) {
+      uint32_t first;
+      const uint32_t c = tile_segment(a.seg, a.map, t, &first);
+      if (!a.dense[c]) continue;
+      if (c != cur) {
+        if (cur != ~0u) flush();
+        for (int i = tid; i < kRestDigits * 256; i += kRestThreads) h[i] = 0;
+        __syncthreads();
+        cur = c;
+      }
+      const uint32_t sb = seg_begin(a.seg, c), t0 = sb + (t - first) * uint32_t(kRestTile);
+      const uint32_t t1 = min(t0 + uint32_t(kRestTile), sb + seg_size(a.seg, c));
+      for (uint32_t r = t0 + (uint32_t(tid) & ~31u); r < t1; r += 4 * kRestThreads) {
+        K k[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t i = r + uint32_t(j) * kRestThreads + lane_id();
+          k[j] = i < t1 ? keys[i] : K(0);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t i0 = r + uint32_t(j) * kRestThreads;
+          if (i0 + 32u <= t1) {
+            // the upper digits are often the whole warp's
+            const uint32_t up = uint32_t(k[j] >> 32);
+            const uint32_t diff = __reduce_or_sync(0xffffffffu, up) ^
+                                  __reduce_and_sync(0xffffffffu, up);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              atomicAdd(&h[256 * q + int(uint32_t(k[j] >> (8 * q)) & 255u)], 1u);
+              uint32_t* hu = &h[256 * (q + 4) + int((up >> (8 * q)) & 255u)];
+              if ((diff >> (8 * q)) & 255u) atomicAdd(hu, 1u);
+              else if (lane_id() == 0) atomicAdd(hu, 32u);
+            }
+          } else if (i0 + lane_id() < t1) {
+#pragma unroll
+            for (int q = 0; q < kRestDigits; ++q)
+              atomicAdd(&h[256 * q + int(uint32_t(k[j] >> (8 * q)) & 255u)], 1u);
+          }
+        }
+      }
+    }
+    if (cur != ~0u) flush();
+  };
+  auto pass = [&](uint32_t j, uint32_t job, uint32_t c, uint32_t first, uint32_t sb, uint32_t n) {
+    const uint32_t mask = a.digits[c], digits = uint32_t(__popc(mask)), steps = passes_of(digits);
+    if (j >= steps) return;
+    // the last pass ends in alt
+    const K* src = j == 0 ? keys : ((steps - j) & 1u) ? tmp : alt;
+    K* dst = ((steps - j) & 1u) ? alt : tmp;
+    const uint32_t t0 = sb + (job - first) * uint32_t(kRestTile);
+    // two sets of descriptor rows: a pass clears what the next one uses
+    uint32_t* desc = a.desc + size_t(j & 1u) * tiles * 256;
+    a.desc[(size_t(~j & 1u) * tiles + job) * 256 + uint32_t(tid)] = 0;
+    if (j >= digits) {
+      const uint32_t t1 = min(t0 + uint32_t(kRestTile), sb + n);
+      for (uint32_t i = t0 + uint32_t(tid); i < t1; i += kRestThreads) dst[i] = src[i];
+      return;
+    }
+    uint32_t rest = mask;
+    for (uint32_t q = 0; q < j; ++q) rest &= rest - 1u;
+    const int p = __ffs(rest) - 1;
+    const uint32_t* dh = a.hist + (size_t(c) * kRestDigits + size_t(p)) * 256;
+    const bool ballots = dh[uint32_t(src[t0] >> (8 * p)) & 255u] > n / 4u;
+    const bool head = job == first;
+    if (head) {  // where the segment's digits begin
+      s_base[256 + tid] = dh[tid];
+      __syncthreads();
+      digit_exclusive_scan<8, kRestThreads>(s_base + 256, s_base, s_base + 512);
+    }
+    bin_zero<K, 8, kRestThreads, kRestKpt, kRankMixed>(smem);
+    __syncthreads();
+    uint32_t* drow = desc + size_t(job) * 256;
+    bin_tile<K, 8, kRestThreads, kRestKpt, kRankMixed, 8>(
+        smem, src, dst, t0, sb + n, a.seg.total, 8 * p, 255u, ballots, 0u,
+        [&](uint32_t d, uint32_t count) {
+          if (!head) st_relaxed(drow + d, kFlagAgg | (count << 2));
+        },
+        [&](uint32_t d, uint32_t count) {
+          const uint32_t excl = head ? sb + s_base[d]
+                                     : look_back<256>(desc, d, int(job), int(first), a.spin_limit,
+                                                      a.status);
+          st_relaxed(drow + d, kFlagInc | ((excl + count) << 2));
+          return excl;
+        });
+  };
+  uint32_t passes = 0;
+  for (int ph = 0, before = -1; ph < kPhases; ++ph) {
+    if (ph >= kPhasePass && ph < kPhaseHeads && uint32_t(ph - kPhasePass) >= passes) continue;
+    const uint32_t jobs = jobs_of(ph);
+    bool waited = before < 0;
+    for (;;) {
+      __syncthreads();  // the last job is finished with the shared memory
+      if (tid == 0) s_job = atomicAdd(tickets + ph, 1u);
+      __syncthreads();
+      const uint32_t job = s_job;
+      if (job >= jobs) break;
+      if (!waited && !wait(before)) return;
+      waited = true;
+      if (ph == kPhaseHist) {
+        histogram(job);
+      } else if (ph == kPhasePlan) {
+        const uint32_t n = seg_size(a.seg, job);
+        if (a.dense[job]) {
+          uint32_t mask = 0;
+#pragma unroll
+          for (int q = 0; q < kRestDigits; ++q) {
+            const uint32_t v = a.hist[(size_t(job) * kRestDigits + size_t(q)) * 256 + size_t(tid)];
+            mask |= uint32_t(!__syncthreads_or(v == n)) << q;
+          }
+          if (tid == 0) {
+            a.digits[job] = mask;
+            atomicMax(a.ctr + kRestPasses, passes_of(uint32_t(__popc(mask))));
+          }
+        }
+      } else {
+        uint32_t first;
+        const uint32_t c = tile_segment(a.seg, a.map, job, &first);
+        if (a.dense[c]) {
+          const uint32_t sb = seg_begin(a.seg, c), n = seg_size(a.seg, c);
+          if (ph == kPhaseZero) {
+            a.desc[size_t(job) * 256 + size_t(tid)] = 0;
+            a.desc[(size_t(tiles) + job) * 256 + size_t(tid)] = 0;
+            if (job == first)
+              for (int i = tid; i < kRestDigits * 256; i += kRestThreads)
+                a.hist[size_t(c) * kRestDigits * 256 + size_t(i)] = 0;
+          } else if (ph == kPhaseHeads) {
+            const uint32_t t0 = sb + (job - first) * uint32_t(kRestTile);
+            const uint32_t t1 = min(t0 + uint32_t(kRestTile), sb + n);
+            uint32_t count = 0, sum;
+            for (uint32_t i = t0 + uint32_t(tid); i < t1; i += kRestThreads)
+              count += uint32_t(i == sb || alt[i] != alt[i - 1]);
+            block_exclusive_scan<kRestThreads>(count, s_base, &sum);
+            if (tid == 0) a.heads[job] = sum;
+          } else {
+            pass(uint32_t(ph - kPhasePass), job, c, first, sb, n);
+          }
+        }
+      }
+      __syncthreads();
+      if (tid == 0)
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(done + ph) : "memory");
+    }
+    if (ph == kPhasePlan) {  // the most passes of any segment
+      if (!waited && !wait(before)) return;
+      if (!wait(ph)) return;
+      passes = ld_relaxed(a.ctr + kRestPasses);
+    }
+    before = ph;
   }
 }
 
@@ -260,38 +520,40 @@ namespace {
 
 template <typename K>
 cudaError_t fix_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_t s) {
+  constexpr size_t smem = BinCfg<K, 8, kRestThreads, kRestKpt, kRankMixed>::kSmem;
   // six blocks need nearly all of the SM's shared memory
   cudaError_t e = cudaFuncSetAttribute(k_sort_fix<K>,
                                        cudaFuncAttributePreferredSharedMemoryCarveout,
                                        int(cudaSharedmemCarveoutMaxShared));
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_sort_long<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             int(long_smem<K>()));
+    e = cudaFuncSetAttribute(k_sort_rest<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             int(smem));
   if (e != cudaSuccess) return e;
-  if (!pl.unique_map.n_tiles) return cudaSuccess;
+  const uint32_t tiles = pl.unique_map.n_tiles;
+  if (!tiles) return cudaSuccess;
+  // two sets of rows in the descriptors of the passes, which are done
+  if (2ull * tiles > uint64_t(sc.passes) * sc.sort_rows) return cudaErrorInvalidValue;
   const int low = sorted_low_bits(sc);  // at most 32
   const uint32_t top = low < 32 ? ~0u << low : 0u;
-  launch_pdl(k_sort_fix<K>, pl.unique_map.n_tiles, kFixThreads, 0, s,
-             static_cast<const K*>(b.tmp), static_cast<K*>(b.alt), top, pl.seg, pl.unique_map,
-             sc.unique_desc, sc.long_run, sc.status);
-  LongArgs a{b.keys, b.tmp, b.alt, pl.seg, pl.unique_map, sc.unique_desc, sc.long_run,
-             sc.sort_desc, sc.tile_ctr + kCtrLong, sc.status};
-  // the passes' descriptors are free by now: a row of digit counts per block
-  const uint64_t rows = uint64_t(sc.passes) * sc.sort_rows;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = uint32_t(std::min<uint64_t>(rows, uint64_t(sc.num_sms)));
-  cfg.blockDim = kLongThreads;
-  cfg.dynamicSmemBytes = long_smem<K>();
-  cfg.stream = s;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_sort_long<K>, a);
+  uint2* runs = reinterpret_cast<uint2*>(sc.rest + size_t(pl.seg.count) * kRestDigits * 256);
+  const uint32_t cap = rest_runs(pl.seg.total);
+  uint32_t* digits = reinterpret_cast<uint32_t*>(runs + cap);
+  launch_pdl(k_sort_fix<K>, tiles, kFixThreads, 0, s, static_cast<const K*>(b.tmp),
+             static_cast<K*>(b.alt), top, pl.seg, pl.unique_map, sc.unique_desc,
+             static_cast<const uint32_t*>(sc.dense), runs, sc.rest_ctr + kRestRuns, cap,
+             sc.status);
+  RestArgs a{b.keys,   b.tmp,       b.alt,   pl.seg, pl.unique_map, sc.dense, sc.unique_desc,
+             sc.sort_desc, sc.rest, sc.rest_ctr, digits, runs, cap, top, low, sc.spin_limit, sc.status};
+  launch_pdl(k_sort_rest<K>, std::min(tiles, uint32_t(sc.num_sms) * kRestBlocks), kRestThreads,
+             smem, s, a);
+  return cudaGetLastError();
 }
 
 }  // namespace
+
+size_t rest_words(uint32_t segments, uint32_t n) {
+  return size_t(segments) * (kRestDigits * 256 + 1) + 2 * size_t(rest_runs(n));
+}
 
 cudaError_t launch_sort_finish(const Bufs& b, const Scratch& sc, const Plan& pl,
                                cudaStream_t s) {
