@@ -348,6 +348,15 @@ int rw_tree_sort_profile(rw_tree_app_data* app, rw_tree_im_storage* im, rw_strea
  * next normal run. */
 int rw_tree_sort_lookback_probe(rw_tree_app_data* app, rw_tree_im_storage* im,
                                 uint32_t spin_limit, rw_stream_t stream);
+/* The same for two other bounded waits, which give up after spin_limit polls for
+ * something that never comes: RW_WAIT_GRID, the barriers of a small cloud's one
+ * launch (a cloud of several blocks: 4,097 points or more), RW_WAIT_JOBS, the
+ * steps of the 64-bit sort of dense keys (u_morton_keys, sorted in place).  Returns
+ * RW_ERR_TIMEOUT, and the scratch is fit for the next normal run. */
+#define RW_WAIT_GRID 0
+#define RW_WAIT_JOBS 1
+int rw_tree_wait_probe(rw_tree_app_data* app, rw_tree_im_storage* im, int32_t which,
+                       uint32_t spin_limit, rw_stream_t stream);
 
 /* ---- learned-CDF bucketed sort (32-bit keys) -------------------------------
  * No reference counterpart.  A 64K-key stratified sample is sorted and 4,095

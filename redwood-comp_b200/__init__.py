@@ -104,7 +104,8 @@ EXPORTS = (
     "rw_tree_batch_total_points", "rw_tree_batch_octree_rows", "rw_tree_batch_offsets",
     "rw_tree_batch_set_sort_variant", "rw_tree_batch_enqueue", "rw_tree_batch_graph_launch",
     "rw_tree_batch_finish", "rw_tree_batch_set_classes", "rw_tree_sort_enqueue",
-    "rw_tree_sort_profile", "rw_tree_sort_lookback_probe", "rw_tree_im_storage_set_options",
+    "rw_tree_sort_profile", "rw_tree_sort_lookback_probe", "rw_tree_wait_probe",
+    "rw_tree_im_storage_set_options",
     "rw_tree_batch_set_learned",
     "rw_tree_learned_create", "rw_tree_learned_destroy", "rw_tree_learned_set_params",
     "rw_tree_learned_set_group", "rw_tree_im_storage_set_learned",
@@ -376,6 +377,17 @@ def sort_lookback_probe(app: AppData, im: ImStorage, spin_limit: int, stream=Non
     return int(lib().rw_tree_sort_lookback_probe(ctypes.byref(app.c), im.handle,
                                                  ctypes.c_uint32(spin_limit),
                                                  _stream_handle(stream)))
+
+
+WAIT_GRID, WAIT_JOBS = 0, 1
+
+
+def wait_probe(app: AppData, im: ImStorage, which: int, spin_limit: int, stream=None) -> int:
+    """Makes another bounded wait run out (rw_tree_wait_probe): WAIT_GRID, the
+    barriers of a small cloud's one launch; WAIT_JOBS, the steps of the 64-bit sort
+    of dense keys.  Returns the rw_status code (RW_ERR_TIMEOUT)."""
+    return int(lib().rw_tree_wait_probe(ctypes.byref(app.c), im.handle, ctypes.c_int32(which),
+                                        ctypes.c_uint32(spin_limit), _stream_handle(stream)))
 
 
 def profile_sort(keys, out, im: ImStorage, reps: int = 5, stream=None) -> dict:

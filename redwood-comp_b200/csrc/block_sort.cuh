@@ -9,11 +9,14 @@ namespace rwt {
 
 // Barrier over the grid's blocks, which all run (cooperative launch): arrivals
 // only ever grow, the host never resets them between launches.  Bounded: a
-// block whose wait runs out reports RW_ERR_TIMEOUT, marks the scratch (until
-// it is cleared) and leaves.
+// block whose wait runs out takes kGaveUp off the arrivals, unless the last one
+// has come by then, reports RW_ERR_TIMEOUT, marks the scratch (until it is cleared)
+// and leaves.  Either every block passes a barrier or, from that moment, none
+// does: no block can go on and report success for work that another has left.
 struct GridBarrier {
+  static constexpr uint32_t kGaveUp = 0x40000000u;  // far more than arrivals
   uint32_t* word;
-  uint32_t blocks, target;
+  uint32_t blocks, target, limit;
   uint32_t* s_ok;       // shared: whether the last wait ended in time
   uint32_t* gave_up;    // set when one did not
   DevStatus* status;    // gets the error
@@ -24,10 +27,17 @@ struct GridBarrier {
     target += blocks;
     if (threadIdx.x == 0) {
       asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(word) : "memory");
-      uint32_t spin = 0;
-      while (int32_t(ld_acquire(word) - target) < 0 && ++spin < kSpinLimit) backoff(spin);
-      *s_ok = spin < kSpinLimit;
-      if (spin >= kSpinLimit) {
+      bool ok = false;
+      for (uint32_t spin = 0;;) {
+        const uint32_t v = ld_acquire(word);
+        const int32_t past = int32_t(v - target);
+        ok = past >= 0;
+        if (ok || past < -int32_t(kGaveUp / 2)) break;
+        if (++spin < limit) backoff(spin);
+        else if (atomicCAS(word, v, v - kGaveUp) == v) break;  // else look again
+      }
+      *s_ok = ok;
+      if (!ok) {
         st_relaxed(gave_up, 1u);
         report_error(status, RW_ERR_TIMEOUT, kSiteGrid);
         if (host_status) *reinterpret_cast<volatile int32_t*>(&host_status->err) = RW_ERR_TIMEOUT;

@@ -133,6 +133,14 @@ int clear_all(rw_tree_im_storage* im, cudaStream_t s) {
   return RW_OK;
 }
 
+// The one-launch pipeline takes a small cloud unless the caller chose how
+// stage 2 sorts (a learned sort, another digit width or another variant).
+bool takes_small(const rw_tree_app_data* app, const rw_tree_im_storage* im) {
+  return im->d_small && !im->learned &&
+         im->sort_variant == rwt::default_sort_variant(im->key_bits, im->radix_bits) &&
+         rwt::small_takes(app->n_input, im->key_bits, im->num_sms);
+}
+
 // Waits for the stream, copies the device status and maps its error word.
 int sync_status(rw_tree_im_storage* im, cudaStream_t s) {
   RW_CUDA(rwt::launch_status_out(im->d_status, im->h_status, s));
@@ -428,6 +436,35 @@ int rw_tree_sort_lookback_probe(rw_tree_app_data* app, rw_tree_im_storage* im,
   return sync_status(im, s);
 }
 
+int rw_tree_wait_probe(rw_tree_app_data* app, rw_tree_im_storage* im, int32_t which,
+                       uint32_t spin_limit, rw_stream_t stream) {
+  if (!app || !im || spin_limit == 0) return RW_ERR_ARG;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  auto sc = scratch_of(im);
+  sc.spin_limit = spin_limit;
+  sc.missing = 1;
+  if (which == RW_WAIT_GRID) {
+    if (int rc = check(app, im, kPoints | kKeys | kAlt | kBrt | kEdge | kOct)) return rc;
+    if (!takes_small(app, im) || app->n_input <= rwt::small_alone()) return RW_ERR_ARG;
+    RW_CUDA(rwt::launch_small(bufs_of(*app, im), sc, app->n_input, im->n_cap, app->oct_capacity,
+                              false, false, im->d_small, im->d_tile_ctr + rwt::kCtrSmall,
+                              im->h_status, s));
+    return rw_tree_pipeline_finish(app, im, stream);
+  }
+  if (which != RW_WAIT_JOBS || !im->low_bits) return RW_ERR_ARG;
+  if (int rc = check(app, im, kKeys)) return rc;
+  if (int rc = clear_all(im, s)) return rc;
+  auto b = bufs_of(*app, im);
+  b.alt = b.keys;  // sorted by k_sort_rest
+  const auto pl = plan_of(*app, im);
+  RW_CUDA(rwt::launch_keys(b, sc, pl, false, true, s));
+  RW_CUDA(rwt::launch_sort_passes(b, sc, pl, s));
+  RW_CUDA(rwt::launch_sort_finish(b, sc, pl, s));
+  const int rc = sync_status(im, s);
+  if (int rc2 = clear_all(im, s)) return rc2;
+  return rc;
+}
+
 // ---- stage 3: unique (cu_dispatcher.cu:597-627) -------------------------------
 int rw_tree_run_stage3(rw_tree_app_data* app, rw_tree_im_storage* im,
                        rw_stream_t stream) {
@@ -498,14 +535,6 @@ int rw_tree_run_stage7(rw_tree_app_data* app, rw_tree_im_storage* im,
 
 // ---- fused pipeline ----------------------------------------------------------
 namespace {
-
-// The one-launch pipeline takes a small cloud unless the caller chose how
-// stage 2 sorts (a learned sort, another digit width or another variant).
-bool takes_small(const rw_tree_app_data* app, const rw_tree_im_storage* im) {
-  return im->d_small && !im->learned &&
-         im->sort_variant == rwt::default_sort_variant(im->key_bits, im->radix_bits) &&
-         rwt::small_takes(app->n_input, im->key_bits, im->num_sms);
-}
 
 // Enqueues the fused pipeline.  When `ev` is given, an event is recorded
 // before the first launch and after every kernel launch (profiling only; it

@@ -162,6 +162,9 @@ struct Scratch {
   DevStatus* status = nullptr;
   // polls of a look-back wait before it gives up with RW_ERR_TIMEOUT
   uint32_t spin_limit = kSpinLimit;
+  // arrivals or jobs that the bounded waits of k_small and k_sort_rest wait for in
+  // vain (rw_tree_wait_probe)
+  uint32_t missing = 0;
   // when set, the sort's kernels (digit histograms, set-up, passes) do their
   // work only if *gate != 0, read on the device: a fallback sort enqueued
   // ahead of the decision that needs it
@@ -281,6 +284,7 @@ constexpr uint32_t kSmallLimit32 = 1100000, kSmallLimit64 = 550000;
 // Sets the kernels up on the current device; *usable: a block of them fits an SM.
 cudaError_t small_prepare(int key_bits, bool* usable);
 uint32_t small_limit(int key_bits);
+uint32_t small_alone();  // points of the largest cloud that one block takes
 bool small_takes(uint32_t n, int key_bits, int sms);
 size_t small_scratch_bytes(uint32_t n_cap, int key_bits, int sms);
 // All seven stages for n points: `scratch` of small_scratch_bytes(n_cap),

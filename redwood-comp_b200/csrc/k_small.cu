@@ -66,6 +66,7 @@ struct SmallArgs {
   bool leaves;
   // scratch
   uint32_t* sync;  // [0] arrivals, [1] arrivals before this launch, [2] a wait gave up
+  uint32_t spin_limit, missing;  // of the barriers: polls; arrivals that never come
   void *samples, *splitters, *first, *last, *region, *tmp;
   uint32_t *fill, *counts, *heads, *mat, *sums;
   uint32_t *far, *far_n, far_cap;
@@ -165,7 +166,8 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
   uint32_t* next = hist + kSortHist;
   const int tid = int(threadIdx.x), lane = tid & 31, warp = tid >> 5;
   const uint32_t P = gridDim.x, b = blockIdx.x;
-  GridBarrier bar{a.sync, P, ld_relaxed(a.sync + 1), &sh.ok, a.sync + 2, a.status, a.host_status};
+  GridBarrier bar{a.sync, P + a.missing, ld_relaxed(a.sync + 1), a.spin_limit,
+                  &sh.ok, a.sync + 2, a.status, a.host_status};
   if (ld_relaxed(a.sync + 2)) {  // an earlier wait gave up and nothing cleared the scratch since
     if (b == 0 && tid == 0)
       *reinterpret_cast<volatile int32_t*>(&a.host_status->err) = RW_ERR_TIMEOUT;
@@ -587,6 +589,8 @@ cudaError_t small_ready(int* per_sm) {
 
 }  // namespace
 
+uint32_t small_alone() { return kSmAlone; }
+
 uint32_t small_limit(int key_bits) { return key_bits == 32 ? kSmallLimit32 : kSmallLimit64; }
 
 bool small_takes(uint32_t n, int key_bits, int sms) {
@@ -677,6 +681,9 @@ cudaError_t launch_small(const Bufs& b, const Scratch& sc, uint32_t n, uint32_t 
   a.far_n = sc.tile_ctr + kCtrLinks;
   a.status = sc.status;
   a.host_status = host_status;
+  a.spin_limit = sc.spin_limit;
+  a.missing = sc.missing;
+  if (a.missing && blocks == 1) return cudaErrorInvalidValue;  // nothing waits
   if (b.key_bits == 64) return small_t<uint64_t, 0>(b, a, blocks, s);
   return geometric ? small_t<uint32_t, 1>(b, a, blocks, s) : small_t<uint32_t, 0>(b, a, blocks, s);
 }

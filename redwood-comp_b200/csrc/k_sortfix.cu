@@ -193,7 +193,7 @@ struct RestArgs {
   const uint2* runs;
   uint32_t runs_cap, top;
   int low;
-  uint32_t spin_limit;
+  uint32_t spin_limit, missing;
   DevStatus* status;
 };
 
@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(kRestThreads, kRestBlocks) k_sort_rest(const R
     __syncthreads();  // the last wait's answer has been read
     if (tid == 0) {
       s_end = 1u;
-      for (uint32_t spin = 0; ld_acquire(done + ph) != jobs_of(ph);) {
+      for (uint32_t spin = 0; ld_acquire(done + ph) != jobs_of(ph) + a.missing;) {
         if (++spin > a.spin_limit || device_failed(a.status)) {
           report_error(a.status, RW_ERR_TIMEOUT, kSiteSort);
           s_end = 0u;
@@ -543,7 +543,8 @@ cudaError_t fix_t(const Bufs& b, const Scratch& sc, const Plan& pl, cudaStream_t
              static_cast<const uint32_t*>(sc.dense), runs, sc.rest_ctr + kRestRuns, cap,
              sc.status);
   RestArgs a{b.keys,   b.tmp,       b.alt,   pl.seg, pl.unique_map, sc.dense, sc.unique_desc,
-             sc.sort_desc, sc.rest, sc.rest_ctr, digits, runs, cap, top, low, sc.spin_limit, sc.status};
+             sc.sort_desc, sc.rest, sc.rest_ctr, digits, runs, cap, top, low, sc.spin_limit,
+             sc.missing, sc.status};
   launch_pdl(k_sort_rest<K>, std::min(tiles, uint32_t(sc.num_sms) * kRestBlocks), kRestThreads,
              smem, s, a);
   return cudaGetLastError();
