@@ -543,11 +543,16 @@ int enqueue_impl(rw_tree_app_data* app, rw_tree_im_storage* im, cudaStream_t s,
                  cudaEvent_t* ev, int* n_ev) {
   if (int rc = check(app, im, kPoints | kKeys | kAlt | kBrt | kEdge | kOct)) return rc;
   if (!ev && takes_small(app, im)) {
-    RW_CUDA(rwt::launch_small(bufs_of(*app, im), scratch_of(im), app->n_input, im->n_cap,
-                              app->oct_capacity, geometric_delta(im),
-                              (im->options & RW_TREE_OPT_LINK_LEAVES) != 0, im->d_small,
-                              im->d_tile_ctr + rwt::kCtrSmall, im->h_status, s));
-    return RW_OK;
+    const cudaError_t e = rwt::launch_small(
+        bufs_of(*app, im), scratch_of(im), app->n_input, im->n_cap, app->oct_capacity,
+        geometric_delta(im), (im->options & RW_TREE_OPT_LINK_LEAVES) != 0, im->d_small,
+        im->d_tile_ctr + rwt::kCtrSmall, im->h_status, s);
+    if (e == cudaSuccess) return RW_OK;
+    // a stream whose context owns a part of the chip cannot hold all blocks at once:
+    // the chain of kernels below does not need that
+    if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported)
+      return cuda_fail(e, "launch_small");
+    cudaGetLastError();
   }
   int k = 0;
   auto mark = [&]() -> cudaError_t {
