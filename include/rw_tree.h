@@ -184,11 +184,23 @@ int rw_tree_pipeline_enqueue(rw_tree_app_data* app, rw_tree_im_storage* im,
 int rw_tree_pipeline_finish(rw_tree_app_data* app, rw_tree_im_storage* im,
                             rw_stream_t stream);
 
+/* 1 if a run of `app` on `im` is one kernel launch: a small cloud (up to 1,100,000
+ * points, 550,000 with 64-bit keys, as far as the chip has room), unless the caller
+ * chose how stage 2 sorts.  (Where that launch is refused, in a context that owns a
+ * part of the chip, the run takes the general chain of kernels.) */
+int rw_tree_pipeline_one_launch(const rw_tree_app_data* app, const rw_tree_im_storage* im);
+/* How many such runs, since the scratch was last cleared, had to sort digit by digit,
+ * because their samples had missed most of the keys.  Waits for `stream`. */
+int rw_tree_im_storage_digit_sorts(rw_tree_im_storage* im, rw_stream_t stream, uint32_t* out);
+
 /* Per-kernel device times of the fused pipeline, the role of the reference's
  * per-stage google-benchmark fixtures (apps/tree/bm_cuda.cpp:25-123): runs
  * the pipeline `reps` times with a CUDA event after every kernel and writes
  * the mean milliseconds of each kernel to kernel_ms (order and names as in
- * rw_tree_pipeline_kernel_names, comma separated). */
+ * rw_tree_pipeline_kernel_names, comma separated).  It always runs the general
+ * chain of kernels, also for a cloud whose runs are one launch
+ * (rw_tree_pipeline_one_launch).  The time of what follows the last pass of a
+ * 64-bit sort counts to that pass. */
 int rw_tree_pipeline_profile(rw_tree_app_data* app, rw_tree_im_storage* im,
                              rw_stream_t stream, int32_t reps, float* kernel_ms,
                              int32_t max_kernels, int32_t* n_kernels);

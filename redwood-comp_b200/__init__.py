@@ -105,6 +105,7 @@ EXPORTS = (
     "rw_tree_batch_set_sort_variant", "rw_tree_batch_enqueue", "rw_tree_batch_graph_launch",
     "rw_tree_batch_finish", "rw_tree_batch_set_classes", "rw_tree_sort_enqueue",
     "rw_tree_sort_profile", "rw_tree_sort_lookback_probe", "rw_tree_wait_probe",
+    "rw_tree_pipeline_one_launch", "rw_tree_im_storage_digit_sorts",
     "rw_tree_im_storage_set_options",
     "rw_tree_batch_set_learned",
     "rw_tree_learned_create", "rw_tree_learned_destroy", "rw_tree_learned_set_params",
@@ -216,6 +217,14 @@ class ImStorage:
         _check(lib().rw_tree_im_storage_learned_stats(self._h, ctypes.byref(st)), "learned_stats")
         return {"max_bucket": st.max_bucket, "big_buckets": st.big_buckets,
                 "fell_back": st.fell_back, "mlp_timeout": st.mlp_timeout}
+
+    def digit_sorts(self, stream=None) -> int:
+        """One-launch runs since the last clear that sorted digit by digit
+        (rw_tree_im_storage_digit_sorts)."""
+        n = ctypes.c_uint32()
+        _check(lib().rw_tree_im_storage_digit_sorts(self._h, _stream_handle(stream),
+                                                    ctypes.byref(n)), "digit_sorts")
+        return n.value
 
     def clear(self, stream=None) -> None:
         _check(lib().rw_tree_im_storage_clear(self._h, _stream_handle(stream)), "clearSmem")
@@ -421,8 +430,14 @@ def run_pipeline(app: AppData, im: ImStorage, stream=None) -> None:
     pipeline_finish(app, im, stream)
 
 
+def one_launch(app: AppData, im: ImStorage) -> bool:
+    """Whether a run of `app` on `im` is one kernel launch (rw_tree_pipeline_one_launch)."""
+    return bool(lib().rw_tree_pipeline_one_launch(ctypes.byref(app.c), im.handle))
+
+
 def profile_pipeline(app: AppData, im: ImStorage, reps: int = 5, stream=None) -> dict:
-    """Mean device milliseconds of every kernel of the fused pipeline."""
+    """Mean device milliseconds of every kernel of the fused pipeline's general
+    chain (which a cloud that takes one launch does not run)."""
     ms = (ctypes.c_float * 64)()
     nk = ctypes.c_int32()
     _check(lib().rw_tree_pipeline_profile(ctypes.byref(app.c), im.handle,

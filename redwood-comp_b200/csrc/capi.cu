@@ -605,6 +605,19 @@ int rw_tree_pipeline_enqueue(rw_tree_app_data* app, rw_tree_im_storage* im,
   return enqueue_impl(app, im, reinterpret_cast<cudaStream_t>(stream), nullptr, nullptr);
 }
 
+int rw_tree_pipeline_one_launch(const rw_tree_app_data* app, const rw_tree_im_storage* im) {
+  return app && im && app->key_bits == im->key_bits && app->n_input >= 1 &&
+         app->n_input <= im->n_cap && takes_small(app, im);
+}
+
+int rw_tree_im_storage_digit_sorts(rw_tree_im_storage* im, rw_stream_t stream, uint32_t* out) {
+  if (!im || !out) return RW_ERR_ARG;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  RW_CUDA(cudaMemcpyAsync(out, im->d_tile_ctr + rwt::kCtrSmall + 3, 4, cudaMemcpyDeviceToHost, s));
+  RW_CUDA(cudaStreamSynchronize(s));
+  return RW_OK;
+}
+
 const char* rw_tree_pipeline_kernel_names(const rw_tree_im_storage* im) {
   static thread_local std::string names;
   if (im && im->learned) {

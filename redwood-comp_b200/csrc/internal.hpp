@@ -288,7 +288,7 @@ uint32_t small_alone();  // points of the largest cloud that one block takes
 bool small_takes(uint32_t n, int key_bits, int sms);
 size_t small_scratch_bytes(uint32_t n_cap, int key_bits, int sms);
 // All seven stages for n points: `scratch` of small_scratch_bytes(n_cap),
-// `sync` three zeroed words that only these launches and a clear change.  The
+// `sync` four zeroed words that only these launches and a clear change.  The
 // counts and the first error go to sc.status and, at the end, to host_status
 // (pinned).
 cudaError_t launch_small(const Bufs& b, const Scratch& sc, uint32_t n, uint32_t n_cap,

@@ -65,7 +65,9 @@ struct SmallArgs {
   OctOut o;
   bool leaves;
   // scratch
-  uint32_t* sync;  // [0] arrivals, [1] arrivals before this launch, [2] a wait gave up
+  // [0] arrivals, [1] arrivals before this launch, [2] a wait gave up, [3] launches
+  // that sorted digit by digit
+  uint32_t* sync;
   uint32_t spin_limit, missing;  // of the barriers: polls; arrivals that never come
   void *samples, *splitters, *first, *last, *region, *tmp;
   uint32_t *fill, *counts, *heads, *mat, *sums;
@@ -349,6 +351,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_small(SmallArgs a) {
       // digit by digit over the grid: every block ranks its share, the counts
       // of all blocks give its keys' places
       K* tmp = static_cast<K*>(a.tmp);
+      if (b == 0 && tid == 0) ++a.sync[3];
       for (int shift = 0; shift < KeyTraits<K>::kCodeBits; shift += 8) {
         const int steps = (c + kSortThreads - 1) / kSortThreads;
         for (int i = c + tid; i < steps * kSortThreads; i += kSmThreads) sa[i] = K(~K(0));
