@@ -105,12 +105,12 @@ def sort_passes(a):
     return -(-bits // (a.radix_bits or 8))
 
 
-def launches_per_step(a):
-    """Kernels of one fused pipeline step: one for a small cloud; else keys, sort set-up,
-    the passes, unique (3), radix tree, scan of the tile sums, octree (2) and the counts'
-    way to the host.  64-bit keys with 8-bit digits end the sort with two kernels more,
-    which count the unique keys' heads."""
-    if a.n <= (1_100_000 if a.key_bits == 32 else 550_000):
+def launches_per_step(a, one_launch):
+    """Kernels of one fused pipeline step: one for a cloud that takes one launch; else
+    keys, sort set-up, the passes, unique (3), radix tree, scan of the tile sums, octree
+    (2) and the counts' way to the host.  64-bit keys with 8-bit digits end the sort with
+    two kernels more, which count the unique keys' heads."""
+    if one_launch:
         return 1
     finish = a.key_bits == 64 and (a.radix_bits or 8) == 8
     return 10 + sort_passes(a) + (1 if finish else 0)
@@ -294,13 +294,13 @@ def kernel_bytes(name, n, u, m, K):
 
 
 def pipeline_bytes(n, u, m, K, passes):
-    """Whole-pipeline algorithmic bytes (per-stage formulas: S1 (16+K)n,
-    S2 K n (1+2P), S3 K(n+u), S4 K u + 11 b, S5 10 b, S6 4 b,
-    S7 (13+K) b + 60 m; stage 6's sums are made inside stage 4, its offsets inside
-    stage 7; the sweep that ends a 64-bit sort is not counted)."""
+    """Whole-pipeline algorithmic bytes of the fused form: stage 1 (16+K) n (the digit
+    counts are made there), the passes 2 P K n, stage 3 K (n+u), stages 4 and 5 K u + 15 b,
+    the tiles' sums 8 bytes per 1,024 nodes, stage 7 (with stage 6's offsets) (13+K) b +
+    60 m.  The sweep that ends a 64-bit sort is not counted."""
     b = u - 1
-    return ((16 + K) * n + K * n * (1 + 2 * passes) + K * (n + u) + K * u + 11 * b
-            + 10 * b + 4 * b + (13 + K) * b + 60 * m)
+    return ((16 + K) * n + 2 * passes * K * n + K * (n + u) + K * u + 15 * b
+            + 8 * -(-b // 1024) + (13 + K) * b + 60 * m)
 
 
 def traffic_table():
@@ -951,8 +951,13 @@ def main():
     roofline = {"bound": "hbm", "kernel": dom, "achieved": dom_gbs, "peak": hbm,
                 "unit": "GB/s", "frac": round(dom_gbs / hbm, 4) if dom_gbs else None,
                 "traffic": dom_traffic, "peak_source": f"{peak_kind} hbm_gbs"}
-    pipe_b = pipeline_bytes(a.n, u, m, K, passes)
+    one_launch = rw.one_launch(app, im)
+    # (a cloud that takes one launch is sorted by one exchange of its keys)
+    pipe_b = pipeline_bytes(a.n, u, m, K, 1 if one_launch else passes)
     pipe_gbs = pipe_b / (ms_step * 1e-3) / 1e9
+    if one_launch:  # the step's one kernel; `stages` has those of the general chain
+        roofline.update({"kernel": "pipeline in one launch", "achieved": round(pipe_gbs, 1),
+                         "frac": round(pipe_gbs / hbm, 4), "traffic": None})
 
     # ---- end to end through the host-facing C ABI call ---------------------
     h_pts = torch.from_numpy(pts).pin_memory()
@@ -1072,9 +1077,12 @@ def main():
         "one_stream": one_stream,
         "pipeline_roofline": {"bytes_per_step": pipe_b, "achieved_gbs": round(pipe_gbs, 1),
                               "frac": round(pipe_gbs / hbm, 4)},
-        "roofline": roofline, "stages": stages, "e2e": e2e, "cpu_baseline": cpu,
+        "roofline": roofline, "stages": stages,
+        "stages_of": "general chain of kernels, which the timed steps do not launch"
+                     if one_launch else "timed steps",
+        "e2e": e2e, "cpu_baseline": cpu,
         "reference_cuda": ref_cuda,
-        "clocks": clocks.summary(), "gpu_launches": launches_per_step(a) * a.steps,
+        "clocks": clocks.summary(), "gpu_launches": launches_per_step(a, one_launch) * a.steps,
         "forms": forms,
     }
     print(json.dumps(line), flush=True)
