@@ -566,7 +566,7 @@ int enqueue_impl(rw_tree_app_data* app, rw_tree_im_storage* im, cudaStream_t s,
   RW_CUDA(mark());
   if (im->learned) {
     // stage 1 without the digit histograms, then the learned-CDF sort (which
-    // waits for its bucket plan once, and falls back to onesweep on `im`)
+    // falls back to onesweep on `im`, decided on the device)
     RW_CUDA(rwt::launch_keys(b, sc, pl, true, false, s));
     RW_CUDA(mark());
     if (int rc = rwt::learned_sort_enqueue(im->learned, static_cast<const uint32_t*>(b.keys),

@@ -11,7 +11,8 @@
 
 // Scratch for one pipeline instance (the reference's cuda::ImStorage,
 // apps/tree/cuda/im_storage.cuh:10-42, with the look-back state this design
-// needs).  The "zero region" is one allocation cleared before every run.
+// needs).  The "zero region" is the part of it that is cleared before every run of the
+// general chain of kernels.
 struct rw_tree_im_storage {
   uint32_t n_cap = 0;   // largest n_input this scratch serves
   int32_t key_bits = 32;

@@ -7,12 +7,11 @@
 // smaller keys (k_sort_fix).  The clouds that this is for have runs of a few
 // keys (uniform) or a few tens (mixtures of sigma 4 and more in a box of 1,024).
 //
-// Two other kinds of keys go to k_sort_rest, one launch behind, which costs 2 us
-// when there is nothing for it:
-//   - Segments dense everywhere: k_sort_init looks at a sample before the passes,
-//     which then leave a dense segment alone (dense_sample below).  It is
-//     sorted by all eight digits, as many passes as without the low bits left
-//     out, in one launch.
+// Two other kinds of keys go to k_sort_rest, one launch behind:
+//   - Segments in which keys mostly share their top bits, as samples taken in
+//     stage 1 tell (dense_sample, k_keys.cu): the passes leave such a segment
+//     alone, and it is sorted by the digits in which its keys differ, as the
+//     passes would without leaving low bits out, in one launch.
 //   - Runs of more than kFixRun keys among sparse ones: each is sorted by itself,
 //     by the digits left out, by one block.
 #include <algorithm>
@@ -36,8 +35,9 @@ constexpr int kFixWin = kFixTile + 2 * kFixRun;
 // any that share their top bits (nearly all of them) is stored as it is; the
 // others find their run's ends in the window's flags ("same top bits as the key
 // before", a bit each).  The window comes by one bulk copy: 25.4 us at 5,000,011
-// points (80 MB: 3.2 TB/s), where plain loads took 27.8 and gathering the sorted
-// tile in a second buffer 26.1.  The last of two waves of tiles is what is left.
+// points, where plain loads took 27.8 and gathering the sorted tile in a second
+// buffer 26.1; with the runs' ends from the flags 21.7 (80 MB: 3.7 TB/s), the empty
+// launch of k_sort_rest included.  The last of two waves of tiles is what is left.
 // Where it is dense, a block's time is what counts: 2,000,000 points in a cube of
 // side 24 (runs of 36) took 381 us in all when each key walked its run from
 // neighbour to neighbour, 269 now; with 1 % of them in a cube of side 4 447 and 248.
