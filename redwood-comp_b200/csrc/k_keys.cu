@@ -55,42 +55,51 @@ __host__ __device__ constexpr uint32_t pass_mask(int p) {
 // run has r keys on average.  The keys are those at random places, not every
 // (n / S)-th: neighbours in the input may be neighbours in space.  Sorted either
 // way the result is the same; a sample that misses costs time only.
-constexpr int kDenseSamples = 1024, kDenseSlots = 2 * kDenseSamples;
+constexpr int kDenseMost = 1024;  // samples of a block
 constexpr uint32_t kDenseRun = 48, kDenseFrom = 4096;
 
+// Enough for about 50 pairs at the line, in as little of the block's time as may be:
+// a batch of 1,000 clouds of 6,000 points takes 502 us without samples, 528 with
+// 1,024 of each cloud and 514 with 256 (256 clouds of 30,000: 558, 577, 574).
+__device__ __forceinline__ uint32_t dense_samples_log2(uint32_t n) {
+  return n <= (1u << 15) ? 8u : n <= (1u << 17) ? 9u : 10u;
+}
 __host__ __device__ __forceinline__ uint32_t dense_blocks(uint32_t segments) {
   return segments == 1 ? 4u : 1u;  // per segment
 }
 __device__ __forceinline__ bool is_dense(uint32_t pairs, uint32_t n, uint32_t segments) {
-  constexpr unsigned long long kAll = (kDenseSamples / 2) * kDenseSamples;
-  return n > kDenseFrom && pairs > 2 && pairs * (unsigned long long)n >
-                                            kDenseRun * kAll * dense_blocks(segments);
+  const unsigned long long all = 1ull << (2u * dense_samples_log2(n) - 1u);
+  return n > kDenseFrom && pairs > 2 &&
+         pairs * (unsigned long long)n > kDenseRun * all * dense_blocks(segments);
 }
 
-// One block's samples: the pairs among kDenseSamples of n keys, which key(i) gives
-// without their low bits, added to *pairs.
+// One block's samples: the pairs among them of n keys, which key(i) gives without
+// their low bits, added to *pairs.
 template <typename KeyAt>
 __device__ __forceinline__ void dense_sample(uint32_t n, const KeyAt& key, uint32_t* pairs) {
   // a slot: the top bits (41 at most) << 20 | how many samples had them
-  __shared__ unsigned long long s_slot[kDenseSlots];
+  __shared__ unsigned long long s_slot[2 * kDenseMost];
   if (n <= kDenseFrom) return;
-  uint64_t k[kDenseSamples / 256];
+  const uint32_t log2s = dense_samples_log2(n), slots = 2u << log2s;
+  const int each = int((1u << log2s) / 256u);  // a thread's samples
+  uint64_t k[kDenseMost / 256];
 #pragma unroll
-  for (int q = 0; q < kDenseSamples / 256; ++q) {
-    uint32_t x = (blockIdx.x * kDenseSamples + 256u * q + threadIdx.x) * 0x9e3779b9u + n;
+  for (int q = 0; q < kDenseMost / 256; ++q) {
+    if (q >= each) break;
+    uint32_t x = (blockIdx.x * kDenseMost + 256u * q + threadIdx.x) * 0x9e3779b9u + n;
     x = (x ^ (x >> 16)) * 0x85ebca6bu;  // murmur3's finisher
     x = (x ^ (x >> 13)) * 0xc2b2ae35u;
     k[q] = key(__umulhi(x ^ (x >> 16), n));
   }
-  for (int i = int(threadIdx.x); i < kDenseSlots; i += 256) s_slot[i] = 0;
+  for (uint32_t i = threadIdx.x; i < slots; i += 256) s_slot[i] = 0;
   __syncthreads();
   uint32_t found = 0;
 #pragma unroll
-  for (int q = 0; q < kDenseSamples / 256; ++q) {
+  for (int q = 0; q < kDenseMost / 256; ++q) {
+    if (q >= each) break;
     const unsigned long long top = (unsigned long long)k[q] << 20;
-    uint32_t at = uint32_t((k[q] * 0x9e3779b97f4a7c15ull) >> 53);
-    static_assert(kDenseSlots == 1 << 11, "11 bits of the hash");
-    for (int probe = 0; probe < kDenseSlots; ++probe, at = (at + 1) % kDenseSlots) {
+    uint32_t at = uint32_t((k[q] * 0x9e3779b97f4a7c15ull) >> (63u - log2s));
+    for (uint32_t probe = 0; probe < slots; ++probe, at = (at + 1) & (slots - 1u)) {
       unsigned long long old = s_slot[at];
       if (old == 0) old = atomicCAS(&s_slot[at], 0ull, top | 1ull);
       if (old == 0) break;
