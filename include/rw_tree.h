@@ -408,7 +408,7 @@ int rw_tree_learned_set_params(rw_tree_learned* learned, const float* params, in
 /* Context group size alone (for rw_tree_learned_features); default 4. */
 int rw_tree_learned_set_group(rw_tree_learned* learned, int32_t group);
 /* Sorts d_keys[0, n) (16-byte aligned) into d_sorted.  With `fallback_im`
- * (storage for n keys) the call is asynchronous on `stream` and capturable in
+ * (storage for n 32-bit keys) the call is asynchronous on `stream` and capturable in
  * a CUDA graph: the bucket sort and a onesweep sort on fallback_im are both
  * enqueued, and the plan's overflow word, on the device, lets exactly one of
  * them write d_sorted.  `stats` (may be NULL) is filled after one wait for

@@ -166,7 +166,7 @@ int sort_enqueue_gated(rw_tree_im_storage* im, const void* keys, void* out, uint
   // sort's kernels load and store keys one at a time, so only the word
   // alignment of the key type is needed
   if (!im || !keys || !out || n < 1 || n > im->n_cap || n >= RW_MAX_POINTS) return RW_ERR_ARG;
-  if (im->low_bits) return RW_ERR_ARG;  // (64-bit keys: what ends their sort is not gated)
+  if (im->key_bits != 32) return RW_ERR_ARG;  // (the keys would be read as 64-bit ones)
   rw_tree_app_data app;
   rw_tree_app_data_init(&app, n, im->key_bits);
   app.u_morton_keys = const_cast<void*>(keys);
@@ -584,7 +584,7 @@ int enqueue_impl(rw_tree_app_data* app, rw_tree_im_storage* im, cudaStream_t s,
       if (ev) RW_CUDA(cudaEventRecord(ev[k - 1], s));  // counts to the last pass
     }
   }
-  RW_CUDA(rwt::launch_unique(b, sc, pl, s, sc.low_bits != 0 && !im->learned));
+  RW_CUDA(rwt::launch_unique(b, sc, pl, s, sc.low_bits != 0));  // (learned: 32-bit keys)
   RW_CUDA(mark());
   RW_CUDA(rwt::launch_radix_tree(b, sc, pl, true, geometric_delta(im), s));
   RW_CUDA(mark());

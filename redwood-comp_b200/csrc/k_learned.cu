@@ -947,7 +947,8 @@ int rw_tree_learned_sort(rw_tree_learned* L, const uint32_t* d_keys, uint32_t* d
                          uint32_t n, int32_t mode, rw_tree_im_storage* fallback_im,
                          rw_stream_t stream, rw_tree_learned_stats* stats) {
   if (!L || !d_keys || !d_sorted || n > L->n_max || n < 1 || !aligned16(d_keys) ||
-      (mode != RW_LEARNED_MLP && mode != RW_LEARNED_SAMPLE_QUANTILES))
+      (mode != RW_LEARNED_MLP && mode != RW_LEARNED_SAMPLE_QUANTILES) ||
+      (fallback_im && (fallback_im->key_bits != 32 || fallback_im->n_cap < n)))
     return RW_ERR_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (stats) std::memset(stats, 0, sizeof *stats);
